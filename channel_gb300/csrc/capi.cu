@@ -96,10 +96,14 @@ struct chgpu_handle {
   void* twz = nullptr;
   void* twx = nullptr;
   void* twh = nullptr;
-  // register-blocked transform kernels (convf.cu), used for the lengths with
-  // a compile-time plan: their per-pass twiddle tables
+  // register-blocked transform kernels (convf.cuh; FP64 and double-float:
+  // the fixed-point ones of convx.cuh), used for the lengths with a
+  // compile-time plan: their per-pass twiddle tables
   void* twzr = nullptr;
   void* twxr = nullptr;
+  void* twhx = nullptr;  // fixed-point pack roots
+  FxFactor fxfac{};
+  double* rdy = nullptr;  // 1/dy per plane
   bool zfast = false, xfast = false;
   int xrvar = 4;  // register-blocked x-row variant: 4 (registers for 3 blocks per SM) or 5 (for 4)
   DevScalars* sc = nullptr;
@@ -323,6 +327,91 @@ int upload_pack_roots(chgpu_handle* h, void** dst, int n, long double scale) {
   return 0;
 }
 
+// a weight w 2^62 as the balanced 32-bit halves of the fixed-point twiddles
+// (fx.cuh); the lower half never -2^31, whose negative would not fit
+void fx_weight(long double w, int* hi, int* lo) {
+  const long long W = (long long)roundl(w * 4611686018427387904.0L);
+  const long long h = (W + 0x80000000ll) >> 32;
+  *hi = (int)h;
+  const long long l = W - (h << 32);
+  *lo = l == -0x80000000ll ? -0x7fffffff : (int)l;
+}
+int4 fx_root(long double phi, long double scale = 1.0L) {  // scale exp(-2 pi i phi)
+  const long double ang = 2.0L * 3.14159265358979323846264338327950288L * phi;
+  int4 e;
+  fx_weight(scale * cosl(ang), &e.x, &e.y);
+  fx_weight(-scale * sinl(ang), &e.z, &e.w);
+  return e;
+}
+bool fx_zlen_plan(int n, int* E, int* TPR) {
+  switch (n) {
+#define CHGPU_LEN(N) case N: *E = RLen<N>::E; *TPR = RLen<N>::TPR; return true;
+    CHGPU_FX_ZLENGTHS(CHGPU_LEN)
+#undef CHGPU_LEN
+    default: return false;
+  }
+}
+bool fx_xlen_plan(int n, int* E, int* TPR) {
+  switch (n) {
+#define CHGPU_LEN(N) case N: *E = FxXLen<N>::E; *TPR = FxXLen<N>::TPR; return true;
+    CHGPU_FX_XLENGTHS(CHGPU_LEN)
+#undef CHGPU_LEN
+    default: return false;
+  }
+}
+// register-blocked plan of a z or x length in this precision's kernels
+bool zplan(int prec, int n, int* E, int* TPR) {
+  return prec == CHGPU_MIXED ? rlen_plan(n, E, TPR) : fx_zlen_plan(n, E, TPR);
+}
+bool xplan(int prec, int n, int* E, int* TPR) {
+  return prec == CHGPU_MIXED ? xlen_plan(n, E, TPR) : fx_xlen_plan(n, E, TPR);
+}
+
+int upload_int4(chgpu_handle* h, void** dst, const std::vector<int4>& w) {
+  CK(h, cudaMalloc(dst, sizeof(int4) * w.size()));
+  CK(h, cudaMemcpy(*dst, w.data(), sizeof(int4) * w.size(), cudaMemcpyHostToDevice));
+  return 0;
+}
+// per-pass twiddles of the fixed-point kernels' plan, in the order of
+// upload_rplan_twiddles
+int upload_fx_twiddles(chgpu_handle* h, void** dst, int E, int TPR) {
+  std::vector<int4> w(std::max(1, rplan_twsize<fx2>(E, TPR)));
+  for (int p = 1; p < rplan_passes(E, TPR); ++p) {
+    const int R = rplan_radix(E, TPR, p), Ns = rplan_ns(E, TPR, p), off = rplan_twoff<fx2>(E, TPR, p);
+    for (int k = 0; k < Ns; ++k)
+      for (int r = 1; r < R; ++r) w[off + k * (R - 1) + r - 1] = fx_root((long double)(r * k) / (long double)(Ns * R));
+  }
+  return upload_int4(h, dst, w);
+}
+// tables of the fixed-point kernels for the lengths that have a plan: pass
+// twiddles, pack roots exp(-i pi k / nxd) then the same times g = factor/2 in
+// [1/2, 1) (FxFactor), 1/dy per plane
+int upload_fx_tables(chgpu_handle* h) {
+  int E = 0, TPR = 0;
+  if (fx_zlen_plan(h->d.nzd, &E, &TPR))
+    if (int rc = upload_fx_twiddles(h, &h->twzr, E, TPR)) return rc;
+  const int M = h->d.nxd;
+  if (fx_xlen_plan(M, &E, &TPR)) {
+    if (int rc = upload_fx_twiddles(h, &h->twxr, E, TPR)) return rc;
+    const long double half = 0.5L / (2.0L * (long double)M * (long double)h->d.nzd);
+    int ex = 0;
+    const long double g = frexpl(half, &ex);
+    h->fxfac.exp = ex;
+    fx_weight(g, &h->fxfac.gh, &h->fxfac.gl);
+    std::vector<int4> w(2 * (size_t)M);
+    for (int k = 0; k < M; ++k) {
+      w[k] = fx_root(0.5L * (long double)k / (long double)M);
+      w[M + k] = fx_root(0.5L * (long double)k / (long double)M, g);
+    }
+    if (int rc = upload_int4(h, &h->twhx, w)) return rc;
+  }
+  std::vector<double> r(h->d.nplanes, 0.0);
+  for (int iy = 1; iy <= h->p.ny - 1; ++iy) r[iy + 1] = 1.0 / h->tab.dy[iy];
+  CK(h, cudaMalloc((void**)&h->rdy, sizeof(double) * r.size()));
+  CK(h, cudaMemcpy(h->rdy, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice));
+  return 0;
+}
+
 // per-pass twiddles of a register-blocked plan (rfft.cuh): pass p >= 1 at
 // rplan_twoff(p), R-1 forward roots w_{Ns R}^{r k} (r = 1..R-1) per k < Ns,
 // padded to R per k in FP32 tables
@@ -332,18 +421,9 @@ int upload_rplan_twiddles(chgpu_handle* h, void** dst, int n, bool xplan = false
   int E = 0, TPR = 0;
   if (!(xplan ? xlen_plan(n, &E, &TPR) : rlen_plan(n, &E, &TPR))) return 0;
   const int np = rplan_passes(E, TPR);
-  const int tail = std::is_same<V2, double2>::value ? rplan_tailsize(E) : 0;
-  std::vector<V2> w(std::max(1, rplan_twsize<V2>(E, TPR) + tail));
-  if constexpr (std::is_same<V2, double2>::value) {  // the composite first pass's twiddled DFTs (rpass_first)
-    for (int k1 = 1; k1 <= 2 && tail > 0; ++k1)
-      lf_stage_entries(&w[rplan_twsize<V2>(E, TPR) + (k1 - 1) * (E / 3 - 1)], 3, E / 3, k1);
-  }
+  std::vector<V2> w(std::max(1, rplan_twsize<V2>(E, TPR)));
   for (int p = 1; p < np; ++p) {
     const int R = rplan_radix(E, TPR, p), Ns = rplan_ns(E, TPR, p), off = rplan_twoff<V2>(E, TPR, p);
-    if constexpr (std::is_same<V2, double2>::value) {  // every pass after the first has a power-of-two radix
-      for (int k = 0; k < Ns; ++k) lf_stage_entries(&w[off + k * (R - 1)], Ns, R, k);
-      continue;
-    }
     for (int k = 0; k < Ns; ++k)
       for (int r = 1; r < R; ++r) {
         const long double ang = 2.0L * 3.14159265358979323846264338327950288L * (long double)(r * k) /
@@ -411,6 +491,9 @@ ConvLaunch conv_launch(chgpu_handle* h, int compute_cfl, int products, int plane
   L.products = products;
   L.twzr = h->twzr;
   L.twxr = h->twxr;
+  L.twhx = h->twhx;
+  L.fxfac = h->fxfac;
+  L.rdy = h->rdy;
   L.zfast = h->zfast;
   L.xfast = h->xfast;
   return L;
@@ -626,7 +709,7 @@ void release(chgpu_handle* h) {
   }
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->fac, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
-                  h->twz, h->twx, h->twh, h->twzr, h->twxr, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
+                  h->twz, h->twx, h->twh, h->twzr, h->twxr, h->twhx, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
                   h->cl_G, h->cl_Z, h->cl_P, h->cl_tau, h->cl_wd, h->cl_twz, h->cl_twx, h->cl_twh,
                   h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean,
                   h->tke_twz, h->tke_twx, h->tke_twh};
@@ -702,15 +785,12 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   Radix rz = make_radix(nzd, false), rx = make_radix(nxd, h->prec == CHGPU_MIXED);
   if (rz.nst < 0 || rx.nst < 0) { delete h; return fail(nullptr, CHGPU_E_PARAM, "unsupported FFT length"); }
   {
-    // register-blocked transforms where they measured faster (GB300, 127x192x127
-    // and 383x384x383): FP32 z and x passes (x-row 92 -> 59 ms, z-forward
-    // 20 -> 10.5 ms per step at 383x384x383); FP64 z passes (even with the
-    // generic kernels; the FP64 x-row kernel stays generic, 977 vs 1017 ms);
-    // double-float keeps the generic kernels (its register-blocked x-row
-    // kernel spills: 820 vs 354 ms)
+    // register-blocked transforms for the lengths that have a plan: FP32 z
+    // and x passes (x-row 92 -> 59 ms, z-forward 20 -> 10.5 ms per step at
+    // 383x384x383); FP64 and double-float on fixed point (convx.cuh)
     int e_ = 0, tpr_ = 0;
-    h->zfast = rlen_plan(nzd, &e_, &tpr_) && h->prec != CHGPU_FP64DD;
-    h->xfast = xlen_plan(nxd, &e_, &tpr_) && h->prec == CHGPU_MIXED;
+    h->zfast = zplan(h->prec, nzd, &e_, &tpr_);
+    h->xfast = xplan(h->prec, nxd, &e_, &tpr_);
   }
   h->halves = d.npairs >= 65536 ? 2 : 1;
   h->solve_form = d.npairs < 65536 ? 3 : 1;
@@ -785,16 +865,14 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
       if ((rc = upload_stage_twiddles<cdd>(h, &h->twz, h->rz))) break;
       if ((rc = upload_stage_twiddles<cdd>(h, &h->twx, h->rx))) break;
       if ((rc = upload_pack_roots<cdd>(h, &h->twh, 2 * nxd, 0.5L * (long double)d.factor))) break;
-      if ((rc = upload_rplan_twiddles<cdd>(h, &h->twzr, nzd))) break;
-      if ((rc = upload_rplan_twiddles<cdd>(h, &h->twxr, nxd, true))) break;
+      if ((rc = upload_fx_tables(h))) break;
       if ((rc = upload_derT<dd>(h))) break;
       if ((rc = upload_derL<double>(h))) break;
     } else {
       if ((rc = upload_stage_twiddles<double2>(h, &h->twz, h->rz))) break;
       if ((rc = upload_stage_twiddles<double2>(h, &h->twx, h->rx))) break;
       if ((rc = upload_pack_roots<double2>(h, &h->twh, 2 * nxd, 0.5L * (long double)d.factor))) break;
-      if ((rc = upload_rplan_twiddles<double2>(h, &h->twzr, nzd))) break;
-      if ((rc = upload_rplan_twiddles<double2>(h, &h->twxr, nxd, true))) break;
+      if ((rc = upload_fx_tables(h))) break;
       if ((rc = upload_derT<double>(h))) break;
       if ((rc = upload_derL<double>(h))) break;
     }
@@ -1357,8 +1435,9 @@ int chgpu_autotune(chgpu_handle* h) {
   }
   h->zthreads = best_zt;
   }
-  // the register-blocked x-row kernel's register cap (3 or 4 resident blocks)
-  if (h->xfast) {
+  // the FP32 register-blocked x-row kernel's register cap (3 or 4 resident
+  // blocks; the fixed-point one has a single form)
+  if (h->xfast && h->prec == CHGPU_MIXED) {
     float best_v = 1e30f;
     int bv = h->xrvar;
     for (int v = 4; v <= 5; ++v) {
@@ -1420,10 +1499,10 @@ int chgpu_set_tiles(chgpu_handle* h, const int tiles[CHGPU_NTILES]) {
   const int zc = tiles[0], xr = tiles[1], xb = tiles[2], zt = tiles[3], xt = tiles[4], sf = tiles[5], hv = tiles[6];
   auto threads_ok = [](int t) { return t >= 64 && t <= 256 && t % 32 == 0; };
   int e_ = 0, tpr_ = 0;
-  const bool zplan = rlen_plan(h->d.nzd, &e_, &tpr_), xplan = xlen_plan(h->d.nxd, &e_, &tpr_);
-  if ((zc == 0 && !zplan) || (zc != 0 && (zc < 1 || zc > 8 || conv_zinv_smem(zc, h->d.nzd, h->d.nzt, ts) > lim)) ||
+  const bool zhas = zplan(h->prec, h->d.nzd, &e_, &tpr_), xhas = xplan(h->prec, h->d.nxd, &e_, &tpr_);
+  if ((zc == 0 && !zhas) || (zc != 0 && (zc < 1 || zc > 8 || conv_zinv_smem(zc, h->d.nzd, h->d.nzt, ts) > lim)) ||
       (xr != 1 && xr != 2 && xr != 4) || h->d.nzd % xr != 0 || conv_x_smem(xr, h->d.nxd, ts) > lim ||
-      (xb >= 4 && !xplan) || xb < 1 || xb > 5 || !threads_ok(zt) || !threads_ok(xt) || sf < 1 || sf > 5 ||
+      (xb >= 4 && !xhas) || xb < 1 || xb > 5 || !threads_ok(zt) || !threads_ok(xt) || sf < 1 || sf > 5 ||
       (hv != 1 && hv != 2))
     return fail(h, CHGPU_E_PARAM, "chgpu_set_tiles: tiles outside what this handle's sizes allow");
   h->zfast = zc == 0;

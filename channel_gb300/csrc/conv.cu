@@ -339,6 +339,17 @@ size_t conv_zinv_smem(int zcols, int nzd, int nzt, size_t ts) {
 }
 size_t conv_x_smem(int xrows, int nxd, size_t ts) { return 3 * (size_t)pad32_size(3 * xrows * nxd) * ts; }
 
+template <> bool launch_convolutions_r<double>(const ConvLaunch& L, cudaStream_t s, int stage) {
+  return stage == 1 ? launch_fx_x(L, s) : launch_fx_z<double>(L, s, stage);
+}
+// the double-float path's work buffers hold FP64 values between its three
+// fixed-point kernels, double-float ones between the generic kernels: all
+// three stages take the same family
+template <> bool launch_convolutions_r<dd>(const ConvLaunch& L, cudaStream_t s, int stage) {
+  if (!L.zfast || !L.xfast || L.tau) return false;
+  return stage == 0 ? launch_fx_z<double>(L, s, 0) : stage == 1 ? launch_fx_x(L, s) : launch_fx_z<dd>(L, s, 2);
+}
+
 template <typename T>
 void launch_convolutions(const ConvLaunch& L, cudaStream_t s, int stage) {
   using V2 = typename C2<T>::t;
@@ -421,9 +432,10 @@ cudaError_t conv_set_smem_limits() {
   if ((e = allow_max_smem(k_xrow<float, 2, true>, optin))) return e;
   if ((e = allow_max_smem(k_xrow<dd, 2, true>, optin))) return e;
   if ((e = allow_max_smem(k_xphys<float>, optin))) return e;
-  if ((e = convr_set_smem_limits<float>())) return e;
-  if ((e = convr_set_smem_limits<double>())) return e;
-  return convr_set_smem_limits<dd>();
+  if ((e = convr_set_smem_limits())) return e;
+  if ((e = fx_z_smem_limits<double>())) return e;
+  if ((e = fx_z_smem_limits<dd>())) return e;
+  return fx_x_smem_limits();
 }
 
 }  // namespace chgpu

@@ -25,8 +25,8 @@
 //              registers, the forward z transform, the last pass storing
 //              only |kz| <= nz (:590) into VV[p][plane][mode].
 //
-// T: double (FP64 step), float (mixed step) or dd (double-float step); one
-// translation unit per type (convf_f32.cu, convf_f64.cu, convf_dd.cu).
+// T: float (the mixed step; convf_f32.cu).  The FP64 and double-float steps
+// have the fixed-point kernels of convx.cuh.
 #pragma once
 
 #include <cuda_runtime.h>

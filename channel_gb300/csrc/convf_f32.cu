@@ -7,9 +7,6 @@ template <>
 bool launch_convolutions_r<float>(const ConvLaunch& L, cudaStream_t s, int stage) {
   return launch_convolutions_r_impl<float>(L, s, stage);
 }
-template <>
-cudaError_t convr_set_smem_limits<float>() {
-  return set_limits_type<float>();
-}
+cudaError_t convr_set_smem_limits() { return set_limits_type<float>(); }
 
 }  // namespace chgpu

@@ -1,0 +1,476 @@
+// The three transform kernels of `convolutions` (dnsdata.f90:487-602) for the
+// FP64 and double-float paths on 64-bit block fixed point (fx.cuh), with the
+// register-blocked passes of rfft.cuh:
+//
+//   k_zinv_x : one group of TPR threads per (plane, component, column kx).
+//              The modes go straight to registers in the transform's input
+//              distribution, the 3/2 zero band stays zero
+//              (dnsdata.f90:504-510); Zb gets the physical-z column.  Two
+//              scales: pass 1 combines one thread's inputs, so the largest
+//              sum over a thread bounds it, the later passes' values are
+//              bounded by the sum over the column.
+//   k_xrow_x : one group per plane row jz, NR rows per block, staged through
+//              shared memory as the zTOx / xTOz transposes
+//              (mpi_transpose.f90:50-117).  Per row: u, v, w packed for the
+//              half-length c2r (dnsdata.f90:533-535) and transformed, each
+//              normalised by the row's largest value so that the six
+//              products (:581-584) are 64x64-bit products of full-width
+//              numbers; the CFL maximum in FP64 (:552-556); the products
+//              transformed forward and unpacked for kx = 0..nx (:586-588).
+//   k_zfwd_x : one group per (plane, product, column): the column's scale
+//              from its largest value, the forward transform, |kz| <= nz
+//              stored (:590).
+//
+// V, Zb and Pb are FP64; VV is FP64 or, in the double-float path (whose
+// stencils read it), double-float.
+//
+// What bounds them (GB300, counters at 255x64x255): instruction issue of 12
+// resident warps per SM (34-43% of the issue slots, the rest fixed-latency and
+// instruction-fetch waits), not memory (1.5 TB/s in k_zinv_x).  Against the
+// FP64-pipe transforms they replace, the whole FP64 step went from 44.9 to
+// 19.3 ms at 127x192x127 and from 262 to 109 ms at 255x256x255 (k_xrow 39,
+// k_zfwd 10, k_zinv 6 ms of it); the double-float step from 16.7 to 15.5 ms.
+// Plans of 24 (16) points per thread need 168 registers; 128-thread blocks
+// keep three of them on an SM.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "chgpu_internal.h"
+#include "cplx.cuh"
+#include "fx.cuh"
+#include "kernels.cuh"
+#include "rfft.cuh"
+
+namespace chgpu {
+
+namespace {
+
+// reductions over a transform group; TPR > 32: through scratch (the group's
+// exchange buffer, not in use)
+enum { kRedMax, kRedSum, kRedOr };
+template <int OP> __device__ __forceinline__ int red_op(int a, int b) {
+  return OP == kRedMax ? max(a, b) : OP == kRedSum ? a + b : (a | b);
+}
+template <int OP, int TPR> __device__ __forceinline__ int group_reduce(int v, void* scratch, int t) {
+#pragma unroll
+  for (int o = (TPR < 32 ? TPR : 32) / 2; o > 0; o >>= 1) v = red_op<OP>(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if constexpr (TPR > 32) {
+    int* s = static_cast<int*>(scratch);
+    if ((t & 31) == 0) s[t >> 5] = v;
+    group_sync<TPR>();
+    v = s[0];
+#pragma unroll
+    for (int k = 1; k < TPR / 32; ++k) v = red_op<OP>(v, s[k]);
+    group_sync<TPR>();
+  }
+  return v;
+}
+
+__device__ __forceinline__ void xblock_max_atomic(double v, double* target) {
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __shared__ double wmax[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) wmax[wid] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double m = 0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) m = wmax[i] > m ? wmax[i] : m;
+    // non-negative doubles order like their bit patterns
+    atomicMax(reinterpret_cast<unsigned long long*>(target), (unsigned long long)__double_as_longlong(m));
+  }
+}
+
+// columns per z block: 128 threads, at most 32 columns
+template <int TPR> constexpr int fx_zcols() { return (128 / TPR) < 32 ? (128 / TPR) : 32; }
+// shared memory per x row in elements: u, v (and w without WREG) in physical
+// space, the padded exchange buffer, then pad so that a block's transposing
+// accesses (NR rows of consecutive elements) spread over the banks: a
+// wavefront of 16-byte elements is 8 lanes, NR rows of 8 / NR elements
+template <int M, int TPR, bool WREG> constexpr int fx_row_stride(int nr) {
+  int s = (WREG ? 3 : 4) * M + TPR;
+  while (s % 8 != (nr < 8 ? 8 / nr : 1)) ++s;
+  return s;
+}
+// rows per x block: at most 32 and 128 threads, within a third (WREG) or half
+// of an SM's 228 KB (1 KB reserved per block)
+template <int M, int TPR, bool WREG> constexpr int fx_xrows() {
+  int nr = 32;
+  const int budget = 233472 / (WREG ? 3 : 2) - 1024;
+  while (nr > 1 && (nr * fx_row_stride<M, TPR, WREG>(nr) * 16 > budget || nr * TPR > 128)) nr /= 2;
+  while (nr * TPR < 32) nr *= 2;
+  return nr;
+}
+// resident blocks the registers are capped for: what shared memory allows,
+// at most 12 warps per SM (168 registers)
+template <int M, int TPR, bool WREG> constexpr int fx_xminb() {
+  const int nr = fx_xrows<M, TPR, WREG>();
+  const int by_smem = 233472 / (nr * fx_row_stride<M, TPR, WREG>(nr) * 16 + 1024);
+  const int by_regs = 384 / (nr * TPR);
+  const int b = by_smem < by_regs ? by_smem : by_regs;
+  return b < 1 ? 1 : b;
+}
+
+}  // namespace
+
+template <int E, int TPR, int NC>
+__global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zinv_x(const double2* __restrict__ V,
+                                                                       double2* __restrict__ Zb,
+                                                                       const fx2* __restrict__ tw, Dims d, int plane0,
+                                                                       int ix_lo, int ix_hi) {
+  using In = FxIo<double>;
+  constexpr int N = E * TPR;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  fx2* buf = reinterpret_cast<fx2*>(smem_raw) + (threadIdx.x / TPR) * rbuf_size<E, TPR>();
+  const int t = threadIdx.x % TPR;
+  const int c = blockIdx.z, plane = plane0 + blockIdx.y;
+  const int ix = ix_lo + blockIdx.x * NC + (int)(threadIdx.x / TPR);
+  const bool active = ix < ix_hi;
+  const int nz = d.nz, nzt = d.nzt;
+  const size_t col = ((size_t)c * d.nplanes + plane) * (d.nx + 1) + (active ? ix : ix_lo);
+  const double2* src = V + col * nzt;
+  double2 raw[E];
+  int emax = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int jz = t + TPR * e;
+    const int izp = jz <= nz ? nz + jz : (jz >= N - nz ? jz - N + nz : -1);
+    raw[e] = make_double2(0.0, 0.0);
+    if (active && izp >= 0) raw[e] = __ldg(src + izp);
+    emax = max(emax, max(In::expo(raw[e].x), In::expo(raw[e].y)));
+  }
+  emax = group_reduce<kRedMax, TPR>(emax, buf, t);
+  unsigned B = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) B += fx_lead_at(raw[e].x, emax) + fx_lead_at(raw[e].y, emax);
+  const unsigned B1 = (unsigned)group_reduce<kRedMax, TPR>((int)B, buf, t);
+  B = (unsigned)group_reduce<kRedSum, TPR>((int)B, buf, t);
+  const int S1 = emax == 0 ? 0 : fx_scale_sum<double>(emax, B1, 62);
+  const int S = emax == 0 ? 0 : fx_scale_sum<double>(emax, B, 62);
+  fx2 a[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) a[e] = fx_load<double>(raw[e], S1);
+  const int So = S - 2;  // one pass at quarter scale
+  const int mode = fx_mode<double>(So, emax == In::kExpMax);
+  double2* dst = Zb + col * N;
+  rfft<E, TPR, +1>(
+      a, buf, t, tw,
+      [&](int o, fx2 v) {
+        if (active) dst[o] = fx_store<double>(v, So, mode);
+      },
+      [&] {
+#pragma unroll
+        for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], S1 - S);
+      });
+}
+
+template <typename T, int E, int TPR, int NC>
+__global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zfwd_x(const double2* __restrict__ Pb,
+                                                                       typename C2<T>::t* __restrict__ VV,
+                                                                       const fx2* __restrict__ tw, Dims d, int plane0) {
+  using V2 = typename C2<T>::t;
+  using Io = FxIo<double>;
+  constexpr int N = E * TPR;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  fx2* buf = reinterpret_cast<fx2*>(smem_raw) + (threadIdx.x / TPR) * rbuf_size<E, TPR>();
+  const int t = threadIdx.x % TPR;
+  const int p = blockIdx.z, plane = plane0 + blockIdx.y;
+  const int nxp = d.nx + 1;
+  const int ix = blockIdx.x * NC + (int)(threadIdx.x / TPR);
+  const bool active = ix < nxp;
+  const int nz = d.nz, nzt = d.nzt;
+  const size_t col = ((size_t)p * d.nplanes + plane) * nxp + (active ? ix : 0);
+  const double2* src = Pb + col * N;
+  double2 raw[E];
+  int emax = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    raw[e] = active ? ldg_v(src + t + TPR * e) : make_double2(0.0, 0.0);
+    emax = max(emax, max(Io::expo(raw[e].x), Io::expo(raw[e].y)));
+  }
+  emax = group_reduce<kRedMax, TPR>(emax, buf, t);
+  // |re|, |im| < 2^(emax - bias + 1)
+  const int S = emax == 0 ? 0 : fx_forward_bits(E, TPR, 62) - (emax - Io::kBias + 1);
+  fx2 a[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) a[e] = fx_load<double>(raw[e], S);
+  const int So = S - 2 * fx_quarters(E, TPR);
+  const int mode = fx_mode<T>(So, emax == Io::kExpMax);
+  V2* dst = VV + col * nzt + nz;
+  rfft<E, TPR, -1>(a, buf, t, tw, [&](int o, fx2 v) {
+    if (!active) return;
+    if (o <= nz) dst[o] = fx_store<T>(v, So, mode);
+    else if (o >= N - nz) dst[o - N] = fx_store<T>(v, So, mode);
+  });
+}
+
+// Row layout in shared memory: u and v in physical space (M each), then the
+// padded exchange buffer X (M + TPR), which first holds the row's w spectrum;
+// without WREG w's physical values take a third slot before X.
+template <int E, int TPR, int NR, int MINB, bool WREG>
+__global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __restrict__ Zb,
+                                                           double2* __restrict__ Pb,
+                                                           const fx2* __restrict__ tw, const fx2* __restrict__ twh,
+                                                           Dims d, FxFactor fac, int plane0, int compute_cfl,
+                                                           const double* __restrict__ rdy, DevScalars* sc) {
+  using V2 = double2;
+  using Io = FxIo<double>;
+  static_assert(sizeof(V2) == sizeof(fx2), "rows are converted in place");
+  constexpr int M = E * TPR;
+  constexpr int RS = fx_row_stride<M, TPR, WREG>(NR);
+  constexpr int NT = NR * TPR;
+  // bits of the physical values: their products, 2 kBits - 64 bits, are the
+  // forward transform's inputs (whose outputs stay below 2^61 for the unpacking)
+  constexpr int kBits = (fx_forward_bits(E, TPR, 61) + 64) / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  V2* S = reinterpret_cast<V2*>(smem_raw);
+  fx2* Sf = reinterpret_cast<fx2*>(smem_raw);
+  const int row = threadIdx.x / TPR, t = threadIdx.x % TPR;
+  fx2* U = Sf + row * RS;
+  fx2* X = U + (WREG ? 2 : 3) * M;  // the exchange buffer; without WREG w's slot sits before it
+  const int nx = d.nx, nxp = nx + 1, nzd = d.nzd;
+  const int plane = plane0 + blockIdx.y;
+  const int jz0 = blockIdx.x * NR;
+  const int nrow = min(NR, nzd - jz0);
+  // the block's rows of the three spectra (zTOx): NR consecutive jz per kx,
+  // w into X (with WREG) or into its own slot
+  for (int c = 0; c < 3; ++c) {
+    const V2* src = Zb + ((size_t)c * d.nplanes + plane) * nxp * nzd + jz0;
+    for (int i = threadIdx.x; i < nxp * NR; i += NT) {
+      const int r = i % NR, k = i / NR;
+      V2 v = make_double2(0.0, 0.0);
+      if (r < nrow) v = ldg_v(src + (size_t)k * nzd + r);
+      S[r * RS + c * M + k] = v;
+    }
+  }
+  __syncthreads();
+  int su = 0, sv = 0, sw = 0;  // scales of u, v, w in physical space
+  int bad = 0;                 // bit c: component c of this row is not finite
+  fx2 w[WREG ? E : 1];  // with WREG: w in physical space, w[e] at x pair t + TPR e
+  // one component: the spectrum in its slot to physical values in a[]
+  auto inverse = [&](int c, fx2 (&a)[E]) {
+    fx2* F = U + c * M;
+    const V2* Fr = reinterpret_cast<const V2*>(F);
+    int emax = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int n = t + TPR * e;
+      if (n <= nx) {
+        const V2 v = Fr[n];
+        emax = max(emax, max(Io::expo(v.x), Io::expo(v.y)));
+      }
+    }
+    emax = group_reduce<kRedMax, TPR>(emax, nullptr, t);
+    // |re|, |im| < 2^57, so that the packed |re|, |im| stay below 2^60
+    const int s0 = emax == 0 ? 0 : 57 - (emax - Io::kBias + 1);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int n = t + TPR * e;
+      if (n <= nx) F[n] = fx_load<double>(Fr[n], s0);
+    }
+    group_sync<TPR>();
+    // c2r by the half-length packing
+    //   Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) e^{+i pi k / M}
+    // (only Re of the kx = 0 entry; the x zero band kx > nx, dnsdata.f90:535)
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int n = t + TPR * e;
+      fx2 xk{0, 0}, xm{0, 0};
+      if (n <= nx) xk = F[n];
+      if (n == 0) xk.y = 0;
+      else if (M - n <= nx) {
+        xm = F[M - n];
+        xm.y = -xm.y;
+      }
+      a[e] = (xk + xm) + mul_is<+1>(fx_cmul4<+1>(xk - xm, fx_ldw(twh + n)));
+    }
+    // the scales of pass 1 (its values are bounded by the largest sum of
+    // |re| + |im| over a thread) and of the later passes (the sum over the
+    // row), both sums below 2^61: shifts d1, then d2
+    unsigned b1 = 0;  // in units of 2^39, at most 2 E 2^21 + 2 E
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      b1 += (unsigned)(abs(fx_up(a[e].x)) >> 7) + (unsigned)(abs(fx_up(a[e].y)) >> 7) + 2u;
+    const unsigned bs = (unsigned)group_reduce<kRedSum, TPR>((int)b1, nullptr, t);
+    b1 = (unsigned)group_reduce<kRedMax, TPR>((int)b1, nullptr, t);
+    const int d1 = max(0, 32 - __clz((int)b1) + 39 - 61), d2 = max(d1, 32 - __clz((int)bs) + 39 - 61) - d1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], d1);
+    group_sync<TPR>();  // every read of the spectrum before its slot or X is written
+    rfft_regs<E, TPR, +1>(a, X, t, tw, [&] {
+#pragma unroll
+      for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], d2);
+    });
+    // normalise: the row's largest |re|, |im| just below 2^kBits
+    int m = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int hx = fx_up(a[e].x), hy = fx_up(a[e].y);
+      m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
+    }
+    m = group_reduce<kRedOr, TPR>(m, nullptr, t);
+    static_assert(kBits >= 60, "values below 2^60 are shifted left");
+    const int sh = __clz(m) - (64 - kBits);
+#pragma unroll
+    for (int e = 0; e < E; ++e) a[e] = fx2{a[e].x << sh, a[e].y << sh};
+    const int sc = s0 - d1 - d2 - 2 + sh;  // one pass at quarter scale
+    if (c == 0) su = sc;
+    else if (c == 1) sv = sc;
+    else sw = sc;
+    if (emax == Io::kExpMax) bad |= 1 << c;
+  };
+  if constexpr (WREG) inverse(2, w);
+#pragma unroll 1
+  for (int c = 0; c < (WREG ? 2 : 3); ++c) {
+    fx2 a[E];
+    inverse(c, a);
+#pragma unroll
+    for (int e = 0; e < E; ++e) U[c * M + t + TPR * e] = a[e];
+  }
+  // each thread reads back only its own physical values
+  auto val = [&](int c, int e) -> fx2 {
+    if (WREG && c == 2) return w[WREG ? e : 0];
+    return U[c * M + t + TPR * e];
+  };
+  // CFL (dnsdata.f90:552-556) over the physical values of this row, in FP64
+  if (compute_cfl) {
+    double cfl = 0.0;
+    bool inf = false;
+    if (plane >= 2 && plane <= d.ny && row < nrow) {
+      double r[3] = {d.rdx, rdy[plane], d.rdz};
+      const int s3[3] = {su, sv, sw};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int md = fx_mode<double>(s3[c], (bad >> c) & 1);
+        inf = inf || md == 2;
+        r[c] = md ? 0.0 : r[c] * __hiloint2double((1023 - s3[c]) << 20, 0);
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const fx2 u = val(0, e), v = val(1, e), ww = val(2, e);
+        auto mag = [](long long x) { return __ll2double_rn(x < 0 ? -x : x); };
+        cfl = fmax(cfl, fma(mag(ww.x), r[2], fma(mag(v.x), r[1], mag(u.x) * r[0])));
+        cfl = fmax(cfl, fma(mag(ww.y), r[2], fma(mag(v.y), r[1], mag(u.y) * r[0])));
+      }
+    }
+    if (inf) cfl = (double)INFINITY;  // a non-finite velocity shows up as an infinite CFL
+    xblock_max_atomic(cfl, &sc->cfl);
+  }
+  // products (dnsdata.f90:581-584), with WREG those with w first (w then
+  // dies): ww, vw, uw, uu, vv, uv -> Pb slots 2, 4, 5, 0, 1, 3; `factor`
+  // enters in the unpacking: g = (factor/2) 2^-fac.exp in [1/2, 1) as fac
+  // and in twh[M + k] = g e^{-i pi k/M}
+#pragma unroll 1
+  for (int q = 0; q < 6; ++q) {
+    const int p = !WREG ? q : (q == 0 ? 2 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 0 : q == 4 ? 1 : 3);
+    // factors of product p (uu, vv, ww, uv, vw, uw)
+    const int fa = p < 3 ? p : (p == 5 ? 0 : p - 3);
+    const int fb = p < 3 ? p : (p == 3 ? 1 : 2);
+    fx2 a[E];
+    if (WREG && q < 3) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const fx2 y = w[WREG ? e : 0], x = q == 0 ? y : U[fa * M + t + TPR * e];
+        a[e] = fx2{fx_mul(x.x, y.x), fx_mul(x.y, y.y)};
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const fx2 x = U[fa * M + t + TPR * e], y = U[fb * M + t + TPR * e];
+        a[e] = fx2{fx_mul(x.x, y.x), fx_mul(x.y, y.y)};
+      }
+    }
+    const int sa = fa == 0 ? su : (fa == 1 ? sv : sw), sb = fb == 0 ? su : (fb == 1 ? sv : sw);
+    const bool nf = ((bad >> fa) | (bad >> fb)) & 1;
+    const int So = sa + sb - 64 - 2 * (1 + fx_quarters(E, TPR)) - fac.exp;
+    const int mode = fx_mode<double>(So, nf);
+    rfft<E, TPR, -1>(a, X, t, tw, [&](int o, fx2 v) { X[o] = v; });
+    group_sync<TPR>();
+    // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586), at quarter scale:
+    //   X = g (Z_k + conj Z_{M-k}) + (g w_k) (-i) (Z_k - conj Z_{M-k})
+    V2 o[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int k = t + TPR * e;
+      if (k <= nx) {
+        const fx2 zk = X[k], zc = X[k == 0 ? 0 : M - k];
+        const fx2 sm{zk.x + zc.x, zk.y - zc.y}, df{zk.x - zc.x, zk.y + zc.y};
+        const fx2 rot = fx_cmul<-1>(fx2{df.y, -df.x}, fx_ldw(twh + M + k));
+        o[e] = fx_store<double>(fx2{fx_mad(rot.x, sm.x, fac.gh, fac.gl), fx_mad(rot.y, sm.y, fac.gh, fac.gl)}, So, mode);
+      }
+    }
+    group_sync<TPR>();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int k = t + TPR * e;
+      if (k <= nx) reinterpret_cast<V2*>(X)[k] = o[e];
+    }
+    __syncthreads();
+    // xTOz: the block's rows of product p, NR consecutive jz per kx
+    V2* dst = Pb + ((size_t)p * d.nplanes + plane) * nxp * nzd + jz0;
+    for (int i = threadIdx.x; i < nxp * NR; i += NT) {
+      const int r = i % NR, k = i / NR;
+      if (r < nrow) dst[(size_t)k * nzd + r] = S[r * RS + (WREG ? 2 : 3) * M + k];
+    }
+    __syncthreads();
+  }
+}
+
+namespace {
+
+template <typename T, int N>
+void fx_launch_z(const ConvLaunch& L, cudaStream_t s, int stage) {
+  using V2 = typename C2<T>::t;
+  constexpr int E = RLen<N>::E, TPR = RLen<N>::TPR, NC = fx_zcols<TPR>();
+  const size_t sm = (size_t)NC * rbuf_size<E, TPR>() * sizeof(fx2);
+  const Dims& d = L.d;
+  if constexpr (std::is_same<T, double>::value) {
+    if (stage == 0) {
+      dim3 grid((L.ix_hi - L.ix_lo + NC - 1) / NC, L.nplanes, 3);
+      k_zinv_x<E, TPR, NC><<<grid, NC * TPR, sm, s>>>(L.V, (double2*)L.Zb, (const fx2*)L.twzr, d, L.plane0, L.ix_lo,
+                                                      L.ix_hi);
+    }
+  }
+  if (stage == 2) {
+    dim3 grid((d.nx + 1 + NC - 1) / NC, L.nplanes, 6);
+    k_zfwd_x<T, E, TPR, NC><<<grid, NC * TPR, sm, s>>>((const double2*)L.Pb, (V2*)L.VV, (const fx2*)L.twzr, d,
+                                                       L.plane0);
+  }
+}
+
+template <int M>
+void fx_launch_x(const ConvLaunch& L, cudaStream_t s) {
+  constexpr int E = FxXLen<M>::E, TPR = FxXLen<M>::TPR;
+  constexpr bool WREG = FxXLen<M>::WREG;
+  constexpr int NR = fx_xrows<M, TPR, WREG>(), MINB = fx_xminb<M, TPR, WREG>();
+  const size_t sm = (size_t)NR * fx_row_stride<M, TPR, WREG>(NR) * sizeof(fx2);
+  const Dims& d = L.d;
+  dim3 grid((d.nzd + NR - 1) / NR, L.nplanes);
+  k_xrow_x<E, TPR, NR, MINB, WREG><<<grid, NR * TPR, sm, s>>>((const double2*)L.Zb, (double2*)L.Pb,
+                                                              (const fx2*)L.twxr, (const fx2*)L.twhx, d, L.fxfac,
+                                                              L.plane0, L.compute_cfl, L.rdy, L.sc);
+}
+
+template <typename K> cudaError_t fx_allow_smem(K* kernel, size_t bytes, bool max_carveout = false) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && max_carveout)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  return e;
+}
+template <typename T, int N> cudaError_t fx_limits_z() {
+  constexpr int E = RLen<N>::E, TPR = RLen<N>::TPR, NC = fx_zcols<TPR>();
+  const size_t sm = (size_t)NC * rbuf_size<E, TPR>() * sizeof(fx2);
+  cudaError_t e = std::is_same<T, double>::value ? fx_allow_smem(k_zinv_x<E, TPR, NC>, sm) : cudaSuccess;
+  return e == cudaSuccess ? fx_allow_smem(k_zfwd_x<T, E, TPR, NC>, sm) : e;
+}
+template <int M> cudaError_t fx_limits_x() {
+  constexpr int E = FxXLen<M>::E, TPR = FxXLen<M>::TPR;
+  constexpr bool WREG = FxXLen<M>::WREG;
+  constexpr int NR = fx_xrows<M, TPR, WREG>(), MINB = fx_xminb<M, TPR, WREG>();
+  return fx_allow_smem(k_xrow_x<E, TPR, NR, MINB, WREG>, (size_t)NR * fx_row_stride<M, TPR, WREG>(NR) * sizeof(fx2),
+                       true);
+}
+
+}  // namespace
+
+}  // namespace chgpu

@@ -1,0 +1,22 @@
+// Fixed-point x rows (convx.cuh).
+#include "convx.cuh"
+
+namespace chgpu {
+
+bool launch_fx_x(const ConvLaunch& L, cudaStream_t s) {
+  switch (L.d.nxd) {
+#define CHGPU_LEN(N) case N: fx_launch_x<N>(L, s); return true;
+    CHGPU_FX_XLENGTHS(CHGPU_LEN)
+#undef CHGPU_LEN
+    default: return false;
+  }
+}
+cudaError_t fx_x_smem_limits() {
+  cudaError_t e = cudaSuccess;
+#define CHGPU_LEN(N) if (e == cudaSuccess) e = fx_limits_x<N>();
+  CHGPU_FX_XLENGTHS(CHGPU_LEN)
+#undef CHGPU_LEN
+  return e;
+}
+
+}  // namespace chgpu

@@ -27,6 +27,12 @@ struct BcRows {
   double d140[5], d14m1[5], d14n[5], d14np1[5];
 };
 
+// factor/2 (dnsdata.f90:124) = (g / 2^62) 2^exp with g / 2^62 in [1/2, 1), g =
+// gh 2^32 + gl, for the fixed-point x rows
+struct FxFactor {
+  int gh, gl, exp;
+};
+
 struct ConvLaunch {
   Dims d;
   RadixDev rz, rx;
@@ -53,21 +59,35 @@ struct ConvLaunch {
   const void* twzr;
   const void* twxr;
   int zfast, xfast;
+  // the fixed-point kernels of the FP64 and double-float paths: pack roots,
+  // factor/2, 1/dy per plane
+  const void* twhx;
+  FxFactor fxfac;
+  const double* rdy;
 };
 
 // stage 0: z-inverse, 1: x rows, 2: z-forward
 template <typename T> void launch_convolutions(const ConvLaunch& L, cudaStream_t s, int stage);
 cudaError_t conv_set_smem_limits();
-// the register-blocked stage kernels; false when the stage's length has no plan
+// the register-blocked stage kernels; false when the stage's length has no
+// plan.  float: convf.cuh (convf_f32.cu); double and dd: the fixed-point ones
+// of convx.cuh (convx_z_f64.cu, convx_z_dd.cu, convx_x.cu)
 template <typename T> bool launch_convolutions_r(const ConvLaunch& L, cudaStream_t s, int stage);
-template <typename T> cudaError_t convr_set_smem_limits();
-// defined in convf_f32.cu, convf_f64.cu, convf_dd.cu
 template <> bool launch_convolutions_r<float>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_convolutions_r<double>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_convolutions_r<dd>(const ConvLaunch& L, cudaStream_t s, int stage);
-template <> cudaError_t convr_set_smem_limits<float>();
-template <> cudaError_t convr_set_smem_limits<double>();
-template <> cudaError_t convr_set_smem_limits<dd>();
+cudaError_t convr_set_smem_limits();
+// stage 0 and 2 (T: VV's type; stage 0 is launch_fx_z<double>), stage 1
+template <typename T> bool launch_fx_z(const ConvLaunch& L, cudaStream_t s, int stage);
+template <> bool launch_fx_z<double>(const ConvLaunch& L, cudaStream_t s, int stage);
+template <> bool launch_fx_z<dd>(const ConvLaunch& L, cudaStream_t s, int stage);
+bool launch_fx_x(const ConvLaunch& L, cudaStream_t s);
+template <typename T> cudaError_t fx_z_smem_limits();
+template <> cudaError_t fx_z_smem_limits<double>();
+template <> cudaError_t fx_z_smem_limits<dd>();
+cudaError_t fx_x_smem_limits();
+#define CHGPU_FX_ZLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536)
+#define CHGPU_FX_XLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768)
 // dynamic shared memory of the z-transform and x-row kernels (padded buffers)
 size_t conv_z_smem(int zcols, int nzd, size_t ts);                     // z-forward
 size_t conv_zinv_smem(int zcols, int nzd, int nzt, size_t ts);         // z-inverse (raw field copy)

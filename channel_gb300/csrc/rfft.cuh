@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "cplx.cuh"
+#include "fx.cuh"
 
 namespace chgpu {
 
@@ -92,43 +93,11 @@ template <int TPR> __device__ __forceinline__ void group_sync() {
   }
 }
 
-// pass 1: one radix-E register DFT per thread.  FP64 with E = 3P: the
-// composite DFT's two twiddled P-point DFTs (twiddles W_{3P}^{r k1}, k1 = 1,
-// 2) in the fused multiply-add form, from the 2 (P-1) pairs at the end of
-// the plan's table
+// pass 1: one radix-E register DFT per thread
 template <int E, int TPR, int SIGN, typename V>
-__device__ __forceinline__ void rpass_first(V (&a)[E], const V* __restrict__ tw) {
-  if constexpr (std::is_same<V, double2>::value && E % 3 == 0 && is_pow2c(E / 3)) {
-    constexpr int P = E / 3;
-    const V* tail = tw + rplan_twsize<V>(E, TPR);
-#pragma unroll
-    for (int r2 = 0; r2 < P; ++r2) {
-      V b[3] = {a[r2], a[P + r2], a[2 * P + r2]};
-      Dft<3, V>::template run<SIGN>(b);
-      a[r2] = b[0];
-      a[P + r2] = b[1];
-      a[2 * P + r2] = b[2];
-    }
-    V y[E];
-#pragma unroll
-    for (int k1 = 0; k1 < 3; ++k1) {
-      V c[P];
-#pragma unroll
-      for (int r2 = 0; r2 < P; ++r2) c[r2] = a[k1 * P + r2];
-      if (k1 == 0) Dft<P, V>::template run<SIGN>(c);
-      else lf_dft<P, SIGN>(c, tail + (k1 - 1) * (P - 1));
-#pragma unroll
-      for (int k2 = 0; k2 < P; ++k2) y[k1 + 3 * k2] = c[k2];
-    }
-#pragma unroll
-    for (int k = 0; k < E; ++k) a[k] = y[k];
-  } else {
-    Dft<E, V>::template run<SIGN>(a);
-  }
-}
-// entries after the per-pass twiddles: FP64 composite first passes only
-__host__ __device__ constexpr int rplan_tailsize(int E) {
-  return (E % 3 == 0 && E / 3 >= 2 && ((E / 3) & (E / 3 - 1)) == 0) ? 2 * (E / 3 - 1) : 0;
+__device__ __forceinline__ void rpass_first(V (&a)[E]) {
+  if constexpr (std::is_same<V, fx2>::value) fx_first<E, SIGN>(a);
+  else Dft<E, V>::template run<SIGN>(a);
 }
 
 // The R-1 twiddles w^1..w^(R-1) of one butterfly from its run of the
@@ -137,8 +106,7 @@ __host__ __device__ constexpr int rplan_tailsize(int E) {
 // w^7 as products with w^4 (one more rounding, ~1e-7), a radix-4 one loads
 // w^1, w^2 as one and forms w^3; fewer loads for these latency-limited
 // kernels (products in place of loads measured 3-4% faster on GB300; the
-// paired loads measured even).  FP64 and double-float load every value
-// (their multiplications bound them).
+// paired loads measured even).
 constexpr bool TW_PRODUCTS = true;
 template <int R, typename V> __device__ __forceinline__ void load_twiddles(const V* w, V (&tw)[R]) {
   if constexpr (TW_PRODUCTS && std::is_same<V, float2>::value && R == 8) {
@@ -163,20 +131,25 @@ template <int R, typename V> __device__ __forceinline__ void load_twiddles(const
   }
 }
 
-// One butterfly of a pass p >= 1: the R-1 twiddles of its run of the table,
-// then the R-point DFT; FP64 in the fused multiply-add form (lf_dft, whose
-// tables hold (c, t) pairs in its order)
-template <int R, int SIGN, typename V> __device__ __forceinline__ void twiddled_dft(V (&b)[R], const V* w) {
+// One butterfly of pass P >= 1: the R-1 twiddles of its run of the table,
+// then the R-point DFT.  Fixed point (fx.cuh): the twiddled inputs, and so
+// the outputs, are a quarter of the true ones in a forward transform and in a
+// backward one's second pass.
+template <int R, int SIGN, int P, typename V> __device__ __forceinline__ void twiddled_dft(V (&b)[R], const V* w) {
   static_assert(is_pow2c(R), "passes after the first have power-of-two radices");
-  if constexpr (std::is_same<V, double2>::value) {
-    lf_dft<R, SIGN>(b, w);
+  if constexpr (std::is_same<V, fx2>::value) {
+    constexpr bool quarter = SIGN < 0 || P == 1;
+    if (quarter) b[0] = fx_quarter(b[0]);
+#pragma unroll
+    for (int r = 1; r < R; ++r)
+      b[r] = quarter ? fx_cmul<SIGN>(b[r], fx_ldw(w + r - 1)) : fx_cmul4<SIGN>(b[r], fx_ldw(w + r - 1));
   } else {
     V tw_[R];
     load_twiddles<R>(w, tw_);
 #pragma unroll
     for (int r = 1; r < R; ++r) b[r] = cmul_s_inner<SIGN>(b[r], tw_[r]);
-    Dft<R, V>::template run<SIGN>(b);
   }
+  Dft<R, V>::template run<SIGN>(b);
 }
 
 // Writes the outputs of a pass whose inputs are in a[] (pass p >= 1) or the
@@ -202,7 +175,7 @@ __device__ __forceinline__ void rpass_store(V (&a)[E], V* buf, int t, const V* _
       V b[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) b[r] = a[i + r * B];
-      twiddled_dft<R, SIGN>(b, twp + k * tw_per_k<V>(R));
+      twiddled_dft<R, SIGN, P>(b, twp + k * tw_per_k<V>(R));
       const int base = (j - k) * R + k;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -244,7 +217,7 @@ __device__ __forceinline__ void rpass_last_any(V (&a)[E], int t, const V* __rest
       V b[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) b[r] = a[i + r * B];
-      twiddled_dft<R, SIGN>(b, twp + j * tw_per_k<V>(R));
+      twiddled_dft<R, SIGN, P>(b, twp + j * tw_per_k<V>(R));
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if constexpr (TO_REGS) a[i + r * B] = b[r];
@@ -256,11 +229,16 @@ __device__ __forceinline__ void rpass_last_any(V (&a)[E], int t, const V* __rest
 
 // Every pass but the last: a[] holds the input distribution on entry and the
 // last pass's inputs on return; buf is the group's padded exchange buffer
-// (rbuf_size elements).  Every thread of the group calls it.
-template <int E, int TPR, int SIGN, typename V>
-__device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __restrict__ tw) {
+// (rbuf_size elements).  after_first() runs between passes 1 and 2.  Every
+// thread of the group calls it.
+struct RNothing {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <int E, int TPR, int SIGN, typename V, typename After = RNothing>
+__device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __restrict__ tw, After after_first = After()) {
   constexpr int NP = rplan_passes(E, TPR);
-  rpass_first<E, TPR, SIGN>(a, tw);
+  rpass_first<E, TPR, SIGN>(a);
+  after_first();
   if constexpr (NP >= 2) {
     rpass_store<E, TPR, 0, SIGN, true>(a, buf, t, tw);
     group_sync<TPR>();
@@ -285,16 +263,18 @@ __device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __r
 // Whole transform, a[] holding the input distribution (x[t + TPR e]) on
 // entry, the outputs handed to sink(index, value).  The caller synchronises
 // the group before reusing buf.
-template <int E, int TPR, int SIGN, typename V, typename Sink>
-__device__ __forceinline__ void rfft(V (&a)[E], V* buf, int t, const V* __restrict__ tw, Sink sink) {
-  rfft_head<E, TPR, SIGN>(a, buf, t, tw);
+template <int E, int TPR, int SIGN, typename V, typename Sink, typename After = RNothing>
+__device__ __forceinline__ void rfft(V (&a)[E], V* buf, int t, const V* __restrict__ tw, Sink sink,
+                                     After after_first = After()) {
+  rfft_head<E, TPR, SIGN>(a, buf, t, tw, after_first);
   rpass_last_any<E, TPR, SIGN, false>(a, t, tw, sink);
 }
 
 // Whole transform with the outputs left in a[] (a[e] = x[t + TPR e]).
-template <int E, int TPR, int SIGN, typename V>
-__device__ __forceinline__ void rfft_regs(V (&a)[E], V* buf, int t, const V* __restrict__ tw) {
-  rfft_head<E, TPR, SIGN>(a, buf, t, tw);
+template <int E, int TPR, int SIGN, typename V, typename After = RNothing>
+__device__ __forceinline__ void rfft_regs(V (&a)[E], V* buf, int t, const V* __restrict__ tw,
+                                          After after_first = After()) {
+  rfft_head<E, TPR, SIGN>(a, buf, t, tw, after_first);
   rpass_last_any<E, TPR, SIGN, true>(a, t, tw, [](int, V) {});
 }
 
@@ -308,6 +288,11 @@ template <> struct RLen<192> { static constexpr int E = 24, TPR = 8; };
 template <> struct RLen<384> { static constexpr int E = 24, TPR = 16; };
 template <> struct RLen<768> { static constexpr int E = 24, TPR = 32; };
 template <> struct RLen<1536> { static constexpr int E = 24, TPR = 64; };
+// lengths that the fixed-point kernels alone have
+template <> struct RLen<128> { static constexpr int E = 16, TPR = 8; };
+template <> struct RLen<256> { static constexpr int E = 16, TPR = 16; };
+template <> struct RLen<512> { static constexpr int E = 16, TPR = 32; };
+template <> struct RLen<1024> { static constexpr int E = 16, TPR = 64; };
 
 // Plans of the x-row kernel.  WREG: w's physical values stay in registers
 // next to the transform being computed (12 elements per thread, 8 for the
@@ -323,6 +308,46 @@ template <> struct XLen<96> { static constexpr int E = 12, TPR = 8; static const
 template <> struct XLen<192> { static constexpr int E = 12, TPR = 16; static constexpr bool WREG = true; };
 template <> struct XLen<384> { static constexpr int E = 12, TPR = 32; static constexpr bool WREG = true; };
 template <> struct XLen<768> { static constexpr int E = 24, TPR = 32; static constexpr bool WREG = false; };
+
+// Plans of the fixed-point x-row kernel (16-byte elements).
+template <int N> struct FxXLen;
+template <> struct FxXLen<32> { static constexpr int E = 8, TPR = 4; static constexpr bool WREG = true; };
+template <> struct FxXLen<48> { static constexpr int E = 12, TPR = 4; static constexpr bool WREG = true; };
+template <> struct FxXLen<64> { static constexpr int E = 8, TPR = 8; static constexpr bool WREG = true; };
+template <> struct FxXLen<96> { static constexpr int E = 12, TPR = 8; static constexpr bool WREG = true; };
+template <> struct FxXLen<128> { static constexpr int E = 8, TPR = 16; static constexpr bool WREG = true; };
+template <> struct FxXLen<192> { static constexpr int E = 12, TPR = 16; static constexpr bool WREG = true; };
+template <> struct FxXLen<256> { static constexpr int E = 8, TPR = 32; static constexpr bool WREG = true; };
+template <> struct FxXLen<384> { static constexpr int E = 12, TPR = 32; static constexpr bool WREG = true; };
+template <> struct FxXLen<512> { static constexpr int E = 16, TPR = 32; static constexpr bool WREG = false; };
+template <> struct FxXLen<768> { static constexpr int E = 24, TPR = 32; static constexpr bool WREG = false; };
+
+// Passes of a forward fixed-point transform at quarter scale (fx.cuh): every
+// one after the first, and inside the first of 16 and 24 points.
+__host__ __device__ constexpr int fx_quarters(int E, int TPR) {
+  return rplan_passes(E, TPR) - 1 + (fx_first_quarter(E, -1) ? 1 : 0);
+}
+// Bits of a forward transform's largest input component: with |re|, |im| <
+// 2^bits every intermediate modulus stays below 2^62 and the outputs' below
+// 2^final.  The moduli grow by the radix of each pass over the quarter
+// scale; a first pass of 24 (16) points by 3 (4), then by 8/4 (4/4).
+__host__ __device__ constexpr int fx_forward_bits(int E, int TPR, int final_bits) {
+  double g = E == 24 ? 3.0 : E == 16 ? 4.0 : (double)E;
+  double mx = g;
+  if (fx_first_quarter(E, -1)) g *= E == 24 ? 2.0 : 1.0;
+  if (g > mx) mx = g;
+  for (int p = 1; p < rplan_passes(E, TPR); ++p) {
+    g *= rplan_radix(E, TPR, p) / 4.0;
+    if (g > mx) mx = g;
+  }
+  int hm = 0, hf = 0;
+  double two = 1.0;
+  for (; two < 1.4143 * mx; two *= 2) ++hm;
+  two = 1.0;
+  for (; two < 1.4143 * g; two *= 2) ++hf;
+  const int a = 62 - hm, b = final_bits - hf;
+  return a < b ? a : b;
+}
 
 inline bool xlen_plan(int n, int* E, int* TPR) {
   switch (n) {
