@@ -76,7 +76,7 @@ template <typename L> __device__ __forceinline__ L conv(double x);
 template <typename L> __device__ __forceinline__ L conv(float x);
 template <typename L> __device__ __forceinline__ L conv(dd x);
 template <> __device__ __forceinline__ double conv<double>(double x) { return x; }
-template <> __device__ __forceinline__ double conv<double>(dd x) { return dd_to_double(x); }
+template <> __device__ __forceinline__ double conv<double>(dd x) { return dd_to_double_int(x); }
 template <> __device__ __forceinline__ dd conv<dd>(float x) { return dd(x); }
 // linear-term value stored in the history type
 template <typename OT> __device__ __forceinline__ OT store_as(double x) { return (OT)x; }
@@ -90,26 +90,39 @@ template <typename T> struct HistT { using t = typename C2<T>::t; };
 template <> struct HistT<dd> { using t = double2; };
 
 // resident 128-thread blocks per SM the registers are capped for
-template <typename T> struct RhsBlocks { static constexpr int value = 4; };
-template <> struct RhsBlocks<float> { static constexpr int value = 3; };
-template <> struct RhsBlocks<dd> { static constexpr int value = 5; };
+template <typename T> struct RhsBlocks { static constexpr int value = 3; };
 
-// RB consecutive rows per thread: the five-row windows of the products and
-// of the field slide down the rows, so each row is loaded (and, in the mixed
-// path, converted to double-float) once instead of five times.
-template <typename T, int RB>
+// rb (at most kRhsMaxRows) consecutive rows per thread: the five-row windows
+// slide down the rows,
+// so each row is loaded (and, in the mixed path, converted to
+// double-float) once instead of five times.
+//
+// FP64 and double-float: the windows hold four combinations of the six product
+// spectra, formed once per row, instead of the products:
+//   expl_v = D1 P + (D2 + k2 D0) Q,  P = k2 vv - kx^2 uu - 2 kx kz uw - kz^2 ww,  Q = i (kx uv + kz vw)
+//   expl_eta = D0 R + D1 S,          R = kx kz (uu - ww) + (kz^2 - kx^2) uw,      S = i (kx vw - kz uv)
+// (dnsdata.f90:636-640, 654 expanded; the mean mode's S = (-uv, -vw), :653),
+// and eta's linear terms act on w = i kz V1 - i kx V3.  Per mode and row: 114
+// FP64 operations where the 13 stencils of the products and the stencils of
+// V1 and V3 took 217; the FP64 pipe bounds the kernel, 80% busy (39.2 -> 23.9
+// ms per step at 255x256x255; double-float, whose linear terms are FP64, 17.4
+// -> 13.0).  The FP32 path keeps the stencils of each product and field, whose
+// FP32 rounding the mixed step's results carry.
+constexpr int kRhsMaxRows = 32;
+template <typename T>
 __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2* __restrict__ V, const typename C2<T>::t* __restrict__ VV,
                                              typename HistT<T>::t* __restrict__ old, double2* __restrict__ rhs,
                                              const typename LinT<T>::t* __restrict__ derL, const T* __restrict__ derT,
                                              Dims d, double ode1, double ode2, double ode3,
                                              const DevScalars* __restrict__ sc, const double2* __restrict__ F,
-                                             int m_lo, int m_hi) {
+                                             int m_lo, int m_hi, int rb) {
   using V2 = typename C2<T>::t;
   using O2 = typename HistT<T>::t;
   using OT = decltype(O2::x);
+  constexpr bool COMB = !std::is_same<T, float>::value;
   const int m = m_lo + blockIdx.x * blockDim.x + threadIdx.x;
-  const int iy0 = blockIdx.y * RB + 1;
-  const int nrows = min(RB, d.ny - iy0);
+  const int iy0 = blockIdx.y * rb + 1;
+  const int nrows = min(rb, d.ny - iy0);
   // ---- linear terms of the field in L (FP64, or double-float in the mixed
   //      path: the FP64 pipe is 1/58 of FP32 here) ----
   // The reference evaluates unkn and impl as separate stencils and combines
@@ -120,12 +133,12 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   //   lambda (S2 - k2 S0) + ni (S4 - 2 k2 S2 + k2^2 S0) = sum_j (A_j + k2 B_j + k2^2 C_j) V2_j
   // and for eta (:658) with w = i kz V1 - i kx V3
   //   lambda S0(w) + ni (S2(w) - k2 S0(w)) = sum_j (D_j + k2 E_j) w_j,
-  // the mean mode (:653) being the k2 = 0 case on (U, W).  The per-row
+  // the mean mode (:653) being the k2 = 0 case on w = (U, W).  The per-row
   // coefficients A..E are formed once per block and row.
   using L = typename LinT<T>::t;
   using LV = typename C2<L>::t;
   const size_t tailL = (size_t)(d.ny + 1) * 20;  // der rows, then alfa0, beta0, ni
-  __shared__ __align__(16) unsigned char cf_raw[RB * 25 * sizeof(L)];
+  __shared__ __align__(16) unsigned char cf_raw[kRhsMaxRows * 25 * sizeof(L)];
   L* cf = reinterpret_cast<L*>(cf_raw);
   for (int t = threadIdx.x; t < 5 * nrows; t += blockDim.x) {
     const int j = t % 5, rr = t / 5;
@@ -144,6 +157,7 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   if (m >= m_hi) return;
   const int ix = m / d.nzt;
   const int iz = m - ix * d.nzt - d.nz;
+  const bool mean = ix == 0 && iz == 0;
   // wavenumbers (derT holds der in T, then alfa0, beta0; derL likewise in L, then ni)
   const size_t tail = (size_t)(d.ny + 1) * 20;
   const T ta = T((float)ix) * derT[tail], tb = T((float)iz) * derT[tail + 1];
@@ -151,6 +165,9 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   const L a = L((float)ix) * derL[tailL], b = L((float)iz) * derL[tailL + 1];
   const L k2 = a * a + b * b;
   const L lode2 = Num<L>::from_double(ode2), lode3 = Num<L>::from_double(ode3);
+  // coefficients of P and R
+  const T taa = COMB ? ta * ta : T(), tbb = COMB ? tb * tb : T(), tab = COMB ? ta * tb : T();
+  const T tab2 = tab + tab, tba = COMB ? tbb - taa : T();
   // STAGED (FP32 path): the next D rows' products (plane iy+3), field rows
   // iy+2 and RK history at iy are copied into a per-thread ring in shared
   // memory while the current row is computed (cp.async), instead of loaded
@@ -182,53 +199,78 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
       cp_async_commit();
     }
   };
-  // windows over rows iy-2..iy+2: the six product spectra (plane = row + 1) and the field
-  V2 vv[6][5];
-  LV v1[5], v2[5], v3[5];
+  // windows over rows iy-2..iy+2: the six product spectra (plane = row + 1)
+  // or their combinations P, Q, R, S, and the field as V2 and w
+  constexpr int NW = COMB ? 4 : 6;
+  V2 vv[NW][5];
+  LV v2[5], w[5], v3[COMB ? 1 : 5];  // w: V1 in the FP32 path
+  auto put_products = [&](int j, const V2 (&p)[6]) {
+    if constexpr (COMB) {  // uu, vv, ww, uv, vw, uw
+      vv[0][j] = mk<V2>(fmaT(tk2, p[1].x, fmaT(-taa, p[0].x, fmaT(-tab2, p[5].x, -(tbb * p[2].x)))),
+                        fmaT(tk2, p[1].y, fmaT(-taa, p[0].y, fmaT(-tab2, p[5].y, -(tbb * p[2].y)))));
+      vv[1][j] = mk<V2>(-fmaT(ta, p[3].y, tb * p[4].y), fmaT(ta, p[3].x, tb * p[4].x));
+      vv[2][j] = mk<V2>(fmaT(tab, p[0].x - p[2].x, tba * p[5].x), fmaT(tab, p[0].y - p[2].y, tba * p[5].y));
+      vv[3][j] = mean ? mk<V2>(-p[3].x, -p[4].x)
+                      : mk<V2>(fmaT(tb, p[3].y, -(ta * p[4].y)), fmaT(ta, p[4].x, -(tb * p[3].x)));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) vv[k][j] = p[k];
+    }
+  };
+  auto put_field = [&](int j, double2 f1, double2 f2, double2 f3) {
+    v2[j] = cvt2<LV>(f2);
+    const LV u = cvt2<LV>(f1), z = cvt2<LV>(f3);
+    if constexpr (COMB) {
+      w[j] = mean ? mk<LV>(u.x, z.x) : mk<LV>(fmaT(a, z.y, -(b * u.y)), fmaT(-a, z.x, b * u.x));
+    } else {
+      w[j] = u;
+      v3[j] = z;
+    }
+  };
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
+    V2 p[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) vv[k][j + 1] = VV[((size_t)k * d.nplanes + (iy0 - 1 + j)) * d.nmodes + m];
-    v1[j + 1] = cvt2<LV>(V[vidx(d, 0, iy0 - 2 + j, m)]);
-    v2[j + 1] = cvt2<LV>(V[vidx(d, 1, iy0 - 2 + j, m)]);
-    v3[j + 1] = cvt2<LV>(V[vidx(d, 2, iy0 - 2 + j, m)]);
+    for (int k = 0; k < 6; ++k) p[k] = VV[((size_t)k * d.nplanes + (iy0 - 1 + j)) * d.nmodes + m];
+    put_products(j + 1, p);
+    put_field(j + 1, V[vidx(d, 0, iy0 - 2 + j, m)], V[vidx(d, 1, iy0 - 2 + j, m)], V[vidx(d, 2, iy0 - 2 + j, m)]);
   }
 #pragma unroll
   for (int q = 0; q < D; ++q) stage(q);
 #pragma unroll 1
-  for (int rr = 0; rr < RB; ++rr) {
-  if (rr >= nrows) break;
+  for (int rr = 0; rr < nrows; ++rr) {
   const int iy = iy0 + rr;
   const L* cfr = cf + rr * 25;
   // slide the windows one row down and load row iy+2
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
 #pragma unroll
-    for (int k = 0; k < 6; ++k) vv[k][j] = vv[k][j + 1];
-    v1[j] = v1[j + 1];
+    for (int k = 0; k < NW; ++k) vv[k][j] = vv[k][j + 1];
     v2[j] = v2[j + 1];
-    v3[j] = v3[j + 1];
+    w[j] = w[j + 1];
+    if constexpr (!COMB) v3[j] = v3[j + 1];
   }
   O2 o_eta, o_d2v;  // RK history at this row
   if constexpr (STAGED) {
     cp_async_wait<D - 1>();  // this row's group has landed
     const int s = rr % (D + 1);
+    V2 p[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) vv[k][4] = *s_vv(s, k);
-    v1[4] = cvt2<LV>(*s_v(s, 0));
-    v2[4] = cvt2<LV>(*s_v(s, 1));
-    v3[4] = cvt2<LV>(*s_v(s, 2));
+    for (int k = 0; k < 6; ++k) p[k] = *s_vv(s, k);
+    put_products(4, p);
+    put_field(4, *s_v(s, 0), *s_v(s, 1), *s_v(s, 2));
     o_eta = *s_old(s, 0);
     o_d2v = *s_old(s, 1);
     stage(rr + D);  // into the slot of row rr-1, already read
   } else {
+    V2 p[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) vv[k][4] = VV[((size_t)k * d.nplanes + (iy + 3)) * d.nmodes + m];
-    v1[4] = cvt2<LV>(V[vidx(d, 0, iy + 2, m)]);
-    v2[4] = cvt2<LV>(V[vidx(d, 1, iy + 2, m)]);
-    v3[4] = cvt2<LV>(V[vidx(d, 2, iy + 2, m)]);
+    for (int k = 0; k < 6; ++k) p[k] = VV[((size_t)k * d.nplanes + (iy + 3)) * d.nmodes + m];
+    const double2 f1 = V[vidx(d, 0, iy + 2, m)], f2 = V[vidx(d, 1, iy + 2, m)], f3 = V[vidx(d, 2, iy + 2, m)];
     o_eta = old[((size_t)0 * (d.ny - 1) + (iy - 1)) * d.nmodes + m];
     o_d2v = old[((size_t)1 * (d.ny - 1) + (iy - 1)) * d.nmodes + m];
+    put_products(4, p);
+    put_field(4, f1, f2, f3);
   }
   // stencil coefficients of this row in T
   const T* drT = derT + (size_t)iy * 20;
@@ -239,30 +281,47 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
     e1[j] = drT[5 + j];
     e2[j] = drT[10 + j];
   }
-  // DD(f,k) (dnsdata.f90:609-610) on product k (0-based) at rows iy-2..iy+2
+  // DD(f,k) (dnsdata.f90:609-610) on window k at rows iy-2..iy+2
   auto DD = [&](const T* c, int k) -> V2 {
     V2 s = mk<V2>(c[0] * vv[k][0].x, c[0] * vv[k][0].y);
 #pragma unroll
     for (int j = 1; j < 5; ++j) s = s + mk<V2>(c[j] * vv[k][j].x, c[j] * vv[k][j].y);
     return s;
   };
-  const V2 DD0_6 = DD(e0, 5), DD1_6 = DD(e1, 5);
-  // rhsu = -i ta DD0(uu) - DD1(uv) - i tb DD0(uw) (dnsdata.f90:636-638), and
-  // rhsv, rhsw alike: with i a z = (-a z.y, a z.x), each component two
-  // fused multiply-adds (a leading 0 - ... would block the fusion)
-  auto rhs3 = [&](V2 X, V2 Y, V2 Z) {
-    return mk<V2>(fmaT(tb, Z.y, fmaT(ta, X.y, -Y.x)), fmaT(-tb, Z.x, fmaT(-ta, X.x, -Y.y)));
-  };
-  const V2 rhsu = rhs3(DD(e0, 0), DD(e1, 3), DD0_6);
-  const V2 rhsv = rhs3(DD(e0, 3), DD(e1, 1), DD(e0, 4));
-  const V2 rhsw = rhs3(DD0_6, DD(e1, 4), DD(e0, 2));
-  // expl_v = i ta (i ta D1uu + D2uv + i tb D1uw) + i tb (i ta D1uw + D2vw + i tb D1ww) - k2 rhsv (:639-640)
-  auto ia_sum = [&](V2 X, V2 Y, V2 Z) {  // i ta X + Y + i tb Z
-    return mk<V2>(fmaT(-tb, Z.y, fmaT(-ta, X.y, Y.x)), fmaT(tb, Z.x, fmaT(ta, X.x, Y.y)));
-  };
-  const V2 in1 = ia_sum(DD(e1, 0), DD(e2, 3), DD1_6), in2 = ia_sum(DD1_6, DD(e2, 4), DD(e1, 2));
-  const V2 explv = mk<V2>(fmaT(-tk2, rhsv.x, fmaT(-ta, in1.y, -(tb * in2.y))),
-                          fmaT(-tk2, rhsv.y, fmaT(ta, in1.x, tb * in2.x)));
+  V2 explv, ee;  // the explicit terms of D2v and eta (of the mean mode: U, W without the pressure gradient)
+  if constexpr (COMB) {
+    auto axpy = [&](V2 s, const T* c, int k) -> V2 {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) s = mk<V2>(fmaT(c[j], vv[k][j].x, s.x), fmaT(c[j], vv[k][j].y, s.y));
+      return s;
+    };
+    T e20[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) e20[j] = fmaT(tk2, e0[j], e2[j]);
+    explv = axpy(DD(e1, 0), e20, 1);
+    ee = axpy(DD(e0, 2), e1, 3);
+  } else {
+    const V2 DD0_6 = DD(e0, 5), DD1_6 = DD(e1, 5);
+    // rhsu = -i ta DD0(uu) - DD1(uv) - i tb DD0(uw) (dnsdata.f90:636-638), and
+    // rhsv, rhsw alike: with i a z = (-a z.y, a z.x), each component two
+    // fused multiply-adds (a leading 0 - ... would block the fusion)
+    auto rhs3 = [&](V2 X, V2 Y, V2 Z) {
+      return mk<V2>(fmaT(tb, Z.y, fmaT(ta, X.y, -Y.x)), fmaT(-tb, Z.x, fmaT(-ta, X.x, -Y.y)));
+    };
+    const V2 rhsu = rhs3(DD(e0, 0), DD(e1, 3), DD0_6);
+    const V2 rhsv = rhs3(DD(e0, 3), DD(e1, 1), DD(e0, 4));
+    const V2 rhsw = rhs3(DD0_6, DD(e1, 4), DD(e0, 2));
+    // expl_v = i ta (i ta D1uu + D2uv + i tb D1uw) + i tb (i ta D1uw + D2vw + i tb D1ww) - k2 rhsv (:639-640)
+    auto ia_sum = [&](V2 X, V2 Y, V2 Z) {  // i ta X + Y + i tb Z
+      return mk<V2>(fmaT(-tb, Z.y, fmaT(-ta, X.y, Y.x)), fmaT(tb, Z.x, fmaT(ta, X.x, Y.y)));
+    };
+    const V2 in1 = ia_sum(DD(e1, 0), DD(e2, 3), DD1_6), in2 = ia_sum(DD1_6, DD(e2, 4), DD(e1, 2));
+    explv = mk<V2>(fmaT(-tk2, rhsv.x, fmaT(-ta, in1.y, -(tb * in2.y))),
+                   fmaT(-tk2, rhsv.y, fmaT(ta, in1.x, tb * in2.x)));
+    // i tb rhsu - i ta rhsw (:654); the mean flow U + iW (:648-654)
+    ee = mean ? mk<V2>(rhsu.x, rhsw.x)
+              : mk<V2>(fmaT(ta, rhsw.y, -(tb * rhsu.y)), fmaT(-ta, rhsw.x, tb * rhsu.x));
+  }
   // body-force terms (dnsdata.f90:644, 651, 658): fv for the v equation,
   // fe for eta (or the mean mode's D0 of Re F1, Re F3)
   LV fv = czero<LV>(), fe = czero<LV>();
@@ -284,7 +343,7 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
       r3 = r3 + c0 * f3.x;
     }
     fv = czero<LV>() - lmul(k2, D0f2) - mul_ia<LV>(a, D1f1) - mul_ia<LV>(b, D1f3);
-    fe = (ix == 0 && iz == 0) ? mk<LV>(r1, r3) : mul_ia<LV>(b, D0f1) - mul_ia<LV>(a, D0f3);
+    fe = mean ? mk<LV>(r1, r3) : mul_ia<LV>(b, D0f1) - mul_ia<LV>(a, D0f3);
   }
   const size_t r0 = ((size_t)0 * (d.ny - 1) + (iy - 1)) * d.nmodes + m;  // eta
   const size_t r1 = ((size_t)1 * (d.ny - 1) + (iy - 1)) * d.nmodes + m;  // d2v
@@ -300,36 +359,26 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
     old[r1] = mk<O2>(store_as<OT>(e.x), store_as<OT>(e.y));
     rhs[r1] = make_double2(Num<L>::to_double(r.x), Num<L>::to_double(r.y));
   }
-  if (ix == 0 && iz == 0) {  // mean flow U + iW (:648-654)
-    LV e = mk<LV>(conv<L>(rhsu.x) + Num<L>::from_double(sc->meanpx),
-                  conv<L>(rhsw.x) + Num<L>::from_double(sc->meanpz));
-    if (F) e = e + fe;
-    L su = cfr[15] * v1[0].x, sw = cfr[15] * v3[0].x;
+  {  // eta and the mean flow (:648-661): unkn = D0(w), impl = ni (D2(w) - k2 D0(w))
+    LV r;
+    if constexpr (COMB) {
+      r = lmul(cfr[15] + k2 * cfr[20], w[0]);
 #pragma unroll
-    for (int j = 1; j < 5; ++j) {
-      su = su + cfr[15 + j] * v1[j].x;
-      sw = sw + cfr[15 + j] * v3[j].x;
-    }
-    LV r = mk<LV>(su, sw);
-    const O2 o = o_eta;
-    r = r + lmul(lode2, e);
-    r = r - lmul(lode3, mk<LV>(conv<L>(o.x), conv<L>(o.y)));
-    old[r0] = mk<O2>(store_as<OT>(e.x), store_as<OT>(e.y));
-    rhs[r0] = make_double2(Num<L>::to_double(r.x), Num<L>::to_double(r.y));
-  } else {  // eta (:656-661): with w = i kz V1 - i kx V3, unkn = D0(w), impl = ni (D2(w) - k2 D0(w))
-    // i tb rhsu - i ta rhsw (:654)
-    const V2 ee = mk<V2>(fmaT(ta, rhsw.y, -(tb * rhsu.y)), fmaT(-ta, rhsw.x, tb * rhsu.x));
-    L nj = cfr[15] + k2 * cfr[20];
-    LV s1 = lmul(nj, v1[0]), s3 = lmul(nj, v3[0]);
+      for (int j = 1; j < 5; ++j) r = r + lmul(cfr[15 + j] + k2 * cfr[20 + j], w[j]);
+    } else {
+      L nj = cfr[15] + k2 * cfr[20];
+      LV s1 = lmul(nj, w[0]), s3 = lmul(nj, v3[0]);
 #pragma unroll
-    for (int j = 1; j < 5; ++j) {
-      nj = cfr[15 + j] + k2 * cfr[20 + j];
-      s1 = s1 + lmul(nj, v1[j]);
-      s3 = s3 + lmul(nj, v3[j]);
+      for (int j = 1; j < 5; ++j) {
+        nj = cfr[15 + j] + k2 * cfr[20 + j];
+        s1 = s1 + lmul(nj, w[j]);
+        s3 = s3 + lmul(nj, v3[j]);
+      }
+      r = mean ? mk<LV>(s1.x, s3.x) : mk<LV>(fmaT(a, s3.y, -(b * s1.y)), fmaT(-a, s3.x, b * s1.x));  // i kz s1 - i kx s3
     }
-    LV r = mk<LV>(fmaT(a, s3.y, -(b * s1.y)), fmaT(-a, s3.x, b * s1.x));  // i kz s1 - i kx s3
     const O2 o = o_eta;
     LV e = mk<LV>(conv<L>(ee.x), conv<L>(ee.y));
+    if (mean) e = e + mk<LV>(Num<L>::from_double(sc->meanpx), Num<L>::from_double(sc->meanpz));
     if (F) e = e + fe;
     r = r + lmul(lode2, e);
     r = r - lmul(lode3, mk<LV>(conv<L>(o.x), conv<L>(o.y)));
@@ -339,21 +388,45 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   }  // rows
 }
 
-// rows per thread: several where the kernel waits on loads (the FP32 path),
-// one where the FP64 pipe binds it and registers are dear
-template <typename T> struct RhsRows { static constexpr int value = 1; };
-template <> struct RhsRows<float> { static constexpr int value = 16; };
+// Rows per thread: the count that minimises the time of the fullest of 152
+// SMs, three blocks at a time.  A block's time is its rows plus the four
+// start-up rows of the windows (1 row's worth; 2 in the FP32 path, which
+// waits on their loads); three resident blocks take 3 units a row, one or two
+// kRhsPart (measured at 32x64x32 and 47x96x47: the FP64 pipe is nearly
+// filled by one block, the FP32 path's latency is not).  Against a fixed 16:
+// FP64 0.285 -> 0.157 ms a step at 32x64x32, 0.487 -> 0.382 at 47x96x47,
+// 1.29 -> 1.06 at 79x101x75; mixed 0.138 -> 0.067, 0.184 -> 0.136, 0.35 -> 0.30.
+template <typename T> struct RhsPart { static constexpr double one = 1.6, two = 2.4; };
+template <> struct RhsPart<double> { static constexpr double one = 1.25, two = 2.1; };
+template <> struct RhsPart<float> { static constexpr double one = 1.95, two = 2.6; };
+template <typename T>
+int rhs_rows(int modes, int ny) {
+  const int cols = (modes + 127) / 128;
+  const int start = std::is_same<T, float>::value ? 2 : 1;
+  int best = kRhsMaxRows;
+  double cost = 1e300;
+  for (int rb = kRhsMaxRows; rb >= 2; --rb) {
+    const long long blocks = (long long)cols * ((ny - 1 + rb - 1) / rb), per_sm = (blocks + 151) / 152;
+    const int part = (int)(per_sm % 3);
+    const double units = 3.0 * (double)(per_sm / 3) + (part == 1 ? RhsPart<T>::one : part == 2 ? RhsPart<T>::two : 0.0);
+    if (units * (rb + start) < cost) {
+      cost = units * (rb + start);
+      best = rb;
+    }
+  }
+  return best;
+}
 
 template <typename T>
 void launch_rhs(const SolveLaunch& L, cudaStream_t s) {
   using V2 = typename C2<T>::t;
   using O2 = typename HistT<T>::t;
-  constexpr int RB = RhsRows<T>::value;
-  if (L.m_hi <= L.m_lo) return;
-  dim3 grid((L.m_hi - L.m_lo + 127) / 128, (L.d.ny - 1 + RB - 1) / RB);
   using LT = typename LinT<T>::t;
-  k_rhs<T, RB><<<grid, 128, 0, s>>>(L.V, (const V2*)L.VV, (O2*)L.old, L.rhs, (const LT*)L.derL, (const T*)L.derT, L.d,
-                                L.ode[0], L.ode[1], L.ode[2], L.sc, L.F, L.m_lo, L.m_hi);
+  if (L.m_hi <= L.m_lo) return;
+  const int rb = rhs_rows<T>(L.m_hi - L.m_lo, L.d.ny);
+  dim3 grid((L.m_hi - L.m_lo + 127) / 128, (L.d.ny - 1 + rb - 1) / rb);
+  k_rhs<T><<<grid, 128, 0, s>>>(L.V, (const V2*)L.VV, (O2*)L.old, L.rhs, (const LT*)L.derL, (const T*)L.derT, L.d,
+                                L.ode[0], L.ode[1], L.ode[2], L.sc, L.F, L.m_lo, L.m_hi, rb);
 }
 template void launch_rhs<double>(const SolveLaunch&, cudaStream_t);
 template void launch_rhs<float>(const SolveLaunch&, cudaStream_t);
