@@ -68,7 +68,7 @@ struct chgpu_handle {
   // k_factor runs beside the FP32 / memory-bound transforms and k_rhs; 4: the
   // factorisation ahead as in 3, the substitutions by the fused kernel's two
   // threads per pair reading the factors; 5: the factorisation ahead, the
-  // substitutions with eight threads per pair (k_solve_ri: one per system,
+  // substitutions with eight threads per pair (k_solve<true>: one per system,
   // mode and real / imaginary component)
   int solve_form = 1;
   cudaStream_t stream2 = nullptr, stream3 = nullptr;
@@ -739,6 +739,15 @@ extern "C" {
 
 const char* chgpu_last_error(const chgpu_handle* h) { return h ? h->err.c_str() : g_create_error.c_str(); }
 
+namespace {
+// Solve form of a handle that has not been tuned: eight threads per pair
+// while its blocks are one wave (16 pairs per 128-thread block, four blocks
+// on each of 152 SMs; ms per mixed step against four threads per pair:
+// 32x64x32 0.51 / 0.66, 47x96x47 1.07 / 1.28, 83x120x85 2.70 / 2.83, but
+// 127x192x127 6.97 / 6.45), then four threads, then the fused kernel
+int default_solve_form(int pairs) { return pairs <= 16 * 4 * 152 ? 5 : pairs < 65536 ? 3 : 1; }
+}  // namespace
+
 int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   if (!p || !out) return fail(nullptr, CHGPU_E_PARAM, "chgpu_create: null argument");
   *out = nullptr;
@@ -793,7 +802,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     h->xfast = xplan(h->prec, nxd, &e_, &tpr_);
   }
   h->halves = d.npairs >= 65536 ? 2 : 1;
-  h->solve_form = d.npairs < 65536 ? 3 : 1;
+  h->solve_form = default_solve_form(d.npairs);
   h->rz.n = rz.n; h->rz.nst = rz.nst; std::memcpy(h->rz.r, rz.r, sizeof rz.r);
   h->rx.n = rx.n; h->rx.nst = rx.nst; std::memcpy(h->rx.r, rx.r, sizeof rx.r);
   set_twiddle_offsets(h->rz);
@@ -1189,6 +1198,13 @@ int chgpu_ensemble_create(const chgpu_params* params, int n, chgpu_ensemble** ou
       return ens_fail(nullptr, rc, msg);
     }
   }
+  // the members share the GPU: their solve form is that of their pairs
+  // together (64 minimal channels, 42 472 pairs, mixed: 8.7 ms per step with
+  // four threads per pair, 10.3 with the eight that each would take alone)
+  long long pairs = 0;
+  for (chgpu_handle* h : e->m) pairs += h->d.npairs;
+  const int form = default_solve_form((int)std::min<long long>(pairs, 65535));
+  for (chgpu_handle* h : e->m) h->solve_form = std::min(h->solve_form, form);
   cudaError_t c = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   if (c == cudaSuccess) c = cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming);
   for (int i = 0; i < n && c == cudaSuccess; ++i) c = cudaEventCreateWithFlags(&e->join[i], cudaEventDisableTiming);

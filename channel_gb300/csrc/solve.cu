@@ -1060,6 +1060,38 @@ __global__ void __launch_bounds__(64, 8) k_factor(double* __restrict__ fac, cons
   }
 }
 
+// ---------------------------------------------------------------------------
+// k_solve: the substitutions with the factors of k_factor, then v' and u, w.
+//
+// RI false: four threads per pair (kx, +-kz), one per (system, mode): warp 0
+// (v, +kz), warp 1 (v, -kz), warp 2 (eta, +kz), warp 3 (eta, -kz), a lane per
+// pair.  RI true: eight, one per (system, mode, component): the systems'
+// coefficients are real, so the real and imaginary parts of every recurrence
+// are independent and run the same operations; lane l takes pair l/2 of the
+// block's 16 and component l%2, and only the u, w recovery exchanges the
+// components, by a shuffle.  The results are bit-identical.
+//
+//   1. LeftLU5divStep1 bottom-up and LeftLU5divStep2 top-down
+//      (rbparmat_blocking.f90:57-100), then the wall and ghost values
+//      (linsolve_blocking.inc:50-61); the (eta, -kz) thread of the mean pair,
+//      whose mode does not exist, solves the unit-forcing response (:62-68).
+//   2. COMPLEXderiv's right-hand sides, the d1 stencil of v with the
+//      one-sided wall derivatives folded in (dnsdata.f90:339-364), parked in
+//      the field's w slot: no recurrence, so all warps take rows, NP parts of
+//      them per mode.
+//   3. Both sweeps of D0mat (dnsdata.f90:365-373) by warps 0 and 1, while the
+//      mean pair's eta warp makes the mean-flow correction
+//      (linsolve_blocking.inc:62-97).
+//   4. u, w (:99-103), rows in parts again.
+//
+// What bounds it: the latency of the four sweeps in few warps.  Four fifths of
+// the instructions are the stencil and the recovery (45 k per warp at
+// 47x96x47 mixed, 6 cycles each when one warp per scheduler ran them inside
+// its sweeps); shared by all warps, outside the recurrences, the mixed step
+// went from 0.64 to 0.51 ms at 32x64x32 and from 1.23 to 1.07 at 47x96x47.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int kAhead = 4;
 // L1 prefetch of a line the thread will load some rows later (no register
 // is held for it); every address passed is inside its buffer
 __device__ __forceinline__ void prefetch_l1(const void* p) {
@@ -1067,305 +1099,197 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
 }
 constexpr int kSolvePrefetch = 6;  // rows ahead
 
-// k_solve: four threads per pair, one per (system, mode): warp 0 (v, +kz),
-// warp 1 (v, -kz), warp 2 (eta, +kz), warp 3 (eta, -kz).  The (eta, -kz)
-// thread of the mean pair, whose mode does not exist, solves the mean
-// mode's unit-forcing response instead.  Each: LeftLU5divStep1 bottom-up and
-// LeftLU5divStep2 top-down with the factors of k_factor (rbparmat_blocking.f90:
-// 57-100), then the wall and ghost values (linsolve_blocking.inc:50-61).
-// After a block barrier the mean pair's eta thread makes the mean-flow
-// correction (:62-97), and warps 0 and 1 take v' and the u, w recovery of
-// the +kz and -kz modes (:99-103).
-__global__ void __launch_bounds__(128, 4) k_solve(double2* __restrict__ V, const double2* rhs, size_t rcs, int roff,
-                                                  const double* __restrict__ fac, const double* __restrict__ der,
-                                                  const double* __restrict__ d0lu, const double* __restrict__ yint,
-                                                  BcRows bc, Dims d, DevScalars* __restrict__ sc,
-                                                  const dd* __restrict__ lindd, int q_lo, int q_hi) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int sys = w >> 1, t = w & 1;
-  const int q = q_lo + blockIdx.x * 32 + lane;
-  const bool active = q < q_hi;
-  const int ny = d.ny, nz = d.nz;
-  const int ix = active ? q / (nz + 1) : 0;
-  const int a = active ? q - ix * (nz + 1) : 0;
-  const int nm = (a == 0) ? 1 : 2;
-  int mm[2];
-  mm[0] = ix * d.nzt + nz + a;
-  mm[1] = ix * d.nzt + nz - a;
-  const bool is00 = (ix == 0 && a == 0);
-  const double ka = ix * d.alfa0, kb = a * d.beta0;
-  const double k2 = ka * ka + kb * kb;
-  const double ni = d.ni;
-  const size_t P = d.npairs;
-  const bool ucor = active && is00 && sys == 1 && t == 1;  // unit-forcing response (linsolve_blocking.inc:62-68)
-  const bool mine = active && t < nm;
-  const int m = mm[ucor ? 0 : t];
-  const int vc = ucor ? 2 : (sys == 0 ? 1 : 0);  // field slot written
-  const bool wallrhs = mine && sys == 1 && is00;
-  double bot[5], botm1[5], top[5], topp1[5];
-#pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    bot[j] = sys ? bc.eta0bc[j] : bc.v0bc[j];
-    botm1[j] = sys ? bc.eta0m1bc[j] : bc.v0m1bc[j];
-    top[j] = sys ? bc.etanbc[j] : bc.vnbc[j];
-    topp1[j] = sys ? bc.etanp1bc[j] : bc.vnp1bc[j];
-  }
-  const double bval0 = wallrhs ? sc->u0 : 0.0, bvaln = wallrhs ? sc->uN : 0.0;
-  if (mine || ucor) {
-    const double* fs = fac + (size_t)5 * sys * P + q;  // this system's factors of row 1
-    const size_t frow = (size_t)kFacPerRow * P;
-    // ---- Step1 bottom-up: x = (b - u1 x(+1) - u2 x(+2)) / d ----
-    const double2* rsrc = rhs + (sys == 0 ? rcs : 0);
-    double2 x1 = cz(), x2 = cz();
-    double2 bn = ucor ? make_double2(1.0, 0.0) : rsrc[(size_t)(ny - 1 + roff) * d.nmodes + m];
-    const double* f = fs + (size_t)(ny - 2) * frow;
-    double dn = f[2 * P], u1n = f[3 * P], u2n = f[4 * P];
-    for (int iy = ny - 1; iy >= 1; --iy) {
-      double2 b = bn;
-      const double dv = dn, u1 = u1n, u2 = u2n;
-      if (iy > 1) {  // one row ahead (global-load latency)
-        if (!ucor) bn = rsrc[(size_t)(iy - 1 + roff) * d.nmodes + m];
-        f -= frow;
-        dn = f[2 * P];
-        u1n = f[3 * P];
-        u2n = f[4 * P];
-      }
-      if (iy - kSolvePrefetch >= 1) {  // and the lines of a row further down
-        const double* fp = f - (size_t)(kSolvePrefetch - 1) * frow;
-        prefetch_l1(fp + 2 * P);
-        prefetch_l1(fp + 3 * P);
-        prefetch_l1(fp + 4 * P);
-        if (!ucor) prefetch_l1(rsrc + (size_t)(iy - kSolvePrefetch + roff) * d.nmodes + m);
-      }
-      if (wallrhs) {
-        if (iy == 1) b = b - make_double2(sc->wallrhs[0], sc->wallrhs[1]);
-        if (iy == 2) b = b - make_double2(sc->wallrhs[2], sc->wallrhs[3]);
-        if (iy == ny - 2) b = b - make_double2(sc->wallrhs[4], sc->wallrhs[5]);
-        if (iy == ny - 1) b = b - make_double2(sc->wallrhs[6], sc->wallrhs[7]);
-      }
-      const double2 x = step1u(b, dv, u1, u2, x1, x2);
-      x2 = x1;
-      x1 = x;
-      V[vidx(d, vc, iy, m)] = x;
-    }
-    // ---- Step2 top-down: v = x - l2 v(-2) - l1 v(-1); rows 1..3 and ny-3..ny-1 kept ----
-    double2 lo[3], hi[3];
-    double2 m2 = cz(), m1 = cz();
-    f = fs;
-    double l2n = f[0], l1n = f[P];
-    double2 vn = V[vidx(d, vc, 1, m)];
-    for (int iy = 1; iy <= ny - 1; ++iy) {
-      const double l2 = l2n, l1 = l1n;
-      const double2 vcur = vn;
-      if (iy < ny - 1) {
-        f += frow;
-        l2n = f[0];
-        l1n = f[P];
-        vn = V[vidx(d, vc, iy + 1, m)];
-      }
-      if (iy + kSolvePrefetch <= ny - 1) {
-        const double* fp = f + (size_t)(kSolvePrefetch - 1) * frow;
-        prefetch_l1(fp);
-        prefetch_l1(fp + P);
-        prefetch_l1(&V[vidx(d, vc, iy + kSolvePrefetch, m)]);
-      }
-      const double2 nv = step2(vcur, l2, l1, m2, m1);
-      V[vidx(d, vc, iy, m)] = nv;
-      m2 = m1;
-      m1 = nv;
-      if (iy == 1) lo[0] = nv;
-      if (iy == 2) lo[1] = nv;
-      if (iy == 3) lo[2] = nv;
-      if (iy == ny - 3) hi[0] = nv;
-      if (iy == ny - 2) hi[1] = nv;
-      if (iy == ny - 1) hi[2] = nv;
-    }
-    // wall and ghost values (linsolve_blocking.inc:50-61)
-    const double2 w0 = cdivr(make_double2(bval0, 0.0) - dot3(lo, bot + 2), bot[1]);
-    const double2 rb[4] = {w0, lo[0], lo[1], lo[2]};
-    const double2 wm1 = cdivr(cz() - dot4(rb, botm1 + 1), botm1[0]);
-    const double2 wn = cdivr(make_double2(bvaln, 0.0) - dot3(hi, top), top[3]);
-    const double2 rt[4] = {hi[0], hi[1], hi[2], wn};
-    const double2 wn1 = cdivr(cz() - dot4(rt, topp1), topp1[4]);
-    V[vidx(d, vc, -1, m)] = wm1;
-    V[vidx(d, vc, 0, m)] = w0;
-    V[vidx(d, vc, ny, m)] = wn;
-    V[vidx(d, vc, ny + 1, m)] = wn1;
-  }
-  __syncthreads();  // v, eta (and the unit response) of this block's pairs are in V
-  if (wallrhs) {  // mean flow (linsolve_blocking.inc:62-97)
-    // flow rates by the non-uniform Simpson rule (dnsdata.f90:312-324)
-    double fu = 0.0, fw = 0.0, fc = 0.0;
-    for (int iy = 1, k = 0; iy <= ny - 1; iy += 2, ++k) {
-      const double a1 = yint[3 * k], a2 = yint[3 * k + 1], a3 = yint[3 * k + 2];
-      const double2 e0 = V[vidx(d, 0, iy - 1, m)], e1 = V[vidx(d, 0, iy, m)], e2 = V[vidx(d, 0, iy + 1, m)];
-      const double2 u0 = V[vidx(d, 2, iy - 1, m)], u1 = V[vidx(d, 2, iy, m)], u2 = V[vidx(d, 2, iy + 1, m)];
-      fu = fu + a1 * e0.x + a2 * e1.x + a3 * e2.x;
-      fw = fw + a1 * e0.y + a2 * e1.y + a3 * e2.y;
-      fc = fc + a1 * u0.x + a2 * u1.x + a3 * u2.x;
-    }
-    double corrpx = sc->corrpx, corrpz = sc->corrpz;
-    const bool cx = fabs(d.meanflowx) > 1.0e-7 && !d.cpi;
-    const bool cz_ = fabs(d.meanflowz) > 1.0e-7 && !d.cpi;
-    if (cx) corrpx = (d.meanflowx - fu) / fc;
-    if (cz_) corrpz = (d.meanflowz - fw) / fc;
-    for (int iy = -1; iy <= ny + 1; ++iy) {
-      const double2 et = V[vidx(d, 0, iy, m)];
-      const double uc = V[vidx(d, 2, iy, m)].x;
-      double U = et.x, W = et.y;
-      if (cx) U = U + corrpx * uc;
-      if (cz_) W = W + corrpz * uc;
-      V[vidx(d, 0, iy, m)] = make_double2(U, 0.0);
-      V[vidx(d, 2, iy, m)] = make_double2(W, 0.0);
-    }
-    sc->fr[0] = fu; sc->fr[1] = fw; sc->fr[2] = fc;
-    sc->corrpx = corrpx; sc->corrpz = corrpz;
-    if (d.cpi) {
-      if (d.cpi_type == 0) sc->meanpx = (1 - d.gamma) * 6 * ni / fu;
-      else sc->meanpx = (1.5 / d.gamma) * fu * ni;
-    }
-  }
-  if (!active || is00 || sys != 0 || t >= nm) return;
-  if (lindd) deriv_uw<dd>(V, der, d0lu, lindd, bc, d, mm[t], ka, (t == 0 ? 1.0 : -1.0) * kb, k2);
-  else deriv_uw<double>(V, der, d0lu, lindd, bc, d, mm[t], ka, (t == 0 ? 1.0 : -1.0) * kb, k2);
-}
-
-// ---------------------------------------------------------------------------
-// The substitutions with eight threads per (kx, +-kz) pair: the systems'
-// coefficients are real, so the real and imaginary parts of every
-// recurrence are independent and each (system, mode) thread of k_solve
-// splits into two, one per component, with the same operations on each (the
-// results are bit-identical to k_solve's).  Twice the warps for a kernel
-// whose y recurrences are latency-bound.  Only the u, w recovery mixes the
-// components (i kx v', i kz eta): each thread takes its partner's values by
-// a shuffle, so no thread reads the half of a slot its partner writes.
-// ---------------------------------------------------------------------------
-namespace {
 // component c of a complex128 in memory
 __device__ __forceinline__ const double* cptr(const double2* p, int c) { return reinterpret_cast<const double*>(p) + c; }
 __device__ __forceinline__ double* cptr(double2* p, int c) { return reinterpret_cast<double*>(p) + c; }
 
+// what a thread of k_solve carries: a complex value, or one component of it
+template <bool RI> struct Part;
+template <> struct Part<false> {
+  using B = double2;
+  __device__ static B ld(const double2* p, int) { return *p; }
+  __device__ static void st(double2* p, int, B v) { *p = v; }
+  __device__ static B real(double v, int) { return make_double2(v, 0.0); }
+  __device__ static B pair(const double* w, int) { return make_double2(w[0], w[1]); }
+};
+template <> struct Part<true> {
+  using B = double;
+  __device__ static B ld(const double2* p, int c) { return *cptr(p, c); }
+  __device__ static void st(double2* p, int c, B v) { *cptr(p, c) = v; }
+  __device__ static B real(double v, int c) { return c == 0 ? v : 0.0; }
+  __device__ static B pair(const double* w, int c) { return w[c]; }
+};
+__device__ __forceinline__ double rmul(double s, double a) { return s * a; }
+__device__ __forceinline__ double cdivr(double a, double s) { return a / s; }
+__device__ __forceinline__ double step1u(double b, double rd, double u1, double u2, double x1, double x2) {
+  return rd * fma(-u2, x2, fma(-u1, x1, b));
+}
+__device__ __forceinline__ double step2(double b, double lm2, double lm1, double bm2, double bm1) {
+  return fma(-lm1, bm1, fma(-lm2, bm2, b));
+}
+template <int N, typename B> __device__ __forceinline__ B dotn(const B* v, const double* c) {
+  B s = rmul(c[0], v[0]);
+#pragma unroll
+  for (int j = 1; j < N; ++j) s = s + rmul(c[j], v[j]);
+  return s;
+}
+
 // one component of DerivOps' arithmetic
 template <typename R> struct DerivC;
 template <> struct DerivC<double> {
-  using S = double;
-  __device__ static S in(double v) { return v; }
-  __device__ static double scal(double v) { return v; }
-  __device__ static S rm(double c, S x) { return c * x; }
-  __device__ static void park(double2* p, int c, S x) { *cptr(p, c) = x; }
-  __device__ static S unpark(const double2* p, int c) { return *cptr(p, c); }
-  __device__ static double out(S x) { return x; }
-  __device__ static S partner(S x, unsigned mask) { return __shfl_xor_sync(mask, x, 1); }
+  using C = double;
+  __device__ static C in(double v) { return v; }
+  __device__ static C rm(double c, C x) { return c * x; }
+  __device__ static void park(double2* p, int c, C x) { *cptr(p, c) = x; }
+  __device__ static C unpark(const double2* p, int c) { return *cptr(p, c); }
+  __device__ static double out(C x) { return x; }
+  __device__ static C partner(C x, unsigned mask) { return __shfl_xor_sync(mask, x, 1); }
 };
 template <> struct DerivC<dd> {
-  using S = dd;
-  __device__ static S in(double v) { return dd_from_double(v); }
-  __device__ static dd scal(double v) { return dd_from_double(v); }
-  __device__ static S rm(dd c, S x) { return c * x; }
-  __device__ static void park(double2* p, int c, S x) { reinterpret_cast<float2*>(p)[c] = make_float2(x.hi, x.lo); }
-  __device__ static S unpark(const double2* p, int c) {
+  using C = dd;
+  __device__ static C in(double v) { return dd_from_double(v); }
+  __device__ static C rm(dd c, C x) { return c * x; }
+  __device__ static void park(double2* p, int c, C x) { reinterpret_cast<float2*>(p)[c] = make_float2(x.hi, x.lo); }
+  __device__ static C unpark(const double2* p, int c) {
     const float2 f = reinterpret_cast<const float2*>(p)[c];
     return dd(f.x, f.y);
   }
-  __device__ static double out(S x) { return dd_to_double_int(x); }
-  __device__ static S partner(S x, unsigned mask) {
+  __device__ static double out(C x) { return dd_to_double_int(x); }
+  __device__ static C partner(C x, unsigned mask) {
     return dd(__shfl_xor_sync(mask, x.hi, 1), __shfl_xor_sync(mask, x.lo, 1));
   }
 };
+template <typename R> struct DerivFull : DerivOps<R> {
+  using C = typename DerivOps<R>::C;
+  __device__ static void park(double2* p, int, C x) { DerivOps<R>::park(p, x); }
+  __device__ static C unpark(const double2* p, int) { return DerivOps<R>::unpark(p); }
+};
+template <typename R, bool RI> struct DerivPart { using t = DerivFull<R>; };
+template <typename R> struct DerivPart<R, true> { using t = DerivC<R>; };
 
-// deriv_uw for component c of mode m (the partner lane, lane ^ 1, holds the
-// other component of the same mode; mask: the lanes taking part)
-template <typename R>
-__device__ __forceinline__ void deriv_uw_c(double2* __restrict__ V, const double* __restrict__ der,
-                                           const double* __restrict__ d0lu, const dd* __restrict__ lindd,
-                                           const BcRows& bc, const Dims& d, int m, double ka, double kz, double k2,
-                                           int c, unsigned mask) {
+// rows r0..r1 of part `part` of NP parts of the interior rows 1..ny-1
+template <int NP> __device__ __forceinline__ void part_rows(int ny, int part, int& r0, int& r1) {
+  r0 = 1 + (ny - 1) * part / NP;
+  r1 = (ny - 1) * (part + 1) / NP;
+}
+
+// steps 2 to 4 for mode m (takes: this thread has one), component c
+template <typename R, bool RI, int NP, typename Mean>
+__device__ __forceinline__ void deriv_uw_parts(double2* __restrict__ V, const double* __restrict__ der,
+                                               const double* __restrict__ d0lu, const dd* __restrict__ lindd,
+                                               const BcRows& bc, const Dims& d, int m, double ka, double kz,
+                                               double k2, int c, int part, bool takes, Mean mean_flow) {
   using O = DerivOps<R>;
-  using Q = DerivC<R>;
-  using S = typename Q::S;
+  using Q = typename DerivPart<R, RI>::t;
+  using P = Part<RI>;
+  using C = typename Q::C;
   const int ny = d.ny;
-  const double rk2 = 1.0 / k2;
-  const R au = O::scal(ka * rk2), bu = O::scal(kz * rk2);
-  S vlo[5], vhi[5];
+  int r0, r1;
+  part_rows<NP>(ny, part, r0, r1);
+  auto v = [&](int iy) -> C { return Q::in(P::ld(&V[vidx(d, 1, iy, m)], c)); };
+  auto dot5r = [&](const C* x, const double* w) {
+    C acc = Q::rm(O::scal(w[0]), x[0]);
 #pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    vlo[j] = Q::in(*cptr(&V[vidx(d, 1, -1 + j, m)], c));
-    vhi[j] = Q::in(*cptr(&V[vidx(d, 1, ny - 3 + j, m)], c));
-  }
-  auto dot5r = [&](const S* v, const double* cf) {
-    S acc = Q::rm(Q::scal(cf[0]), v[0]);
-#pragma unroll
-    for (int j = 1; j < 5; ++j) acc = acc + Q::rm(Q::scal(cf[j]), v[j]);
+    for (int j = 1; j < 5; ++j) acc = acc + Q::rm(O::scal(w[j]), x[j]);
     return acc;
   };
-  const S f0 = dot5r(vlo, bc.d140), fm1 = dot5r(vlo, bc.d14m1);
-  const S fn = dot5r(vhi, bc.d14n), fn1 = dot5r(vhi, bc.d14np1);
-  {
-    S win[5];
-    win[1] = vhi[1];
-    win[2] = vhi[2];
-    win[3] = vhi[3];
-    win[4] = vhi[4];
-    S x1 = S(), x2 = S();
-    double wnext = *cptr(&V[vidx(d, 1, ny - 3, m)], c);
-    for (int iy = ny - 1; iy >= 1; --iy) {
-      win[0] = Q::in(wnext);
-      if (iy > 1) wnext = *cptr(&V[vidx(d, 1, iy - 3, m)], c);
-      S f = Q::rm(O::d1(der, lindd, iy, 0), win[0]);
+  C f0 = C(), fm1 = C(), fn = C(), fn1 = C();
+  if (takes && r0 <= r1) {
+    C win[5];
+    if (r0 <= 2) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) win[j] = v(-1 + j);
+      f0 = dot5r(win, bc.d140);
+      fm1 = dot5r(win, bc.d14m1);
+    }
+    if (r1 >= ny - 2) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) win[j] = v(ny - 3 + j);
+      fn = dot5r(win, bc.d14n);
+      fn1 = dot5r(win, bc.d14np1);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) win[j + 1] = v(r0 - 2 + j);
+    typename P::B next = P::ld(&V[vidx(d, 1, r0 + 2, m)], c);  // v one row ahead
+    for (int iy = r0; iy <= r1; ++iy) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) win[j] = win[j + 1];
+      win[4] = Q::in(next);
+      if (iy < r1) next = P::ld(&V[vidx(d, 1, iy + 3, m)], c);
+      C f = Q::rm(O::d1(der, lindd, iy, 0), win[0]);
 #pragma unroll
       for (int j = 1; j < 5; ++j) f = f + Q::rm(O::d1(der, lindd, iy, j), win[j]);
       if (iy == ny - 1) f = f - (Q::rm(O::d0(der, lindd, iy, 3), fn) + Q::rm(O::d0(der, lindd, iy, 4), fn1));
       if (iy == ny - 2) f = f - Q::rm(O::d0(der, lindd, iy, 4), fn);
       if (iy == 1) f = f - (Q::rm(O::d0(der, lindd, iy, 1), f0) + Q::rm(O::d0(der, lindd, iy, 0), fm1));
       if (iy == 2) f = f - Q::rm(O::d0(der, lindd, iy, 0), f0);
-      S x;
-      if constexpr (std::is_same<R, double>::value) {
-        x = O::lu(d0lu, lindd, iy, 2) * fma(-O::lu(d0lu, lindd, iy, 4), x2, fma(-O::lu(d0lu, lindd, iy, 3), x1, f));
-      } else {
-        const S s = Q::rm(O::lu(d0lu, lindd, iy, 3), x1) + Q::rm(O::lu(d0lu, lindd, iy, 4), x2);
-        x = Q::rm(O::lu(d0lu, lindd, iy, 2), f - s);
-      }
-      x2 = x1;
-      x1 = x;
-      Q::park(&V[vidx(d, 2, iy, m)], c, x);
-#pragma unroll
-      for (int j = 4; j > 0; --j) win[j] = win[j - 1];
+      Q::park(&V[vidx(d, 2, iy, m)], c, f);
     }
   }
-  {
-    S bm2 = S(), bm1 = fm1;
-    double etn = *cptr(&V[vidx(d, 0, -1, m)], c);
-    S xn = S();
-    for (int iy = -1; iy <= ny + 1; ++iy) {
-      const S et = Q::in(etn);
-      const S xs = xn;
-      if (iy < ny + 1) etn = *cptr(&V[vidx(d, 0, iy + 1, m)], c);
-      if (iy + 1 >= 1 && iy + 1 <= ny - 1) xn = Q::unpark(&V[vidx(d, 2, iy + 1, m)], c);
-      S vp;
-      if (iy == -1) vp = fm1;
-      else if (iy == 0) vp = f0;
-      else if (iy == ny) vp = fn;
-      else if (iy == ny + 1) vp = fn1;
-      else if constexpr (std::is_same<R, double>::value)
-        vp = fma(-O::lu(d0lu, lindd, iy, 1), bm1, fma(-O::lu(d0lu, lindd, iy, 0), bm2, xs));
-      else
-        vp = xs - (Q::rm(O::lu(d0lu, lindd, iy, 0), bm2) + Q::rm(O::lu(d0lu, lindd, iy, 1), bm1));
-      if (iy >= 0 && iy <= ny - 1) {
-        bm2 = bm1;
-        bm1 = vp;
-      }
-      // u = (i kx v' - i kz eta)/k2, w = (i kz v' + i kx eta)/k2: each
-      // component takes the other component of v' and eta
-      const S vo = Q::partner(vp, mask), eo = Q::partner(et, mask);
-      S u, w;
-      if constexpr (std::is_same<R, double>::value) {  // deriv_uw's fused forms
-        if (c == 0) {
-          u = fma(bu, eo, -(au * vo));
-          w = fma(-au, eo, -(bu * vo));
-        } else {
-          u = fma(au, vo, -(bu * eo));
-          w = fma(bu, vo, au * eo);
+  __syncthreads();  // every row's right-hand side is parked
+  mean_flow();
+  if (takes && part == 0) {
+    {  // Step1 of D0mat: x = A2 (f - A3 x1 - A4 x2)
+      C x1 = C(), x2 = C(), fx[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) fx[u] = Q::unpark(&V[vidx(d, 2, max(ny - 1 - u, 1), m)], c);
+      for (int top = ny - 1; top >= 1; top -= kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int iy = top - u;
+          if (iy < 1) break;
+          const C f = fx[u];
+          if (iy - kAhead >= 1) fx[u] = Q::unpark(&V[vidx(d, 2, iy - kAhead, m)], c);
+          C x;
+          if constexpr (std::is_same<R, double>::value) {
+            x = step1u(f, O::lu(d0lu, lindd, iy, 2), O::lu(d0lu, lindd, iy, 3), O::lu(d0lu, lindd, iy, 4), x1, x2);
+          } else {
+            const C t = Q::rm(O::lu(d0lu, lindd, iy, 3), x1) + Q::rm(O::lu(d0lu, lindd, iy, 4), x2);
+            x = Q::rm(O::lu(d0lu, lindd, iy, 2), f - t);
+          }
+          x2 = x1;
+          x1 = x;
+          Q::park(&V[vidx(d, 2, iy, m)], c, x);
         }
+      }
+    }
+    {  // Step2: vp = x - (l2 bm2 + l1 bm1)
+      C bm2 = fm1, bm1 = f0, xs[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) xs[u] = Q::unpark(&V[vidx(d, 2, min(1 + u, ny - 1), m)], c);
+      for (int low = 1; low <= ny - 1; low += kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int iy = low + u;
+          if (iy > ny - 1) break;
+          const C x = xs[u];
+          if (iy + kAhead <= ny - 1) xs[u] = Q::unpark(&V[vidx(d, 2, iy + kAhead, m)], c);
+          C vp;
+          if constexpr (std::is_same<R, double>::value)
+            vp = step2(x, O::lu(d0lu, lindd, iy, 0), O::lu(d0lu, lindd, iy, 1), bm2, bm1);
+          else
+            vp = x - (Q::rm(O::lu(d0lu, lindd, iy, 0), bm2) + Q::rm(O::lu(d0lu, lindd, iy, 1), bm1));
+          bm2 = bm1;
+          bm1 = vp;
+          Q::park(&V[vidx(d, 2, iy, m)], c, vp);
+        }
+      }
+    }
+  }
+  __syncthreads();  // v' of every row is parked
+  const unsigned mask = __ballot_sync(0xffffffffu, takes);
+  if (!takes) return;
+  const double rk2 = 1.0 / k2;
+  const R au = O::scal(ka * rk2), bu = O::scal(kz * rk2);
+  // u = (i kx v' - i kz eta)/k2, w = (i kz v' + i kx eta)/k2; in FP64 with
+  // explicit fused multiply-adds, so that both forms round alike
+  auto recover = [&](int iy, C vp, C et) {
+    C u, w;
+    if constexpr (RI) {
+      const C vo = Q::partner(vp, mask), eo = Q::partner(et, mask);
+      if constexpr (std::is_same<R, double>::value) {
+        u = c == 0 ? fma(bu, eo, -(au * vo)) : fma(au, vo, -(bu * eo));
+        w = c == 0 ? fma(-au, eo, -(bu * vo)) : fma(bu, vo, au * eo);
       } else if (c == 0) {
         u = bu * eo - au * vo;
         w = R() - bu * vo - au * eo;
@@ -1373,181 +1297,292 @@ __device__ __forceinline__ void deriv_uw_c(double2* __restrict__ V, const double
         u = au * vo - bu * eo;
         w = bu * vo + au * eo;
       }
-      *cptr(&V[vidx(d, 0, iy, m)], c) = Q::out(u);
-      *cptr(&V[vidx(d, 2, iy, m)], c) = Q::out(w);
+    } else if constexpr (std::is_same<R, double>::value) {
+      u.x = fma(bu, et.y, -(au * vp.y));
+      u.y = fma(au, vp.x, -(bu * et.x));
+      w.x = fma(-au, et.y, -(bu * vp.y));
+      w.y = fma(bu, vp.x, au * et.x);
+    } else {
+      u.x = bu * et.y - au * vp.y;
+      u.y = au * vp.x - bu * et.x;
+      w.x = R() - bu * vp.y - au * et.y;
+      w.y = bu * vp.x + au * et.x;
     }
+    P::st(&V[vidx(d, 0, iy, m)], c, Q::out(u));
+    P::st(&V[vidx(d, 2, iy, m)], c, Q::out(w));
+  };
+  auto eta = [&](int iy) -> C { return Q::in(P::ld(&V[vidx(d, 0, iy, m)], c)); };
+  if (part == 0) {
+    recover(-1, fm1, eta(-1));
+    recover(0, f0, eta(0));
   }
+  if (part == NP - 1) {
+    recover(ny, fn, eta(ny));
+    recover(ny + 1, fn1, eta(ny + 1));
+  }
+#pragma unroll 2
+  for (int iy = r0; iy <= r1; ++iy) recover(iy, Q::unpark(&V[vidx(d, 2, iy, m)], c), eta(iy));
 }
 }  // namespace
 
-// Eight threads per pair: warp w is the role of k_solve's warp w (system w/2,
-// mode w%2); lane l takes pair l/2 of the block's 16 and component l%2.
-__global__ void __launch_bounds__(128, 4) k_solve_ri(double2* __restrict__ V, const double2* rhs, size_t rcs,
-                                                     int roff, const double* __restrict__ fac,
-                                                     const double* __restrict__ der, const double* __restrict__ d0lu,
-                                                     const double* __restrict__ yint, BcRows bc, Dims d,
-                                                     DevScalars* __restrict__ sc, const dd* __restrict__ lindd,
-                                                     int q_lo, int q_hi) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int sys = w >> 1, t = w & 1, c = lane & 1;
-  const int q = q_lo + blockIdx.x * 16 + (lane >> 1);
+template <bool RI, int NP>
+__global__ void __launch_bounds__(64 * NP, 8 / NP) k_solve(double2* __restrict__ V, const double2* rhs, size_t rcs,
+                                                          int roff, const double* __restrict__ fac,
+                                                          const double* __restrict__ der,
+                                                          const double* __restrict__ d0lu,
+                                                          const double* __restrict__ yint, BcRows bc, Dims d,
+                                                          DevScalars* __restrict__ sc, const dd* __restrict__ lindd,
+                                                          int q_lo, int q_hi) {
+  static_assert(NP >= 2, "four warps solve");
+  using P = Part<RI>;
+  using B = typename P::B;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int part = wp >> 1, t = wp & 1, c = RI ? lane & 1 : 0;
+  const int sys = part;  // warps 0..3
+  const int q = q_lo + (RI ? (int)blockIdx.x * 16 + (lane >> 1) : (int)blockIdx.x * 32 + lane);
   const bool active = q < q_hi;
   const int ny = d.ny, nz = d.nz;
   const int ix = active ? q / (nz + 1) : 0;
   const int a = active ? q - ix * (nz + 1) : 0;
   const int nm = (a == 0) ? 1 : 2;
-  int mm[2];
-  mm[0] = ix * d.nzt + nz + a;
-  mm[1] = ix * d.nzt + nz - a;
+  const int mt = ix * d.nzt + nz + (t == 0 ? a : -a);
   const bool is00 = (ix == 0 && a == 0);
   const double ka = ix * d.alfa0, kb = a * d.beta0;
   const double k2 = ka * ka + kb * kb;
   const double ni = d.ni;
-  const size_t P = d.npairs;
+  const size_t NPR = d.npairs;
   const bool ucor = active && is00 && sys == 1 && t == 1;  // unit-forcing response (linsolve_blocking.inc:62-68)
-  const bool mine = active && t < nm;
-  const int m = mm[ucor ? 0 : t];
+  const bool mine = active && t < nm && sys < 2;
+  const int m = mt;
   const int vc = ucor ? 2 : (sys == 0 ? 1 : 0);  // field slot written
   const bool wallrhs = mine && sys == 1 && is00;
-  double bot[5], botm1[5], top[5], topp1[5];
-#pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    bot[j] = sys ? bc.eta0bc[j] : bc.v0bc[j];
-    botm1[j] = sys ? bc.eta0m1bc[j] : bc.v0m1bc[j];
-    top[j] = sys ? bc.etanbc[j] : bc.vnbc[j];
-    topp1[j] = sys ? bc.etanp1bc[j] : bc.vnp1bc[j];
-  }
-  // the wall velocity enters the real component only
-  const double bval0 = (wallrhs && c == 0) ? sc->u0 : 0.0, bvaln = (wallrhs && c == 0) ? sc->uN : 0.0;
   if (mine || ucor) {
-    const double* fs = fac + (size_t)5 * sys * P + q;
-    const size_t frow = (size_t)kFacPerRow * P;
-    // ---- Step1 bottom-up: x = (b - u1 x(+1) - u2 x(+2)) / d ----
+    double bot[5], botm1[5], top[5], topp1[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      bot[j] = sys ? bc.eta0bc[j] : bc.v0bc[j];
+      botm1[j] = sys ? bc.eta0m1bc[j] : bc.v0m1bc[j];
+      top[j] = sys ? bc.etanbc[j] : bc.vnbc[j];
+      topp1[j] = sys ? bc.etanp1bc[j] : bc.vnp1bc[j];
+    }
+    const double bval0 = wallrhs ? sc->u0 : 0.0, bvaln = wallrhs ? sc->uN : 0.0;
+    const double* fs = fac + (size_t)5 * sys * NPR + q;  // this system's factors of row 1
+    const size_t frow = (size_t)kFacPerRow * NPR;
     const double2* rsrc = rhs + (sys == 0 ? rcs : 0);
-    double x1 = 0.0, x2 = 0.0;
-    double bn = ucor ? (c == 0 ? 1.0 : 0.0) : *cptr(&rsrc[(size_t)(ny - 1 + roff) * d.nmodes + m], c);
-    const double* f = fs + (size_t)(ny - 2) * frow;
-    double dn = f[2 * P], u1n = f[3 * P], u2n = f[4 * P];
-    for (int iy = ny - 1; iy >= 1; --iy) {
-      double b = bn;
-      const double dv = dn, u1 = u1n, u2 = u2n;
-      if (iy > 1) {  // one row ahead (global-load latency)
-        if (!ucor) bn = *cptr(&rsrc[(size_t)(iy - 1 + roff) * d.nmodes + m], c);
-        f -= frow;
-        dn = f[2 * P];
-        u1n = f[3 * P];
-        u2n = f[4 * P];
-      }
-      if (iy - kSolvePrefetch >= 1) {  // and the lines of a row further down
-        const double* fp = f - (size_t)(kSolvePrefetch - 1) * frow;
-        prefetch_l1(fp + 2 * P);
-        prefetch_l1(fp + 3 * P);
-        prefetch_l1(fp + 4 * P);
-        if (!ucor) prefetch_l1(rsrc + (size_t)(iy - kSolvePrefetch + roff) * d.nmodes + m);
-      }
-      if (wallrhs) {
-        if (iy == 1) b = b - sc->wallrhs[0 + c];
-        if (iy == 2) b = b - sc->wallrhs[2 + c];
-        if (iy == ny - 2) b = b - sc->wallrhs[4 + c];
-        if (iy == ny - 1) b = b - sc->wallrhs[6 + c];
-      }
-      const double x = dv * fma(-u2, x2, fma(-u1, x1, b));
-      x2 = x1;
-      x1 = x;
-      *cptr(&V[vidx(d, vc, iy, m)], c) = x;
-    }
-    // ---- Step2 top-down: v = x - l2 v(-2) - l1 v(-1); rows 1..3 and ny-3..ny-1 kept ----
-    double lo[3], hi[3];
-    double m2 = 0.0, m1 = 0.0;
-    f = fs;
-    double l2n = f[0], l1n = f[P];
-    double vn = *cptr(&V[vidx(d, vc, 1, m)], c);
-    for (int iy = 1; iy <= ny - 1; ++iy) {
-      const double l2 = l2n, l1 = l1n;
-      const double vcur = vn;
-      if (iy < ny - 1) {
-        f += frow;
-        l2n = f[0];
-        l1n = f[P];
-        vn = *cptr(&V[vidx(d, vc, iy + 1, m)], c);
-      }
-      if (iy + kSolvePrefetch <= ny - 1) {
-        const double* fp = f + (size_t)(kSolvePrefetch - 1) * frow;
-        prefetch_l1(fp);
-        prefetch_l1(fp + P);
-        prefetch_l1(&V[vidx(d, vc, iy + kSolvePrefetch, m)]);
-      }
-      const double nv = fma(-l1, m1, fma(-l2, m2, vcur));
-      *cptr(&V[vidx(d, vc, iy, m)], c) = nv;
-      m2 = m1;
-      m1 = nv;
-      if (iy == 1) lo[0] = nv;
-      if (iy == 2) lo[1] = nv;
-      if (iy == 3) lo[2] = nv;
-      if (iy == ny - 3) hi[0] = nv;
-      if (iy == ny - 2) hi[1] = nv;
-      if (iy == ny - 1) hi[2] = nv;
-    }
-    // wall and ghost values (linsolve_blocking.inc:50-61), per component as dot3/dot4/cdivr
-    auto d3 = [](const double* v, const double* cf) {
-      double s = cf[0] * v[0];
-      s = s + cf[1] * v[1];
-      return s + cf[2] * v[2];
+    B lo[3], hi[3];  // rows 1..3 and ny-3..ny-1 of the solution
+    auto keep = [&](int iy, B v) {
+      if (iy == 1) lo[0] = v;
+      if (iy == 2) lo[1] = v;
+      if (iy == 3) lo[2] = v;
+      if (iy == ny - 3) hi[0] = v;
+      if (iy == ny - 2) hi[1] = v;
+      if (iy == ny - 1) hi[2] = v;
     };
-    auto d4 = [](const double* v, const double* cf) {
-      double s = cf[0] * v[0];
-      s = s + cf[1] * v[1];
-      s = s + cf[2] * v[2];
-      return s + cf[3] * v[3];
+    // the packed wall velocity (linsolve_blocking.inc:26-27,40-41)
+    auto wall_terms = [&](int iy, B b) -> B {
+      if (iy == 1) b = b - P::pair(sc->wallrhs, c);
+      if (iy == 2) b = b - P::pair(sc->wallrhs + 2, c);
+      if (iy == ny - 2) b = b - P::pair(sc->wallrhs + 4, c);
+      if (iy == ny - 1) b = b - P::pair(sc->wallrhs + 6, c);
+      return b;
     };
-    const double w0 = (bval0 - d3(lo, bot + 2)) / bot[1];
-    const double rb[4] = {w0, lo[0], lo[1], lo[2]};
-    const double wm1 = (0.0 - d4(rb, botm1 + 1)) / botm1[0];
-    const double wn = (bvaln - d3(hi, top)) / top[3];
-    const double rt[4] = {hi[0], hi[1], hi[2], wn};
-    const double wn1 = (0.0 - d4(rt, topp1)) / topp1[4];
-    *cptr(&V[vidx(d, vc, -1, m)], c) = wm1;
-    *cptr(&V[vidx(d, vc, 0, m)], c) = w0;
-    *cptr(&V[vidx(d, vc, ny, m)], c) = wn;
-    *cptr(&V[vidx(d, vc, ny + 1, m)], c) = wn1;
+    // operands ahead of the recurrence: kAhead rows in registers where a warp
+    // has its scheduler nearly to itself (NP 4; 32x64x32 mixed 0.538 -> 0.511
+    // ms per step), else one row in registers and the lines of six rows
+    // further prefetched into L1 (79x101x75 mixed 2.96 -> 2.83 the other way)
+    if constexpr (NP == 4) {
+      {  // ---- Step1 bottom-up: x = (b - u1 x(+1) - u2 x(+2)) / d ----
+        B bq[kAhead];
+        double dq[kAhead], u1q[kAhead], u2q[kAhead];
+        auto fetch = [&](int u, int iy) {
+          bq[u] = ucor ? P::real(1.0, c) : P::ld(&rsrc[(size_t)(iy + roff) * d.nmodes + m], c);
+          const double* f = fs + (size_t)(iy - 1) * frow;
+          dq[u] = f[2 * NPR];
+          u1q[u] = f[3 * NPR];
+          u2q[u] = f[4 * NPR];
+        };
+  #pragma unroll
+        for (int u = 0; u < kAhead; ++u) fetch(u, max(ny - 1 - u, 1));
+        B x1 = P::real(0.0, 0), x2 = x1;
+        for (int hi = ny - 1; hi >= 1; hi -= kAhead) {
+  #pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            const int iy = hi - u;
+            if (iy < 1) break;
+            B b = bq[u];
+            const double dv = dq[u], u1 = u1q[u], u2 = u2q[u];
+            if (iy - kAhead >= 1) fetch(u, iy - kAhead);
+            if (wallrhs) b = wall_terms(iy, b);
+            const B x = step1u(b, dv, u1, u2, x1, x2);
+            x2 = x1;
+            x1 = x;
+            P::st(&V[vidx(d, vc, iy, m)], c, x);
+          }
+        }
+      }
+      // ---- Step2 top-down: v = x - l2 v(-2) - l1 v(-1) ----
+      {
+        B vq[kAhead];
+        double l2q[kAhead], l1q[kAhead];
+        auto fetch = [&](int u, int iy) {
+          vq[u] = P::ld(&V[vidx(d, vc, iy, m)], c);
+          const double* f = fs + (size_t)(iy - 1) * frow;
+          l2q[u] = f[0];
+          l1q[u] = f[NPR];
+        };
+  #pragma unroll
+        for (int u = 0; u < kAhead; ++u) fetch(u, min(1 + u, ny - 1));
+        B m2 = P::real(0.0, 0), m1 = m2;
+        for (int low = 1; low <= ny - 1; low += kAhead) {
+  #pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            const int iy = low + u;
+            if (iy > ny - 1) break;
+            const B x = vq[u];
+            const double l2 = l2q[u], l1 = l1q[u];
+            if (iy + kAhead <= ny - 1) fetch(u, iy + kAhead);
+            const B nv = step2(x, l2, l1, m2, m1);
+            P::st(&V[vidx(d, vc, iy, m)], c, nv);
+            m2 = m1;
+            m1 = nv;
+            keep(iy, nv);
+          }
+        }
+      }
+    } else {
+      {  // ---- Step1 bottom-up: x = (b - u1 x(+1) - u2 x(+2)) / d ----
+        B x1 = P::real(0.0, 0), x2 = x1;
+        B bn = ucor ? P::real(1.0, c) : P::ld(&rsrc[(size_t)(ny - 1 + roff) * d.nmodes + m], c);
+        const double* f = fs + (size_t)(ny - 2) * frow;
+        double dn = f[2 * NPR], u1n = f[3 * NPR], u2n = f[4 * NPR];
+        for (int iy = ny - 1; iy >= 1; --iy) {
+          B b = bn;
+          const double dv = dn, u1 = u1n, u2 = u2n;
+          if (iy > 1) {  // one row ahead (global-load latency)
+            if (!ucor) bn = P::ld(&rsrc[(size_t)(iy - 1 + roff) * d.nmodes + m], c);
+            f -= frow;
+            dn = f[2 * NPR];
+            u1n = f[3 * NPR];
+            u2n = f[4 * NPR];
+          }
+          if (iy - kSolvePrefetch >= 1) {  // and the lines of a row further down
+            const double* fp = f - (size_t)(kSolvePrefetch - 1) * frow;
+            prefetch_l1(fp + 2 * NPR);
+            prefetch_l1(fp + 3 * NPR);
+            prefetch_l1(fp + 4 * NPR);
+            if (!ucor) prefetch_l1(rsrc + (size_t)(iy - kSolvePrefetch + roff) * d.nmodes + m);
+          }
+          if (wallrhs) b = wall_terms(iy, b);
+          const B x = step1u(b, dv, u1, u2, x1, x2);
+          x2 = x1;
+          x1 = x;
+          P::st(&V[vidx(d, vc, iy, m)], c, x);
+        }
+      }
+      // ---- Step2 top-down: v = x - l2 v(-2) - l1 v(-1) ----
+      {
+        B m2 = P::real(0.0, 0), m1 = m2;
+        const double* f = fs;
+        double l2n = f[0], l1n = f[NPR];
+        B vn = P::ld(&V[vidx(d, vc, 1, m)], c);
+        for (int iy = 1; iy <= ny - 1; ++iy) {
+          const double l2 = l2n, l1 = l1n;
+          const B vcur = vn;
+          if (iy < ny - 1) {
+            f += frow;
+            l2n = f[0];
+            l1n = f[NPR];
+            vn = P::ld(&V[vidx(d, vc, iy + 1, m)], c);
+          }
+          if (iy + kSolvePrefetch <= ny - 1) {
+            const double* fp = f + (size_t)(kSolvePrefetch - 1) * frow;
+            prefetch_l1(fp);
+            prefetch_l1(fp + NPR);
+            prefetch_l1(&V[vidx(d, vc, iy + kSolvePrefetch, m)]);
+          }
+          const B nv = step2(vcur, l2, l1, m2, m1);
+          P::st(&V[vidx(d, vc, iy, m)], c, nv);
+          m2 = m1;
+          m1 = nv;
+          keep(iy, nv);
+        }
+      }
+    }
+    // wall and ghost values (linsolve_blocking.inc:50-61); the wall velocity is real
+    const B zero = P::real(0.0, c);
+    const B w0 = cdivr(P::real(bval0, c) - dotn<3>(lo, bot + 2), bot[1]);
+    const B rb[4] = {w0, lo[0], lo[1], lo[2]};
+    const B wm1 = cdivr(zero - dotn<4>(rb, botm1 + 1), botm1[0]);
+    const B wn = cdivr(P::real(bvaln, c) - dotn<3>(hi, top), top[3]);
+    const B rt[4] = {hi[0], hi[1], hi[2], wn};
+    const B wn1 = cdivr(zero - dotn<4>(rt, topp1), topp1[4]);
+    P::st(&V[vidx(d, vc, -1, m)], c, wm1);
+    P::st(&V[vidx(d, vc, 0, m)], c, w0);
+    P::st(&V[vidx(d, vc, ny, m)], c, wn);
+    P::st(&V[vidx(d, vc, ny + 1, m)], c, wn1);
   }
   __syncthreads();  // v, eta (and the unit response) of this block's pairs are in V
-  if (wallrhs && c == 0) {  // mean flow (linsolve_blocking.inc:62-97), both components
-    double fu = 0.0, fw = 0.0, fc = 0.0;
-    for (int iy = 1, k = 0; iy <= ny - 1; iy += 2, ++k) {
-      const double a1 = yint[3 * k], a2 = yint[3 * k + 1], a3 = yint[3 * k + 2];
-      const double2 e0 = V[vidx(d, 0, iy - 1, m)], e1 = V[vidx(d, 0, iy, m)], e2 = V[vidx(d, 0, iy + 1, m)];
-      const double2 u0 = V[vidx(d, 2, iy - 1, m)], u1 = V[vidx(d, 2, iy, m)], u2 = V[vidx(d, 2, iy + 1, m)];
-      fu = fu + a1 * e0.x + a2 * e1.x + a3 * e2.x;
-      fw = fw + a1 * e0.y + a2 * e1.y + a3 * e2.y;
-      fc = fc + a1 * u0.x + a2 * u1.x + a3 * u2.x;
-    }
-    double corrpx = sc->corrpx, corrpz = sc->corrpz;
+  // mean flow (linsolve_blocking.inc:62-97): the flow rates' sums by the mean
+  // pair's first eta lane, the correction of the rows by its warp
+  auto mean_flow = [&] {
+    if (wp != 2) return;
+    const unsigned has = __ballot_sync(0xffffffffu, wallrhs && c == 0);
+    if (has == 0) return;
+    const int src = __ffs(has) - 1;
+    const int mm = __shfl_sync(0xffffffffu, m, src);
+    double corrpx = 0.0, corrpz = 0.0;
     const bool cx = fabs(d.meanflowx) > 1.0e-7 && !d.cpi;
     const bool cz_ = fabs(d.meanflowz) > 1.0e-7 && !d.cpi;
-    if (cx) corrpx = (d.meanflowx - fu) / fc;
-    if (cz_) corrpz = (d.meanflowz - fw) / fc;
-    for (int iy = -1; iy <= ny + 1; ++iy) {
-      const double2 et = V[vidx(d, 0, iy, m)];
-      const double uc = V[vidx(d, 2, iy, m)].x;
+    if (lane == src) {
+      // flow rates by the non-uniform Simpson rule (dnsdata.f90:312-324)
+      double fu = 0.0, fw = 0.0, fc = 0.0;
+#pragma unroll 4
+      for (int iy = 1, k = 0; iy <= ny - 1; iy += 2, ++k) {
+        const double a1 = yint[3 * k], a2 = yint[3 * k + 1], a3 = yint[3 * k + 2];
+        const double2 e0 = V[vidx(d, 0, iy - 1, mm)], e1 = V[vidx(d, 0, iy, mm)], e2 = V[vidx(d, 0, iy + 1, mm)];
+        const double2 u0 = V[vidx(d, 2, iy - 1, mm)], u1 = V[vidx(d, 2, iy, mm)], u2 = V[vidx(d, 2, iy + 1, mm)];
+        fu = fu + a1 * e0.x + a2 * e1.x + a3 * e2.x;
+        fw = fw + a1 * e0.y + a2 * e1.y + a3 * e2.y;
+        fc = fc + a1 * u0.x + a2 * u1.x + a3 * u2.x;
+      }
+      corrpx = sc->corrpx;
+      corrpz = sc->corrpz;
+      if (cx) corrpx = (d.meanflowx - fu) / fc;
+      if (cz_) corrpz = (d.meanflowz - fw) / fc;
+      sc->fr[0] = fu; sc->fr[1] = fw; sc->fr[2] = fc;
+      sc->corrpx = corrpx; sc->corrpz = corrpz;
+      if (d.cpi) {
+        if (d.cpi_type == 0) sc->meanpx = (1 - d.gamma) * 6 * ni / fu;
+        else sc->meanpx = (1.5 / d.gamma) * fu * ni;
+      }
+    }
+    corrpx = __shfl_sync(0xffffffffu, corrpx, src);
+    corrpz = __shfl_sync(0xffffffffu, corrpz, src);
+    for (int iy = -1 + lane; iy <= ny + 1; iy += 32) {
+      const double2 et = V[vidx(d, 0, iy, mm)];
+      const double uc = V[vidx(d, 2, iy, mm)].x;
       double U = et.x, W = et.y;
       if (cx) U = U + corrpx * uc;
       if (cz_) W = W + corrpz * uc;
-      V[vidx(d, 0, iy, m)] = make_double2(U, 0.0);
-      V[vidx(d, 2, iy, m)] = make_double2(W, 0.0);
+      V[vidx(d, 0, iy, mm)] = make_double2(U, 0.0);
+      V[vidx(d, 2, iy, mm)] = make_double2(W, 0.0);
     }
-    sc->fr[0] = fu; sc->fr[1] = fw; sc->fr[2] = fc;
-    sc->corrpx = corrpx; sc->corrpz = corrpz;
-    if (d.cpi) {
-      if (d.cpi_type == 0) sc->meanpx = (1 - d.gamma) * 6 * ni / fu;
-      else sc->meanpx = (1.5 / d.gamma) * fu * ni;
+  };
+  const bool takes = active && !is00 && t < nm;
+  const double kz = (t == 0 ? 1.0 : -1.0) * kb;
+  // four threads per pair in FP64: one thread's two sweeps of a mode, whose
+  // FP64 operations are few (127x192x127: 16.7 ms per step, 16.9 in parts);
+  // the double-float recovery is instruction-bound and goes in parts
+  // (47x96x47 mixed 1.42 -> 1.28, 127x192x127 6.54 -> 6.45)
+  if constexpr (!RI) {
+    if (!lindd) {
+      mean_flow();
+      if (takes && part == 0) deriv_uw<double>(V, der, d0lu, lindd, bc, d, mt, ka, kz, k2);
+      return;
     }
   }
-  const bool takes = active && !is00 && sys == 0 && t < nm;  // the same for both lanes of a pair
-  const unsigned mask = __ballot_sync(0xffffffffu, takes);
-  if (!takes) return;
-  if (lindd) deriv_uw_c<dd>(V, der, d0lu, lindd, bc, d, mm[t], ka, (t == 0 ? 1.0 : -1.0) * kb, k2, c, mask);
-  else deriv_uw_c<double>(V, der, d0lu, lindd, bc, d, mm[t], ka, (t == 0 ? 1.0 : -1.0) * kb, k2, c, mask);
+  if (lindd) deriv_uw_parts<dd, RI, NP>(V, der, d0lu, lindd, bc, d, mt, ka, kz, k2, c, part, takes, mean_flow);
+  else deriv_uw_parts<double, RI, NP>(V, der, d0lu, lindd, bc, d, mt, ka, kz, k2, c, part, takes, mean_flow);
 }
 
 void launch_factor(const SolveLaunch& L, cudaStream_t s) {
@@ -1568,9 +1603,12 @@ void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
   }
   if (!L.factored) launch_factor(L, s);
   if (L.split_solve == 3) {
-    k_solve_ri<<<(unsigned)((L.q_hi - L.q_lo + 15) / 16), 128, 0, s>>>(
-        L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint, L.bc, L.d, L.sc,
-        (const dd*)L.lindd, L.q_lo, L.q_hi);
+    // four parts where that still is one wave (two 256-thread blocks on each
+    // of 152 SMs), else two (four 128-thread blocks)
+    const unsigned g16 = (unsigned)((L.q_hi - L.q_lo + 15) / 16);
+    auto kern = g16 <= 304 ? k_solve<true, 4> : k_solve<true, 2>;
+    kern<<<g16, g16 <= 304 ? 256 : 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu,
+                                                L.yint, L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi);
     return;
   }
   if (L.split_solve == 2) {
@@ -1579,8 +1617,8 @@ void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
                                          L.nud, L.q_lo, L.q_hi);
     return;
   }
-  k_solve<<<grid, 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint, L.bc,
-                               L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi);
+  k_solve<false, 2><<<grid, 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint,
+                                         L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi);
 }
 
 // ---------------------------------------------------------------------------

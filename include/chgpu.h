@@ -155,8 +155,9 @@ const char* chgpu_ensemble_last_error(const chgpu_ensemble* e);
  * the step on one stream or in two kx halves, timed as whole steps.  Keeps the fastest; the field, the RK history and the module
  * scalars are saved and put back, and the results of a step do not depend on
  * the tiles.  Optional: without it the handle uses tiles sized from the
- * shared-memory budget, the split solve with the factorisation ahead below
- * 65 536 pairs and the fused solve in two halves from there on.  No
+ * shared-memory budget, the factorisation ahead with eight threads per pair
+ * up to 9 728 pairs and four below 65 536 (an ensemble's members by their
+ * pairs together), and the fused solve in two halves from there on.  No
  * counterpart in the reference. */
 #define CHGPU_NTILES 7
 int chgpu_autotune(chgpu_handle* h);
