@@ -336,13 +336,32 @@ void fx_weight(long double w, int* hi, int* lo) {
   const long long l = W - (h << 32);
   *lo = l == -0x80000000ll ? -0x7fffffff : (int)l;
 }
-int4 fx_root(long double phi, long double scale = 1.0L) {  // scale exp(-2 pi i phi)
-  const long double ang = 2.0L * 3.14159265358979323846264338327950288L * phi;
-  int4 e;
-  fx_weight(scale * cosl(ang), &e.x, &e.y);
-  fx_weight(-scale * sinl(ang), &e.z, &e.w);
-  return e;
-}
+// the n-th roots of unity (n a multiple of 8) from one octant's sines and
+// cosines: extended precision is slow where it is software
+struct FxRoots {
+  int n;
+  std::vector<long double> c, s;
+  explicit FxRoots(int len) : n(len), c(len / 8 + 1), s(len / 8 + 1) {
+    for (int j = 0; j <= n / 8; ++j) {
+      const long double ang = 2.0L * 3.14159265358979323846264338327950288L * (long double)j / (long double)n;
+      c[j] = cosl(ang);
+      s[j] = sinl(ang);
+    }
+  }
+  int4 operator()(int m, long double scale = 1.0L) const {  // scale exp(-2 pi i m / n), 0 <= m < n
+    const int quarter = m / (n / 4), p = m % (n / 4);
+    long double x = p <= n / 8 ? c[p] : s[n / 4 - p], y = p <= n / 8 ? s[p] : c[n / 4 - p];
+    for (int q = 0; q < quarter; ++q) {
+      const long double t = x;
+      x = -y;
+      y = t;
+    }
+    int4 e;
+    fx_weight(scale * x, &e.x, &e.y);
+    fx_weight(-scale * y, &e.z, &e.w);
+    return e;
+  }
+};
 bool fx_zlen_plan(int n, int* E, int* TPR) {
   switch (n) {
 #define CHGPU_LEN(N) case N: *E = RLen<N>::E; *TPR = RLen<N>::TPR; return true;
@@ -375,11 +394,12 @@ int upload_int4(chgpu_handle* h, void** dst, const std::vector<int4>& w) {
 // per-pass twiddles of the fixed-point kernels' plan, in the order of
 // upload_rplan_twiddles
 int upload_fx_twiddles(chgpu_handle* h, void** dst, int E, int TPR) {
+  const FxRoots root(E * TPR);
   std::vector<int4> w(std::max(1, rplan_twsize<fx2>(E, TPR)));
   for (int p = 1; p < rplan_passes(E, TPR); ++p) {
     const int R = rplan_radix(E, TPR, p), Ns = rplan_ns(E, TPR, p), off = rplan_twoff<fx2>(E, TPR, p);
     for (int k = 0; k < Ns; ++k)
-      for (int r = 1; r < R; ++r) w[off + k * (R - 1) + r - 1] = fx_root((long double)(r * k) / (long double)(Ns * R));
+      for (int r = 1; r < R; ++r) w[off + k * (R - 1) + r - 1] = root(r * k * (E * TPR / (Ns * R)));
   }
   return upload_int4(h, dst, w);
 }
@@ -398,10 +418,11 @@ int upload_fx_tables(chgpu_handle* h) {
     const long double g = frexpl(half, &ex);
     h->fxfac.exp = ex;
     fx_weight(g, &h->fxfac.gh, &h->fxfac.gl);
+    const FxRoots root(2 * M);
     std::vector<int4> w(2 * (size_t)M);
     for (int k = 0; k < M; ++k) {
-      w[k] = fx_root(0.5L * (long double)k / (long double)M);
-      w[M + k] = fx_root(0.5L * (long double)k / (long double)M, g);
+      w[k] = root(k);
+      w[M + k] = root(k, g);
     }
     if (int rc = upload_int4(h, &h->twhx, w)) return rc;
   }
@@ -841,7 +862,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_copy_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_copy_join, cudaEventDisableTiming);
     if (e != cudaSuccess) { rc = cuda_fail(h, e, "cudaStreamCreate"); break; }
-    e = conv_set_smem_limits();
+    e = conv_set_smem_limits(h->prec, nzd, nxd);
     if (e != cudaSuccess) { rc = cuda_fail(h, e, "cudaFuncSetAttribute"); break; }
     if ((rc = dev_alloc((void**)&h->V, sizeof(double2) * 3 * nplanes * nmodes, "field"))) break;
     if ((rc = dev_alloc(&h->old, ts * 2 * (p->ny - 1) * nmodes, "RK history"))) break;

@@ -405,37 +405,38 @@ cudaError_t allow_max_smem(K* kernel, int optin) {
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
 }
+// the generic kernels of one type
+template <typename T>
+cudaError_t generic_limits(int optin) {
+  cudaError_t e;
+  if ((e = allow_max_smem(k_zinv<T>, optin))) return e;
+  if ((e = allow_max_smem(k_zfwd<T>, optin))) return e;
+  if ((e = allow_max_smem(k_xrow<T, 1>, optin))) return e;
+  if ((e = allow_max_smem(k_xrow<T, 2>, optin))) return e;
+  if ((e = allow_max_smem(k_xrow<T, 3>, optin))) return e;
+  return allow_max_smem(k_xrow<T, 2, true>, optin);
+}
 }  // namespace
 
-cudaError_t conv_set_smem_limits() {
+cudaError_t conv_set_smem_limits(int prec, int nzd, int nxd) {
   int dev = 0, optin = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  if ((e = allow_max_smem(k_zinv<double>, optin))) return e;
+  // the closure's gradient transforms, FP32 in every precision
   if ((e = allow_max_smem(k_zinv<float>, optin))) return e;
-  if ((e = allow_max_smem(k_zinv<dd>, optin))) return e;
-  if ((e = allow_max_smem(k_zfwd<double>, optin))) return e;
-  if ((e = allow_max_smem(k_zfwd<float>, optin))) return e;
-  if ((e = allow_max_smem(k_zfwd<dd>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<double, 1>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<double, 2>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<double, 3>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<float, 1>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<float, 2>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<float, 3>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<dd, 1>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<dd, 2>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<dd, 3>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<double, 2, true>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<float, 2, true>, optin))) return e;
-  if ((e = allow_max_smem(k_xrow<dd, 2, true>, optin))) return e;
   if ((e = allow_max_smem(k_xphys<float>, optin))) return e;
-  if ((e = convr_set_smem_limits())) return e;
-  if ((e = fx_z_smem_limits<double>())) return e;
-  if ((e = fx_z_smem_limits<dd>())) return e;
-  return fx_x_smem_limits();
+  if (prec == CHGPU_MIXED) {
+    if ((e = generic_limits<float>(optin))) return e;
+    if ((e = convr_set_smem_limits(nzd))) return e;
+    return convr_set_smem_limits(nxd);
+  }
+  if ((e = fx_z_smem_limits<double>(nzd))) return e;
+  if ((e = fx_x_smem_limits(nxd))) return e;
+  if (prec == CHGPU_FP64) return generic_limits<double>(optin);
+  if ((e = fx_z_smem_limits<dd>(nzd))) return e;
+  return generic_limits<dd>(optin);
 }
 
 }  // namespace chgpu

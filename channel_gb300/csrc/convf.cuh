@@ -396,17 +396,18 @@ cudaError_t set_limits_len() {
 }
 
 template <typename T>
-cudaError_t set_limits_type() {
-  cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = set_limits_len<T, 32>();
-  if (e == cudaSuccess) e = set_limits_len<T, 48>();
-  if (e == cudaSuccess) e = set_limits_len<T, 64>();
-  if (e == cudaSuccess) e = set_limits_len<T, 96>();
-  if (e == cudaSuccess) e = set_limits_len<T, 192>();
-  if (e == cudaSuccess) e = set_limits_len<T, 384>();
-  if (e == cudaSuccess) e = set_limits_len<T, 768>();
-  if (e == cudaSuccess) e = set_limits_len<T, 1536>();
-  return e;
+cudaError_t set_limits_type(int n) {
+  switch (n) {
+    case 32: return set_limits_len<T, 32>();
+    case 48: return set_limits_len<T, 48>();
+    case 64: return set_limits_len<T, 64>();
+    case 96: return set_limits_len<T, 96>();
+    case 192: return set_limits_len<T, 192>();
+    case 384: return set_limits_len<T, 384>();
+    case 768: return set_limits_len<T, 768>();
+    case 1536: return set_limits_len<T, 1536>();
+    default: return cudaSuccess;
+  }
 }
 
 }  // namespace

@@ -7,6 +7,6 @@ template <>
 bool launch_convolutions_r<float>(const ConvLaunch& L, cudaStream_t s, int stage) {
   return launch_convolutions_r_impl<float>(L, s, stage);
 }
-cudaError_t convr_set_smem_limits() { return set_limits_type<float>(); }
+cudaError_t convr_set_smem_limits(int n) { return set_limits_type<float>(n); }
 
 }  // namespace chgpu

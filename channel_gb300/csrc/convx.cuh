@@ -457,6 +457,7 @@ template <typename K> cudaError_t fx_allow_smem(K* kernel, size_t bytes, bool ma
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   return e;
 }
+// shared-memory limits of one length's kernels
 template <typename T, int N> cudaError_t fx_limits_z() {
   constexpr int E = RLen<N>::E, TPR = RLen<N>::TPR, NC = fx_zcols<TPR>();
   const size_t sm = (size_t)NC * rbuf_size<E, TPR>() * sizeof(fx2);

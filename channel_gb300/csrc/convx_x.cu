@@ -11,12 +11,13 @@ bool launch_fx_x(const ConvLaunch& L, cudaStream_t s) {
     default: return false;
   }
 }
-cudaError_t fx_x_smem_limits() {
-  cudaError_t e = cudaSuccess;
-#define CHGPU_LEN(N) if (e == cudaSuccess) e = fx_limits_x<N>();
-  CHGPU_FX_XLENGTHS(CHGPU_LEN)
+cudaError_t fx_x_smem_limits(int nxd) {
+  switch (nxd) {
+#define CHGPU_LEN(N) case N: return fx_limits_x<N>();
+    CHGPU_FX_XLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
-  return e;
+    default: return cudaSuccess;
+  }
 }
 
 }  // namespace chgpu

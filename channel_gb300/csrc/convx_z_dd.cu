@@ -11,12 +11,13 @@ template <> bool launch_fx_z<dd>(const ConvLaunch& L, cudaStream_t s, int stage)
     default: return false;
   }
 }
-template <> cudaError_t fx_z_smem_limits<dd>() {
-  cudaError_t e = cudaSuccess;
-#define CHGPU_LEN(N) if (e == cudaSuccess) e = fx_limits_z<dd, N>();
-  CHGPU_FX_ZLENGTHS(CHGPU_LEN)
+template <> cudaError_t fx_z_smem_limits<dd>(int nzd) {
+  switch (nzd) {
+#define CHGPU_LEN(N) case N: return fx_limits_z<dd, N>();
+    CHGPU_FX_ZLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
-  return e;
+    default: return cudaSuccess;
+  }
 }
 
 }  // namespace chgpu

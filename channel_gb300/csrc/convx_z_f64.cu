@@ -11,12 +11,13 @@ template <> bool launch_fx_z<double>(const ConvLaunch& L, cudaStream_t s, int st
     default: return false;
   }
 }
-template <> cudaError_t fx_z_smem_limits<double>() {
-  cudaError_t e = cudaSuccess;
-#define CHGPU_LEN(N) if (e == cudaSuccess) e = fx_limits_z<double, N>();
-  CHGPU_FX_ZLENGTHS(CHGPU_LEN)
+template <> cudaError_t fx_z_smem_limits<double>(int nzd) {
+  switch (nzd) {
+#define CHGPU_LEN(N) case N: return fx_limits_z<double, N>();
+    CHGPU_FX_ZLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
-  return e;
+    default: return cudaSuccess;
+  }
 }
 
 }  // namespace chgpu

@@ -68,7 +68,10 @@ struct ConvLaunch {
 
 // stage 0: z-inverse, 1: x rows, 2: z-forward
 template <typename T> void launch_convolutions(const ConvLaunch& L, cudaStream_t s, int stage);
-cudaError_t conv_set_smem_limits();
+// shared-memory limits of the transform kernels a handle of this precision
+// (CHGPU_FP64, ...) and these lengths can launch; the others are not touched,
+// so the driver need not load them
+cudaError_t conv_set_smem_limits(int prec, int nzd, int nxd);
 // the register-blocked stage kernels; false when the stage's length has no
 // plan.  float: convf.cuh (convf_f32.cu); double and dd: the fixed-point ones
 // of convx.cuh (convx_z_f64.cu, convx_z_dd.cu, convx_x.cu)
@@ -76,16 +79,16 @@ template <typename T> bool launch_convolutions_r(const ConvLaunch& L, cudaStream
 template <> bool launch_convolutions_r<float>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_convolutions_r<double>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_convolutions_r<dd>(const ConvLaunch& L, cudaStream_t s, int stage);
-cudaError_t convr_set_smem_limits();
+cudaError_t convr_set_smem_limits(int n);  // FP32 kernels of length n
 // stage 0 and 2 (T: VV's type; stage 0 is launch_fx_z<double>), stage 1
 template <typename T> bool launch_fx_z(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_fx_z<double>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_fx_z<dd>(const ConvLaunch& L, cudaStream_t s, int stage);
 bool launch_fx_x(const ConvLaunch& L, cudaStream_t s);
-template <typename T> cudaError_t fx_z_smem_limits();
-template <> cudaError_t fx_z_smem_limits<double>();
-template <> cudaError_t fx_z_smem_limits<dd>();
-cudaError_t fx_x_smem_limits();
+template <typename T> cudaError_t fx_z_smem_limits(int nzd);
+template <> cudaError_t fx_z_smem_limits<double>(int nzd);
+template <> cudaError_t fx_z_smem_limits<dd>(int nzd);
+cudaError_t fx_x_smem_limits(int nxd);
 #define CHGPU_FX_ZLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536)
 #define CHGPU_FX_XLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768)
 // dynamic shared memory of the z-transform and x-row kernels (padded buffers)
