@@ -364,7 +364,7 @@ struct FxRoots {
 };
 bool fx_zlen_plan(int n, int* E, int* TPR) {
   switch (n) {
-#define CHGPU_LEN(N) case N: *E = RLen<N>::E; *TPR = RLen<N>::TPR; return true;
+#define CHGPU_LEN(N) case N: *E = FxLen<N>::E; *TPR = FxLen<N>::TPR; return true;
     CHGPU_FX_ZLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
     default: return false;
@@ -372,7 +372,7 @@ bool fx_zlen_plan(int n, int* E, int* TPR) {
 }
 bool fx_xlen_plan(int n, int* E, int* TPR) {
   switch (n) {
-#define CHGPU_LEN(N) case N: *E = FxXLen<N>::E; *TPR = FxXLen<N>::TPR; return true;
+#define CHGPU_LEN(N) case N: *E = FxLen<N>::E; *TPR = FxLen<N>::TPR; return true;
     CHGPU_FX_XLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
     default: return false;

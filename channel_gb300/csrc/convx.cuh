@@ -24,14 +24,16 @@
 // V, Zb and Pb are FP64; VV is FP64 or, in the double-float path (whose
 // stencils read it), double-float.
 //
-// What bounds them (GB300, counters at 255x64x255): instruction issue of 12
-// resident warps per SM (34-43% of the issue slots, the rest fixed-latency and
-// instruction-fetch waits), not memory (1.5 TB/s in k_zinv_x).  Against the
-// FP64-pipe transforms they replace, the whole FP64 step went from 44.9 to
-// 19.3 ms at 127x192x127 and from 262 to 109 ms at 255x256x255 (k_xrow 39,
-// k_zfwd 10, k_zinv 6 ms of it); the double-float step from 16.7 to 15.5 ms.
-// Plans of 24 (16) points per thread need 168 registers; 128-thread blocks
-// keep three of them on an SM.
+// What bounds them (GB300, counters at 255x64x255): k_xrow_x instruction issue
+// with the 12 warps per SM that its rows' shared memory allows (46% of the
+// issue slots; fixed-latency and shared-memory waits the rest); the z kernels
+// the same, and the FP64 pipe's conversions of their inputs and outputs (60%
+// busy).  Not memory: 2 TB/s in k_zinv_x.  Against the FP64-pipe transforms
+// they replace, the FP64 step went from 44.9 to 15.3 ms at 127x192x127 (k_xrow
+// 4.7, k_zfwd 1.55, k_zinv 0.85 of it; with the right-hand sides' change) and
+// from 262 to 82 ms at 255x256x255 (28.3, 9.4, 5.1); the double-float step
+// from 16.7 to 14.4 ms at 127x192x127.  In-place packing by pairs of entries,
+// one code path for the three inverse rows: k_xrow_x 38.7 -> 28.3 ms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -83,38 +85,44 @@ __device__ __forceinline__ void xblock_max_atomic(double v, double* target) {
 
 // columns per z block: 128 threads, at most 32 columns
 template <int TPR> constexpr int fx_zcols() { return (128 / TPR) < 32 ? (128 / TPR) : 32; }
-// shared memory per x row in elements: u, v (and w without WREG) in physical
-// space, the padded exchange buffer, then pad so that a block's transposing
-// accesses (NR rows of consecutive elements) spread over the banks: a
-// wavefront of 16-byte elements is 8 lanes, NR rows of 8 / NR elements
-template <int M, int TPR, bool WREG> constexpr int fx_row_stride(int nr) {
-  int s = (WREG ? 3 : 4) * M + TPR;
+// shared memory per x row in elements: u, v in physical space, the padded
+// exchange buffer, then pad so that a block's transposing accesses (NR rows
+// of consecutive elements) spread over the banks: a wavefront of 16-byte
+// elements is 8 lanes, NR rows of 8 / NR elements
+template <int M, int TPR> constexpr int fx_row_stride(int nr) {
+  int s = 3 * M + TPR;
   while (s % 8 != (nr < 8 ? 8 / nr : 1)) ++s;
   return s;
 }
-// rows per x block: at most 32 and 128 threads, within a third (WREG) or half
-// of an SM's 228 KB (1 KB reserved per block)
-template <int M, int TPR, bool WREG> constexpr int fx_xrows() {
+// rows per x block: at most 32 and 128 threads, within a third of an SM's 228
+// KB (1 KB reserved per block)
+template <int M, int TPR> constexpr int fx_xrows() {
   int nr = 32;
-  const int budget = 233472 / (WREG ? 3 : 2) - 1024;
-  while (nr > 1 && (nr * fx_row_stride<M, TPR, WREG>(nr) * 16 > budget || nr * TPR > 128)) nr /= 2;
+  const int budget = 233472 / 3 - 1024;
+  while (nr > 1 && (nr * fx_row_stride<M, TPR>(nr) * 16 > budget || nr * TPR > 128)) nr /= 2;
   while (nr * TPR < 32) nr *= 2;
   return nr;
 }
-// resident blocks the registers are capped for: what shared memory allows,
-// at most 12 warps per SM (168 registers)
-template <int M, int TPR, bool WREG> constexpr int fx_xminb() {
-  const int nr = fx_xrows<M, TPR, WREG>();
-  const int by_smem = 233472 / (nr * fx_row_stride<M, TPR, WREG>(nr) * 16 + 1024);
-  const int by_regs = 384 / (nr * TPR);
+// resident blocks the registers are capped for: what shared memory allows, at
+// most 12 warps per SM (168 registers) with 12 points per thread, 16 with 8
+template <int M, int TPR> constexpr int fx_xminb() {
+  const int nr = fx_xrows<M, TPR>();
+  const int by_smem = 233472 / (nr * fx_row_stride<M, TPR>(nr) * 16 + 1024);
+  const int by_regs = (M / TPR == 8 ? 512 : 384) / (nr * TPR);
   const int b = by_smem < by_regs ? by_smem : by_regs;
   return b < 1 ? 1 : b;
+}
+// resident z blocks: as many as the registers allow, 12, 20 or 24 warps per SM
+// with 24, 12 or 8 points per thread (k_zfwd_x at nzd = 256 and 79x101x75:
+// 0.382 ms per step with 12 warps, 0.322 with 20, 0.300 with 24)
+template <int E, int TPR, int NC> constexpr int fx_zminb() {
+  return (E == 24 ? 384 : E == 12 ? 640 : 768) / (NC * TPR);
 }
 
 }  // namespace
 
 template <int E, int TPR, int NC>
-__global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zinv_x(const double2* __restrict__ V,
+__global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zinv_x(const double2* __restrict__ V,
                                                                        double2* __restrict__ Zb,
                                                                        const fx2* __restrict__ tw, Dims d, int plane0,
                                                                        int ix_lo, int ix_hi) {
@@ -149,7 +157,11 @@ __global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zinv_x(const dou
   const int S = emax == 0 ? 0 : fx_scale_sum<double>(emax, B, 62);
   fx2 a[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) a[e] = fx_load<double>(raw[e], S1);
+  for (int e = 0; e < E; ++e) {  // conversions only where there is a mode: they fill half the FP64 pipe
+    const int jz = t + TPR * e;
+    a[e] = fx2{0, 0};
+    if (jz <= nz || jz >= N - nz) a[e] = fx_load<double>(raw[e], S1);
+  }
   const int So = S - 2;  // one pass at quarter scale
   const int mode = fx_mode<double>(So, emax == In::kExpMax);
   double2* dst = Zb + col * N;
@@ -165,7 +177,7 @@ __global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zinv_x(const dou
 }
 
 template <typename T, int E, int TPR, int NC>
-__global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zfwd_x(const double2* __restrict__ Pb,
+__global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zfwd_x(const double2* __restrict__ Pb,
                                                                        typename C2<T>::t* __restrict__ VV,
                                                                        const fx2* __restrict__ tw, Dims d, int plane0) {
   using V2 = typename C2<T>::t;
@@ -205,9 +217,10 @@ __global__ void __launch_bounds__(NC * TPR, 384 / (NC * TPR)) k_zfwd_x(const dou
 }
 
 // Row layout in shared memory: u and v in physical space (M each), then the
-// padded exchange buffer X (M + TPR), which first holds the row's w spectrum;
-// without WREG w's physical values take a third slot before X.
-template <int E, int TPR, int NR, int MINB, bool WREG>
+// padded exchange buffer X (M + TPR), which first holds the row's w spectrum.
+// w stays in registers: the last pass leaves each thread exactly the elements
+// the products' forward transforms start from.
+template <int E, int TPR, int NR, int MINB>
 __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __restrict__ Zb,
                                                            double2* __restrict__ Pb,
                                                            const fx2* __restrict__ tw, const fx2* __restrict__ twh,
@@ -217,17 +230,22 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
   using Io = FxIo<double>;
   static_assert(sizeof(V2) == sizeof(fx2), "rows are converted in place");
   constexpr int M = E * TPR;
-  constexpr int RS = fx_row_stride<M, TPR, WREG>(NR);
+  constexpr int RS = fx_row_stride<M, TPR>(NR);
   constexpr int NT = NR * TPR;
-  // bits of the physical values: their products, 2 kBits - 64 bits, are the
-  // forward transform's inputs (whose outputs stay below 2^61 for the unpacking)
-  constexpr int kBits = (fx_forward_bits(E, TPR, 61) + 64) / 2;
+  // physical values below 2^60: their products are below 2^56, and after the
+  // forward transform's first pass (24 points at most) below 2^62; before its
+  // other passes they are scaled by their actual largest value to kMid bits,
+  // from which no later value exceeds 2^62 and the outputs 2^61 (for the
+  // unpacking)
+  constexpr int kBits = 60, kMid = fx_bits(fx_growth(E, TPR, false), 61);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V2* S = reinterpret_cast<V2*>(smem_raw);
   fx2* Sf = reinterpret_cast<fx2*>(smem_raw);
   const int row = threadIdx.x / TPR, t = threadIdx.x % TPR;
   fx2* U = Sf + row * RS;
-  fx2* X = U + (WREG ? 2 : 3) * M;  // the exchange buffer; without WREG w's slot sits before it
+  fx2* X = U + 2 * M;  // the exchange buffer; without WREG w's slot sits before it
+  __shared__ int red[TPR > 32 ? NR * (TPR / 32) : 1];
+  int* scratch = red + (TPR > 32 ? row * (TPR / 32) : 0);
   const int nx = d.nx, nxp = nx + 1, nzd = d.nzd;
   const int plane = plane0 + blockIdx.y;
   const int jz0 = blockIdx.x * NR;
@@ -246,44 +264,41 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
   __syncthreads();
   int su = 0, sv = 0, sw = 0;  // scales of u, v, w in physical space
   int bad = 0;                 // bit c: component c of this row is not finite
-  fx2 w[WREG ? E : 1];  // with WREG: w in physical space, w[e] at x pair t + TPR e
-  // one component: the spectrum in its slot to physical values in a[]
-  auto inverse = [&](int c, fx2 (&a)[E]) {
+  fx2 w[E];                    // w in physical space, w[e] at x pair t + TPR e
+  // w first: its spectrum sits in the exchange buffer
+#pragma unroll 1
+  for (int cc = 0; cc < 3; ++cc) {
+    const int c = cc == 0 ? 2 : cc - 1;
     fx2* F = U + c * M;
-    const V2* Fr = reinterpret_cast<const V2*>(F);
+    V2* Fr = reinterpret_cast<V2*>(F);
     int emax = 0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int n = t + TPR * e;
-      if (n <= nx) {
-        const V2 v = Fr[n];
-        emax = max(emax, max(Io::expo(v.x), Io::expo(v.y)));
-      }
-    }
-    emax = group_reduce<kRedMax, TPR>(emax, nullptr, t);
+#pragma unroll 4
+    for (int n = t; n <= nx; n += TPR) emax = max(emax, max(Io::expo(Fr[n].x), Io::expo(Fr[n].y)));
+    emax = group_reduce<kRedMax, TPR>(emax, scratch, t);
     // |re|, |im| < 2^57, so that the packed |re|, |im| stay below 2^60
     const int s0 = emax == 0 ? 0 : 57 - (emax - Io::kBias + 1);
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int n = t + TPR * e;
-      if (n <= nx) F[n] = fx_load<double>(Fr[n], s0);
-    }
-    group_sync<TPR>();
-    // c2r by the half-length packing
-    //   Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) e^{+i pi k / M}
-    // (only Re of the kx = 0 entry; the x zero band kx > nx, dnsdata.f90:535)
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int n = t + TPR * e;
+    // c2r by the half-length packing, in place and two entries at a time
+    // (only Re of the kx = 0 entry; the x zero band kx > nx, dnsdata.f90:535):
+    // with s = X_k + conj X_{M-k} and r = i (X_k - conj X_{M-k}) e^{+i pi k/M}
+    //   Z_k = s + r,  Z_{M-k} = conj(s - r)
+#pragma unroll 2
+    for (int k = t; k <= M / 2; k += TPR) {
+      const int kc = M - k;
       fx2 xk{0, 0}, xm{0, 0};
-      if (n <= nx) xk = F[n];
-      if (n == 0) xk.y = 0;
-      else if (M - n <= nx) {
-        xm = F[M - n];
+      if (k <= nx) xk = fx_load<double>(Fr[k], s0);
+      if (k == 0) xk.y = 0;
+      else if (kc <= nx) {
+        xm = fx_load<double>(Fr[kc], s0);
         xm.y = -xm.y;
       }
-      a[e] = (xk + xm) + mul_is<+1>(fx_cmul4<+1>(xk - xm, fx_ldw(twh + n)));
+      const fx2 s = xk + xm, r = mul_is<+1>(fx_cmul4<+1>(xk - xm, fx_ldw(twh + k)));
+      F[k] = s + r;
+      if (k > 0 && kc != k) F[kc] = fx2{s.x - r.x, r.y - s.y};
     }
+    group_sync<TPR>();
+    fx2 a[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) a[e] = F[t + TPR * e];
     // the scales of pass 1 (its values are bounded by the largest sum of
     // |re| + |im| over a thread) and of the later passes (the sum over the
     // row), both sums below 2^61: shifts d1, then d2
@@ -291,12 +306,12 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
 #pragma unroll
     for (int e = 0; e < E; ++e)
       b1 += (unsigned)(abs(fx_up(a[e].x)) >> 7) + (unsigned)(abs(fx_up(a[e].y)) >> 7) + 2u;
-    const unsigned bs = (unsigned)group_reduce<kRedSum, TPR>((int)b1, nullptr, t);
-    b1 = (unsigned)group_reduce<kRedMax, TPR>((int)b1, nullptr, t);
+    const unsigned bs = (unsigned)group_reduce<kRedSum, TPR>((int)b1, scratch, t);
+    b1 = (unsigned)group_reduce<kRedMax, TPR>((int)b1, scratch, t);
     const int d1 = max(0, 32 - __clz((int)b1) + 39 - 61), d2 = max(d1, 32 - __clz((int)bs) + 39 - 61) - d1;
 #pragma unroll
     for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], d1);
-    group_sync<TPR>();  // every read of the spectrum before its slot or X is written
+    group_sync<TPR>();  // every read of the packed row before its slot or X is written
     rfft_regs<E, TPR, +1>(a, X, t, tw, [&] {
 #pragma unroll
       for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], d2);
@@ -308,8 +323,7 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
       const int hx = fx_up(a[e].x), hy = fx_up(a[e].y);
       m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
     }
-    m = group_reduce<kRedOr, TPR>(m, nullptr, t);
-    static_assert(kBits >= 60, "values below 2^60 are shifted left");
+    m = group_reduce<kRedOr, TPR>(m, scratch, t);
     const int sh = __clz(m) - (64 - kBits);
 #pragma unroll
     for (int e = 0; e < E; ++e) a[e] = fx2{a[e].x << sh, a[e].y << sh};
@@ -318,19 +332,17 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
     else if (c == 1) sv = sc;
     else sw = sc;
     if (emax == Io::kExpMax) bad |= 1 << c;
-  };
-  if constexpr (WREG) inverse(2, w);
-#pragma unroll 1
-  for (int c = 0; c < (WREG ? 2 : 3); ++c) {
-    fx2 a[E];
-    inverse(c, a);
+    if (cc == 0) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) U[c * M + t + TPR * e] = a[e];
+      for (int e = 0; e < E; ++e) w[e] = a[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) F[t + TPR * e] = a[e];
+    }
   }
   // each thread reads back only its own physical values
   auto val = [&](int c, int e) -> fx2 {
-    if (WREG && c == 2) return w[WREG ? e : 0];
-    return U[c * M + t + TPR * e];
+    return c == 2 ? w[e] : U[c * M + t + TPR * e];
   };
   // CFL (dnsdata.f90:552-556) over the physical values of this row, in FP64
   if (compute_cfl) {
@@ -356,21 +368,21 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
     if (inf) cfl = (double)INFINITY;  // a non-finite velocity shows up as an infinite CFL
     xblock_max_atomic(cfl, &sc->cfl);
   }
-  // products (dnsdata.f90:581-584), with WREG those with w first (w then
-  // dies): ww, vw, uw, uu, vv, uv -> Pb slots 2, 4, 5, 0, 1, 3; `factor`
+  // products (dnsdata.f90:581-584), those with w first (w then dies): ww,
+  // vw, uw, uu, vv, uv -> Pb slots 2, 4, 5, 0, 1, 3; `factor`
   // enters in the unpacking: g = (factor/2) 2^-fac.exp in [1/2, 1) as fac
   // and in twh[M + k] = g e^{-i pi k/M}
 #pragma unroll 1
   for (int q = 0; q < 6; ++q) {
-    const int p = !WREG ? q : (q == 0 ? 2 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 0 : q == 4 ? 1 : 3);
+    const int p = q == 0 ? 2 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 0 : q == 4 ? 1 : 3;
     // factors of product p (uu, vv, ww, uv, vw, uw)
     const int fa = p < 3 ? p : (p == 5 ? 0 : p - 3);
     const int fb = p < 3 ? p : (p == 3 ? 1 : 2);
     fx2 a[E];
-    if (WREG && q < 3) {
+    if (q < 3) {
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const fx2 y = w[WREG ? e : 0], x = q == 0 ? y : U[fa * M + t + TPR * e];
+        const fx2 y = w[e], x = q == 0 ? y : U[fa * M + t + TPR * e];
         a[e] = fx2{fx_mul(x.x, y.x), fx_mul(x.y, y.y)};
       }
     } else {
@@ -382,35 +394,49 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
     }
     const int sa = fa == 0 ? su : (fa == 1 ? sv : sw), sb = fb == 0 ? su : (fb == 1 ? sv : sw);
     const bool nf = ((bad >> fa) | (bad >> fb)) & 1;
-    const int So = sa + sb - 64 - 2 * (1 + fx_quarters(E, TPR)) - fac.exp;
-    const int mode = fx_mode<double>(So, nf);
-    rfft<E, TPR, -1>(a, X, t, tw, [&](int o, fx2 v) { X[o] = v; });
-    group_sync<TPR>();
-    // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586), at quarter scale:
-    //   X = g (Z_k + conj Z_{M-k}) + (g w_k) (-i) (Z_k - conj Z_{M-k})
-    V2 o[E];
+    int mid = 0;  // shift to the left between passes 1 and 2
+    rfft<E, TPR, -1, true>(a, X, t, tw, [&](int o, fx2 v) { X[o] = v; }, [&] {
+      int m = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int k = t + TPR * e;
-      if (k <= nx) {
-        const fx2 zk = X[k], zc = X[k == 0 ? 0 : M - k];
-        const fx2 sm{zk.x + zc.x, zk.y - zc.y}, df{zk.x - zc.x, zk.y + zc.y};
-        const fx2 rot = fx_cmul<-1>(fx2{df.y, -df.x}, fx_ldw(twh + M + k));
-        o[e] = fx_store<double>(fx2{fx_mad(rot.x, sm.x, fac.gh, fac.gl), fx_mad(rot.y, sm.y, fac.gh, fac.gl)}, So, mode);
+      for (int e = 0; e < E; ++e) {
+        const int hx = fx_up(a[e].x), hy = fx_up(a[e].y);
+        m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
       }
-    }
-    group_sync<TPR>();
+      m = group_reduce<kRedOr, TPR>(m, scratch, t);
+      mid = kMid - (64 - __clz(m));
+      if (mid >= 0) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int k = t + TPR * e;
-      if (k <= nx) reinterpret_cast<V2*>(X)[k] = o[e];
+        for (int e = 0; e < E; ++e) a[e] = fx2{a[e].x << mid, a[e].y << mid};
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], -mid);
+      }
+    });
+    // the passes after the first and the unpacking are at quarter scale
+    const int So = sa + sb - 64 + mid - 2 * rplan_passes(E, TPR) - fac.exp;
+    const int mode = fx_mode<double>(So, nf);
+    group_sync<TPR>();
+    // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586), at quarter scale, in
+    // place and two entries at a time: with s = g (Z_k + conj Z_{M-k}) and
+    // r = (g w_k) (-i) (Z_k - conj Z_{M-k})
+    //   X_k = s + r,  X_{M-k} = conj(s - r)
+    V2* Xr = reinterpret_cast<V2*>(X);
+#pragma unroll 2
+    for (int k = t; k <= min(M / 2, nx); k += TPR) {
+      const int kc = M - k;
+      const fx2 zk = X[k], zc = X[k == 0 ? 0 : kc];
+      const fx2 sm{zk.x + zc.x, zk.y - zc.y}, df{zk.x - zc.x, zk.y + zc.y};
+      const fx2 r = fx_cmul<-1>(fx2{df.y, -df.x}, fx_ldw(twh + M + k));
+      const fx2 s{fx_mad(0, sm.x, fac.gh, fac.gl), fx_mad(0, sm.y, fac.gh, fac.gl)};
+      Xr[k] = fx_store<double>(s + r, So, mode);
+      if (kc <= nx && kc != k) Xr[kc] = fx_store<double>(fx2{s.x - r.x, r.y - s.y}, So, mode);
     }
     __syncthreads();
     // xTOz: the block's rows of product p, NR consecutive jz per kx
     V2* dst = Pb + ((size_t)p * d.nplanes + plane) * nxp * nzd + jz0;
     for (int i = threadIdx.x; i < nxp * NR; i += NT) {
       const int r = i % NR, k = i / NR;
-      if (r < nrow) dst[(size_t)k * nzd + r] = S[r * RS + (WREG ? 2 : 3) * M + k];
+      if (r < nrow) dst[(size_t)k * nzd + r] = S[r * RS + 2 * M + k];
     }
     __syncthreads();
   }
@@ -421,7 +447,7 @@ namespace {
 template <typename T, int N>
 void fx_launch_z(const ConvLaunch& L, cudaStream_t s, int stage) {
   using V2 = typename C2<T>::t;
-  constexpr int E = RLen<N>::E, TPR = RLen<N>::TPR, NC = fx_zcols<TPR>();
+  constexpr int E = FxLen<N>::E, TPR = FxLen<N>::TPR, NC = fx_zcols<TPR>();
   const size_t sm = (size_t)NC * rbuf_size<E, TPR>() * sizeof(fx2);
   const Dims& d = L.d;
   if constexpr (std::is_same<T, double>::value) {
@@ -440,13 +466,12 @@ void fx_launch_z(const ConvLaunch& L, cudaStream_t s, int stage) {
 
 template <int M>
 void fx_launch_x(const ConvLaunch& L, cudaStream_t s) {
-  constexpr int E = FxXLen<M>::E, TPR = FxXLen<M>::TPR;
-  constexpr bool WREG = FxXLen<M>::WREG;
-  constexpr int NR = fx_xrows<M, TPR, WREG>(), MINB = fx_xminb<M, TPR, WREG>();
-  const size_t sm = (size_t)NR * fx_row_stride<M, TPR, WREG>(NR) * sizeof(fx2);
+  constexpr int E = FxLen<M>::E, TPR = FxLen<M>::TPR;
+  constexpr int NR = fx_xrows<M, TPR>(), MINB = fx_xminb<M, TPR>();
+  const size_t sm = (size_t)NR * fx_row_stride<M, TPR>(NR) * sizeof(fx2);
   const Dims& d = L.d;
   dim3 grid((d.nzd + NR - 1) / NR, L.nplanes);
-  k_xrow_x<E, TPR, NR, MINB, WREG><<<grid, NR * TPR, sm, s>>>((const double2*)L.Zb, (double2*)L.Pb,
+  k_xrow_x<E, TPR, NR, MINB><<<grid, NR * TPR, sm, s>>>((const double2*)L.Zb, (double2*)L.Pb,
                                                               (const fx2*)L.twxr, (const fx2*)L.twhx, d, L.fxfac,
                                                               L.plane0, L.compute_cfl, L.rdy, L.sc);
 }
@@ -459,16 +484,15 @@ template <typename K> cudaError_t fx_allow_smem(K* kernel, size_t bytes, bool ma
 }
 // shared-memory limits of one length's kernels
 template <typename T, int N> cudaError_t fx_limits_z() {
-  constexpr int E = RLen<N>::E, TPR = RLen<N>::TPR, NC = fx_zcols<TPR>();
+  constexpr int E = FxLen<N>::E, TPR = FxLen<N>::TPR, NC = fx_zcols<TPR>();
   const size_t sm = (size_t)NC * rbuf_size<E, TPR>() * sizeof(fx2);
   cudaError_t e = std::is_same<T, double>::value ? fx_allow_smem(k_zinv_x<E, TPR, NC>, sm) : cudaSuccess;
   return e == cudaSuccess ? fx_allow_smem(k_zfwd_x<T, E, TPR, NC>, sm) : e;
 }
 template <int M> cudaError_t fx_limits_x() {
-  constexpr int E = FxXLen<M>::E, TPR = FxXLen<M>::TPR;
-  constexpr bool WREG = FxXLen<M>::WREG;
-  constexpr int NR = fx_xrows<M, TPR, WREG>(), MINB = fx_xminb<M, TPR, WREG>();
-  return fx_allow_smem(k_xrow_x<E, TPR, NR, MINB, WREG>, (size_t)NR * fx_row_stride<M, TPR, WREG>(NR) * sizeof(fx2),
+  constexpr int E = FxLen<M>::E, TPR = FxLen<M>::TPR;
+  constexpr int NR = fx_xrows<M, TPR>(), MINB = fx_xminb<M, TPR>();
+  return fx_allow_smem(k_xrow_x<E, TPR, NR, MINB>, (size_t)NR * fx_row_stride<M, TPR>(NR) * sizeof(fx2),
                        true);
 }
 

@@ -302,10 +302,10 @@ template <int P, int SIGN, bool QUARTER> __device__ __forceinline__ void fx_dft3
 // thread are scaled by a quarter inside, whose two bits let the input use
 // the word's full width; backward ones run at full scale.
 __host__ __device__ constexpr bool fx_first_quarter(int E, int SIGN) { return SIGN < 0 && (E == 16 || E == 24); }
-template <int E, int SIGN> __device__ __forceinline__ void fx_first(fx2* a) {
-  if constexpr (E == 24) fx_dft3p<8, SIGN, fx_first_quarter(E, SIGN)>(a);
+template <int E, int SIGN, bool QUARTER> __device__ __forceinline__ void fx_first(fx2* a) {
+  if constexpr (E == 24) fx_dft3p<8, SIGN, QUARTER>(a);
   else if constexpr (E == 12) fx_dft3p<4, SIGN, false>(a);
-  else if constexpr (E == 16) fx_dft16<SIGN, fx_first_quarter(E, SIGN)>(a);
+  else if constexpr (E == 16) fx_dft16<SIGN, QUARTER>(a);
   else Dft<E, fx2>::template run<SIGN>(a);
 }
 

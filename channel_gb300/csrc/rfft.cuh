@@ -93,10 +93,11 @@ template <int TPR> __device__ __forceinline__ void group_sync() {
   }
 }
 
-// pass 1: one radix-E register DFT per thread
-template <int E, int TPR, int SIGN, typename V>
+// pass 1: one radix-E register DFT per thread (fixed point: FULL at full
+// scale, else as fx_first_quarter says)
+template <int E, int TPR, int SIGN, bool FULL, typename V>
 __device__ __forceinline__ void rpass_first(V (&a)[E]) {
-  if constexpr (std::is_same<V, fx2>::value) fx_first<E, SIGN>(a);
+  if constexpr (std::is_same<V, fx2>::value) fx_first<E, SIGN, !FULL && fx_first_quarter(E, SIGN)>(a);
   else Dft<E, V>::template run<SIGN>(a);
 }
 
@@ -234,10 +235,10 @@ __device__ __forceinline__ void rpass_last_any(V (&a)[E], int t, const V* __rest
 struct RNothing {
   __device__ __forceinline__ void operator()() const {}
 };
-template <int E, int TPR, int SIGN, typename V, typename After = RNothing>
+template <int E, int TPR, int SIGN, bool FULL = false, typename V, typename After = RNothing>
 __device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __restrict__ tw, After after_first = After()) {
   constexpr int NP = rplan_passes(E, TPR);
-  rpass_first<E, TPR, SIGN>(a);
+  rpass_first<E, TPR, SIGN, FULL>(a);
   after_first();
   if constexpr (NP >= 2) {
     rpass_store<E, TPR, 0, SIGN, true>(a, buf, t, tw);
@@ -263,10 +264,10 @@ __device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __r
 // Whole transform, a[] holding the input distribution (x[t + TPR e]) on
 // entry, the outputs handed to sink(index, value).  The caller synchronises
 // the group before reusing buf.
-template <int E, int TPR, int SIGN, typename V, typename Sink, typename After = RNothing>
+template <int E, int TPR, int SIGN, bool FULL = false, typename V, typename Sink, typename After = RNothing>
 __device__ __forceinline__ void rfft(V (&a)[E], V* buf, int t, const V* __restrict__ tw, Sink sink,
                                      After after_first = After()) {
-  rfft_head<E, TPR, SIGN>(a, buf, t, tw, after_first);
+  rfft_head<E, TPR, SIGN, FULL>(a, buf, t, tw, after_first);
   rpass_last_any<E, TPR, SIGN, false>(a, t, tw, sink);
 }
 
@@ -288,12 +289,6 @@ template <> struct RLen<192> { static constexpr int E = 24, TPR = 8; };
 template <> struct RLen<384> { static constexpr int E = 24, TPR = 16; };
 template <> struct RLen<768> { static constexpr int E = 24, TPR = 32; };
 template <> struct RLen<1536> { static constexpr int E = 24, TPR = 64; };
-// lengths that the fixed-point kernels alone have
-template <> struct RLen<128> { static constexpr int E = 16, TPR = 8; };
-template <> struct RLen<256> { static constexpr int E = 16, TPR = 16; };
-template <> struct RLen<512> { static constexpr int E = 16, TPR = 32; };
-template <> struct RLen<1024> { static constexpr int E = 16, TPR = 64; };
-
 // Plans of the x-row kernel.  WREG: w's physical values stay in registers
 // next to the transform being computed (12 elements per thread, 8 for the
 // power-of-two lengths, so that three or four blocks share an SM); without
@@ -309,44 +304,61 @@ template <> struct XLen<192> { static constexpr int E = 12, TPR = 16; static con
 template <> struct XLen<384> { static constexpr int E = 12, TPR = 32; static constexpr bool WREG = true; };
 template <> struct XLen<768> { static constexpr int E = 24, TPR = 32; static constexpr bool WREG = false; };
 
-// Plans of the fixed-point x-row kernel (16-byte elements).
-template <int N> struct FxXLen;
-template <> struct FxXLen<32> { static constexpr int E = 8, TPR = 4; static constexpr bool WREG = true; };
-template <> struct FxXLen<48> { static constexpr int E = 12, TPR = 4; static constexpr bool WREG = true; };
-template <> struct FxXLen<64> { static constexpr int E = 8, TPR = 8; static constexpr bool WREG = true; };
-template <> struct FxXLen<96> { static constexpr int E = 12, TPR = 8; static constexpr bool WREG = true; };
-template <> struct FxXLen<128> { static constexpr int E = 8, TPR = 16; static constexpr bool WREG = true; };
-template <> struct FxXLen<192> { static constexpr int E = 12, TPR = 16; static constexpr bool WREG = true; };
-template <> struct FxXLen<256> { static constexpr int E = 8, TPR = 32; static constexpr bool WREG = true; };
-template <> struct FxXLen<384> { static constexpr int E = 12, TPR = 32; static constexpr bool WREG = true; };
-template <> struct FxXLen<512> { static constexpr int E = 16, TPR = 32; static constexpr bool WREG = false; };
-template <> struct FxXLen<768> { static constexpr int E = 24, TPR = 32; static constexpr bool WREG = false; };
+// Plans of the fixed-point kernels (16-byte elements): 12 or 8 points per
+// thread.  Occupancy decides: 24 (16) points need fewer passes but 168
+// registers; with 12 (8) and 102 registers k_zinv_x + k_zfwd_x went from 3.09
+// to 2.44 ms per step at nzd = 384 (127x192x127), from 16.1 to 14.4 at 768, and
+// k_xrow_x from 57 to 32 ms at nxd = 768 (383x64x383), where 24 points leave
+// shared memory for 4 warps per SM.  1536 would need five passes of 12.
+template <int N> struct FxLen;
+template <> struct FxLen<32> { static constexpr int E = 8, TPR = 4; };
+template <> struct FxLen<48> { static constexpr int E = 12, TPR = 4; };
+template <> struct FxLen<64> { static constexpr int E = 8, TPR = 8; };
+template <> struct FxLen<96> { static constexpr int E = 12, TPR = 8; };
+template <> struct FxLen<128> { static constexpr int E = 8, TPR = 16; };
+template <> struct FxLen<192> { static constexpr int E = 12, TPR = 16; };
+template <> struct FxLen<256> { static constexpr int E = 8, TPR = 32; };
+template <> struct FxLen<384> { static constexpr int E = 12, TPR = 32; };
+template <> struct FxLen<512> { static constexpr int E = 8, TPR = 64; };
+template <> struct FxLen<768> { static constexpr int E = 12, TPR = 64; };
+template <> struct FxLen<1024> { static constexpr int E = 8, TPR = 128; };
+template <> struct FxLen<1536> { static constexpr int E = 24, TPR = 64; };
 
 // Passes of a forward fixed-point transform at quarter scale (fx.cuh): every
 // one after the first, and inside the first of 16 and 24 points.
 __host__ __device__ constexpr int fx_quarters(int E, int TPR) {
   return rplan_passes(E, TPR) - 1 + (fx_first_quarter(E, -1) ? 1 : 0);
 }
-// Bits of a forward transform's largest input component: with |re|, |im| <
-// 2^bits every intermediate modulus stays below 2^62 and the outputs' below
-// 2^final.  The moduli grow by the radix of each pass over the quarter
-// scale; a first pass of 24 (16) points by 3 (4), then by 8/4 (4/4).
-__host__ __device__ constexpr int fx_forward_bits(int E, int TPR, int final_bits) {
-  double g = E == 24 ? 3.0 : E == 16 ? 4.0 : (double)E;
+// Growth of the moduli over the passes from `first` on at quarter scale, as
+// its largest value on the way and at the end; before them a factor g (a first
+// pass of 24 (16) points with its inner quarter: 3 (4), then 8/4 (4/4)).
+struct FxGrowth {
+  double most, last;
+};
+__host__ __device__ constexpr FxGrowth fx_growth(int E, int TPR, bool with_first) {
+  double g = !with_first ? 1.0 : E == 24 ? 3.0 : E == 16 ? 4.0 : (double)E;
   double mx = g;
-  if (fx_first_quarter(E, -1)) g *= E == 24 ? 2.0 : 1.0;
+  if (with_first && fx_first_quarter(E, -1)) g *= E == 24 ? 2.0 : 1.0;
   if (g > mx) mx = g;
   for (int p = 1; p < rplan_passes(E, TPR); ++p) {
     g *= rplan_radix(E, TPR, p) / 4.0;
     if (g > mx) mx = g;
   }
+  return FxGrowth{mx, g};
+}
+// Bits of the largest component with which every later modulus stays below
+// 2^62 and the outputs' below 2^final.
+__host__ __device__ constexpr int fx_bits(FxGrowth g, int final_bits) {
   int hm = 0, hf = 0;
   double two = 1.0;
-  for (; two < 1.4143 * mx; two *= 2) ++hm;
+  for (; two < 1.4143 * g.most; two *= 2) ++hm;
   two = 1.0;
-  for (; two < 1.4143 * g; two *= 2) ++hf;
+  for (; two < 1.4143 * g.last; two *= 2) ++hf;
   const int a = 62 - hm, b = final_bits - hf;
   return a < b ? a : b;
+}
+__host__ __device__ constexpr int fx_forward_bits(int E, int TPR, int final_bits) {
+  return fx_bits(fx_growth(E, TPR, true), final_bits);
 }
 
 inline bool xlen_plan(int n, int* E, int* TPR) {
