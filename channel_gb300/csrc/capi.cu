@@ -105,7 +105,7 @@ struct chgpu_handle {
   FxFactor fxfac{};
   double* rdy = nullptr;  // 1/dy per plane
   bool zfast = false, xfast = false;
-  int xrvar = 4;  // register-blocked x-row variant: 4 (registers for 3 blocks per SM) or 5 (for 4)
+  int xrvar = 4;  // FP32 register-blocked x-row variant: 4 (registers for 3 blocks per SM) or 5 (for 4)
   DevScalars* sc = nullptr;
   DevScalars* sc_host = nullptr;  // pinned
   cudaGraphExec_t graph = nullptr;
@@ -821,6 +821,10 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     int e_ = 0, tpr_ = 0;
     h->zfast = zplan(h->prec, nzd, &e_, &tpr_);
     h->xfast = xplan(h->prec, nxd, &e_, &tpr_);
+    // four resident blocks for the plans of 12 points a thread: 0.217 ms per
+    // step against 0.244 at 47x96x47, 1.456 : 1.536 at 127x192x127,
+    // 5.60 : 5.82 at 255x128x255; with 8 points (nxd = 64) 0.079 : 0.077
+    h->xrvar = nxd % 3 == 0 ? 5 : 4;
   }
   h->halves = d.npairs >= 65536 ? 2 : 1;
   h->solve_form = default_solve_form(d.npairs);

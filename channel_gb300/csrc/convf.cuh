@@ -58,25 +58,23 @@ __device__ __forceinline__ void rblock_max_atomic(double v, double* target) {
 
 // blocks of the z kernels: 256 threads, at most 32 columns
 template <int TPR> constexpr int z_cols() { return (256 / TPR) < 32 ? (256 / TPR) : 32; }
-// shared memory per x row: u, v (and w without WREG) in physical space,
-// the padded exchange buffer, one bank shift
-template <int M, int TPR, bool WREG> constexpr int x_row_stride() { return (WREG ? 3 : 4) * M + TPR + 1; }
+// shared memory per x row: u and v in physical space, the padded exchange
+// buffer, one bank shift
+template <int M, int TPR> constexpr int x_row_stride() { return 3 * M + TPR + 1; }
 // rows per x block: as many as keep the block's shared memory within 74 KB
-// with w in registers (three resident blocks per SM) or 102 KB without (two),
-// at least one warp, at most 256 threads
-template <int M, int TPR, bool WREG, int S> constexpr int x_rows() {
+// (three resident blocks per SM), at least one warp, at most 256 threads
+template <int M, int TPR, int S> constexpr int x_rows() {
   int nr = 32;
-  const int budget = (WREG ? 74 : 102) * 1024;
-  while (nr > 1 && (nr * x_row_stride<M, TPR, WREG>() * S > budget || nr * TPR > 256)) nr /= 2;
+  const int budget = 74 * 1024;
+  while (nr > 1 && (nr * x_row_stride<M, TPR>() * S > budget || nr * TPR > 256)) nr /= 2;
   while (nr * TPR < 32) nr *= 2;
   return nr;
 }
 // resident blocks per SM the x-row kernel's registers are capped for: as
 // many as its shared memory lets share an SM (1 KB reserved per block), at
 // most CAP (tiles x-row variant 4: 3, variant 5: 4; the autotuner times both)
-template <int M, int TPR, bool WREG, int S, int CAP> constexpr int x_minb() {
-  if (!WREG) return 1;  // no register cap: two blocks' shared memory set the residency
-  const int bytes = x_rows<M, TPR, WREG, S>() * x_row_stride<M, TPR, WREG>() * S + 1024;
+template <int M, int TPR, int S, int CAP> constexpr int x_minb() {
+  const int bytes = x_rows<M, TPR, S>() * x_row_stride<M, TPR>() * S + 1024;
   const int by_smem = 233472 / bytes;
   const int b = by_smem < CAP ? by_smem : CAP;
   return b < 1 ? 1 : b;
@@ -146,10 +144,15 @@ __global__ void __launch_bounds__(NC * TPR) k_zfwd_r(const typename C2<T>::t* __
 
 // Row layout in shared memory: u and v in physical space (M each), then the
 // padded exchange buffer X (M + TPR), which first holds the row's w
-// spectrum; without WREG w's physical values take a third slot before X.  With WREG w stays in registers after its transform: the last pass
-// leaves each thread exactly the elements the products' forward transforms
-// start from, so only u and v need shared memory.
-template <typename T, int E, int TPR, int NR, int MINB, bool WREG>
+// spectrum; w stays in registers after its transform: the last pass leaves
+// each thread exactly the elements the products' forward transforms start
+// from, so only u and v need shared memory.
+//
+// Bound by the FP32 pipe and the shared-memory exchanges together, at 12 warps
+// per SM.  At 768 points a fourth slot for w left two blocks per SM: with w in
+// registers and the unpacking in pairs 10.95 -> 8.92 ms per step
+// (383x64x383); the unpacking alone 1.63 -> 1.54 ms at 127x192x127.
+template <typename T, int E, int TPR, int NR, int MINB>
 __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>::t* __restrict__ Zb,
                                                            typename C2<T>::t* __restrict__ Pb,
                                                            const typename C2<T>::t* __restrict__ tw,
@@ -158,21 +161,20 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>:
                                                            int compute_cfl, DevScalars* sc) {
   using V2 = typename C2<T>::t;
   constexpr int M = E * TPR;
-  constexpr int RS = x_row_stride<M, TPR, WREG>();
+  constexpr int RS = x_row_stride<M, TPR>();
   constexpr int NT = NR * TPR;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V2* S = reinterpret_cast<V2*>(smem_raw);
   const int row = threadIdx.x / TPR, t = threadIdx.x % TPR;
   V2* U = S + row * RS;
   V2* Vv = U + M;
-  V2* X = U + (WREG ? 2 : 3) * M;  // the exchange buffer; without WREG w's slot sits before it
+  V2* X = Vv + M;  // the exchange buffer
   const int nx = d.nx, nxp = nx + 1, nzd = d.nzd;
   const int plane = plane0 + blockIdx.y;
   const int jz0 = blockIdx.x * NR;
   const int nrow = min(NR, nzd - jz0);
   // the block's rows of the three spectra (zTOx): NR consecutive jz per kx,
-  // u into U, v into V, w into X (with WREG) or into its own slot W
-  V2* Wp = U + 2 * M;  // w in physical space without WREG
+  // u into U, v into V, w into X
   for (int c = 0; c < 3; ++c) {
     const V2* src = Zb + ((size_t)c * d.nplanes + plane) * nxp * nzd + jz0;
     const int off = c * M;
@@ -199,25 +201,18 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>:
       a[e] = ev + mul_is<+1>(od);
     }
   };
-  V2 w[WREG ? E : 1];  // with WREG: w in physical space, w[e] at x pair t + TPR e
-  if constexpr (WREG) {
-    pack(X, w);
-    group_sync<TPR>();  // every read of the w spectrum before X becomes the exchange buffer
-    rfft_regs<E, TPR, +1>(w, X, t, tw);
-  }
+  V2 w[E];  // w in physical space, w[e] at x pair t + TPR e
+  pack(X, w);
+  group_sync<TPR>();  // every read of the w spectrum before X becomes the exchange buffer
+  rfft_regs<E, TPR, +1>(w, X, t, tw);
 #pragma unroll 1
-  for (int c = 0; c < (WREG ? 2 : 3); ++c) {
-    V2* F = c == 0 ? U : (c == 1 ? Vv : Wp);
+  for (int c = 0; c < 2; ++c) {
+    V2* F = c == 0 ? U : Vv;
     V2 a[E];
     pack(F, a);
     rfft<E, TPR, +1>(a, X, t, tw, [&](int o, V2 v) { F[o] = v; });
   }
   group_sync<TPR>();
-  // w at pair t + TPR e
-  auto wv = [&](int e) -> V2 {
-    if constexpr (WREG) return w[e];
-    else return Wp[t + TPR * e];
-  };
   // CFL (dnsdata.f90:552-556) over the physical values of this row
   if (compute_cfl) {
     T cfl = T();
@@ -228,7 +223,7 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>:
 #pragma unroll
       for (int e = 0; e < E; ++e) {
         const int n = t + TPR * e;
-        const V2 u = U[n], v = Vv[n], ww = wv(e);
+        const V2 u = U[n], v = Vv[n], ww = w[e];
         const T c0 = Nm::abs(u.x) * rdx + Nm::abs(v.x) * rdy + Nm::abs(ww.x) * rdz;
         const T c1 = Nm::abs(u.y) * rdx + Nm::abs(v.y) * rdy + Nm::abs(ww.y) * rdz;
         cfl = Nm::max(cfl, Nm::max(c0, c1));
@@ -245,27 +240,44 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>:
   const T g = cst[0];
 #pragma unroll 1
   for (int q = 0; q < 6; ++q) {
-    // with WREG the products with w first (w then dies): ww, vw, uw, uu, vv, uv
-    const int p = !WREG ? q : (q == 0 ? 2 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 0 : q == 4 ? 1 : 3);
+    const int p = q == 0 ? 2 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 0 : q == 4 ? 1 : 3;
     V2 a[E];
-    if constexpr (!WREG) {
-      // factors of product p (uu, vv, ww, uv, vw, uw) from the u, v, w slots
-      const int fa = p < 3 ? p : (p == 5 ? 0 : p - 3);
-      const int fb = p < 3 ? p : (p == 3 ? 1 : 2);
-      const V2* A = U + fa * M;
-      const V2* B = U + fb * M;
+    if constexpr (E == 24) {
+      const V2* A = q < 3 ? nullptr : (q == 4 ? Vv : U);          // null: w
+      const V2* B = q == 0 ? nullptr : (q == 2 || q == 3 ? U : Vv);
+      auto factors = [&](int e, V2& x, V2& y) {
+        x = A ? A[t + TPR * e] : w[e];
+        y = B ? B[t + TPR * e] : w[e];
+      };
+      // pass 1 column by column, the products fused into the sums of its
+      // 3-point transforms: only the column's factors are live
+      constexpr int P = E / 3;
+      const T s = -Num<T>::sqrt3_2();
+      auto sums = [](T x0, T y0, T x1, T y1, T x2, T y2, T& b0, T& m, T& df) {
+        const T p0 = __fmul_rn(x0, y0), p2 = __fmul_rn(x2, y2);
+        const T t1 = fma(x1, y1, p2);
+        df = fma(x1, y1, -p2);
+        m = fma(T(-0.5f), t1, p0);
+        b0 = __fadd_rn(p0, t1);
+      };
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int n = t + TPR * e;
-        const V2 x = A[n], y = B[n];
-        a[e] = mk<V2>(x.x * y.x, x.y * y.y);
+      for (int r = 0; r < P; ++r) {
+        V2 x0, y0, x1, y1, x2, y2, m, df;
+        factors(r, x0, y0);
+        factors(r + P, x1, y1);
+        factors(r + 2 * P, x2, y2);
+        sums(x0.x, y0.x, x1.x, y1.x, x2.x, y2.x, a[r].x, m.x, df.x);
+        sums(x0.y, y0.y, x1.y, y1.y, x2.y, y2.y, a[r].y, m.y, df.y);
+        a[r + P] = mk<V2>(fma(-s, df.y, m.x), fma(s, df.x, m.y));
+        a[r + 2 * P] = mk<V2>(fma(s, df.y, m.x), fma(-s, df.x, m.y));
       }
-    } else if (q < 3) {
+      Dft<E, V2>::template after_dft3<-1>(a);
+    } else if (q < 3) {  // products rounded once, not fused into pass 1
       const V2* B = q == 1 ? Vv : U;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const V2 y = wv(e), x = q == 0 ? y : B[t + TPR * e];
-        a[e] = mk<V2>(x.x * y.x, x.y * y.y);
+        const V2 y = w[e], x = q == 0 ? y : B[t + TPR * e];
+        a[e] = mk<V2>(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
       }
     } else {
       const V2* A = q == 4 ? Vv : U;
@@ -274,40 +286,33 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_r(const typename C2<T>:
       for (int e = 0; e < E; ++e) {
         const int n = t + TPR * e;
         const V2 x = A[n], y = B[n];
-        a[e] = mk<V2>(x.x * y.x, x.y * y.y);
+        a[e] = mk<V2>(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
       }
     }
-    rfft<E, TPR, -1>(a, X, t, tw, [&](int o, V2 v) { X[o] = v; });
+    if constexpr (E != 24) rpass_first<E, TPR, -1, false>(a);
+    rfft_middle<E, TPR, -1>(a, X, t, tw);
+    rpass_last_any<E, TPR, -1, false>(a, t, tw, [&](int o, V2 v) { X[o] = v; });
     group_sync<TPR>();
-    // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586):
-    //   X = g (Z_k + conj Z_{M-k}) + (g w_k) (-i) (Z_k - conj Z_{M-k})
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int k = t + TPR * e;
-      if (k <= nx) {
-        const V2 zk = X[k];
-        const V2 zm = conjg(X[k == 0 ? 0 : M - k]);
-        const V2 sm = zk + zm, df = zk - zm;
-        const V2 wk = ldg_v(twh + 2 * M + k);
-        if constexpr (std::is_same<T, dd>::value) {
-          a[e] = scale(sm, g) + cmul(wk, mk<V2>(df.y, T() - df.x));
-        } else {
-          a[e] = mk<V2>(fma(g, sm.x, fma(wk.x, df.y, wk.y * df.x)), fma(g, sm.y, fma(wk.y, df.y, -(wk.x * df.x))));
-        }
-      }
-    }
-    group_sync<TPR>();
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int k = t + TPR * e;
-      if (k <= nx) X[k] = a[e];
+    // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586), in place and two
+    // entries at a time:
+    //   X_k = g s + r,  X_{M-k} = conj(g s - r)
+    // with s = Z_k + conj Z_{M-k}, r = (g w_k) (-i) (Z_k - conj Z_{M-k})
+#pragma unroll 2
+    for (int k = t; k <= min(M / 2, nx); k += TPR) {
+      const int kc = M - k;
+      const V2 zk = X[k], zm = conjg(X[k == 0 ? 0 : kc]);
+      const V2 sm = zk + zm, df = zk - zm;
+      const V2 wk = ldg_v(twh + 2 * M + k);
+      const T rx = fma(wk.x, df.y, wk.y * df.x), ry = fma(wk.y, df.y, -(wk.x * df.x));
+      X[k] = mk<V2>(fma(g, sm.x, rx), fma(g, sm.y, ry));
+      if (kc <= nx && kc != k) X[kc] = mk<V2>(fma(g, sm.x, -rx), -fma(g, sm.y, -ry));
     }
     __syncthreads();
     // xTOz: the block's rows of product p, NR consecutive jz per kx
     V2* dst = Pb + ((size_t)p * d.nplanes + plane) * nxp * nzd + jz0;
     for (int i = threadIdx.x; i < nxp * NR; i += NT) {
       const int r = i % NR, k = i / NR;
-      if (r < nrow) dst[(size_t)k * nzd + r] = S[r * RS + (WREG ? 2 : 3) * M + k];
+      if (r < nrow) dst[(size_t)k * nzd + r] = S[r * RS + 2 * M + k];
     }
     __syncthreads();
   }
@@ -336,13 +341,12 @@ template <typename T, int M, int CAP>
 void launch_x_len(const ConvLaunch& L, cudaStream_t s) {
   using V2 = typename C2<T>::t;
   constexpr int E = XLen<M>::E, TPR = XLen<M>::TPR;
-  constexpr bool WREG = XLen<M>::WREG;
-  constexpr int NR = x_rows<M, TPR, WREG, (int)sizeof(V2)>();
-  constexpr int MINB = x_minb<M, TPR, WREG, (int)sizeof(V2), CAP>();
-  const size_t sm = (size_t)NR * x_row_stride<M, TPR, WREG>() * sizeof(V2);
+  constexpr int NR = x_rows<M, TPR, (int)sizeof(V2)>();
+  constexpr int MINB = x_minb<M, TPR, (int)sizeof(V2), CAP>();
+  const size_t sm = (size_t)NR * x_row_stride<M, TPR>() * sizeof(V2);
   const Dims& d = L.d;
   dim3 grid((d.nzd + NR - 1) / NR, L.nplanes);
-  k_xrow_r<T, E, TPR, NR, MINB, WREG><<<grid, NR * TPR, sm, s>>>((const V2*)L.Zb, (V2*)L.Pb, (const V2*)L.twxr, (const V2*)L.twh,
+  k_xrow_r<T, E, TPR, NR, MINB><<<grid, NR * TPR, sm, s>>>((const V2*)L.Zb, (V2*)L.Pb, (const V2*)L.twxr, (const V2*)L.twh,
                                                       (const T*)L.cst, d, L.plane0, L.compute_cfl, L.sc);
 }
 
@@ -365,7 +369,7 @@ bool launch_len(const ConvLaunch& L, cudaStream_t s, int stage) {
   return true;
 }
 
-// carveout: the x-row kernel with w in registers asks for the largest
+// carveout: the x-row kernel asks for the largest
 // shared-memory carveout (three or four 74 KB blocks); the others keep the default,
 // whose larger L1 serves their twiddle loads (the largest carveout made
 // z-forward 30% slower)
@@ -385,12 +389,11 @@ cudaError_t set_limits_len() {
   if (e == cudaSuccess) e = allow_smem(k_zfwd_r<T, E, TPR, NC>, (size_t)NC * rbuf_size<E, TPR>() * sizeof(V2));
   if constexpr (x_plan<N>()) {
     constexpr int XE = XLen<N>::E, XT = XLen<N>::TPR;
-    constexpr bool WR = XLen<N>::WREG;
-    constexpr int XNR = x_rows<N, XT, WR, (int)sizeof(V2)>();
-    constexpr size_t xsm = (size_t)XNR * x_row_stride<N, XT, WR>() * sizeof(V2);
-    constexpr int MB3 = x_minb<N, XT, WR, (int)sizeof(V2), 3>(), MB4 = x_minb<N, XT, WR, (int)sizeof(V2), 4>();
-    if (e == cudaSuccess) e = allow_smem(k_xrow_r<T, XE, XT, XNR, MB3, WR>, xsm, WR);
-    if (e == cudaSuccess) e = allow_smem(k_xrow_r<T, XE, XT, XNR, MB4, WR>, xsm, WR);
+    constexpr int XNR = x_rows<N, XT, (int)sizeof(V2)>();
+    constexpr size_t xsm = (size_t)XNR * x_row_stride<N, XT>() * sizeof(V2);
+    constexpr int MB3 = x_minb<N, XT, (int)sizeof(V2), 3>(), MB4 = x_minb<N, XT, (int)sizeof(V2), 4>();
+    if (e == cudaSuccess) e = allow_smem(k_xrow_r<T, XE, XT, XNR, MB3>, xsm, true);
+    if (e == cudaSuccess) e = allow_smem(k_xrow_r<T, XE, XT, XNR, MB4>, xsm, true);
   }
   return e;
 }

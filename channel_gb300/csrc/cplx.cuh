@@ -231,8 +231,6 @@ template <typename V> struct Dft<16, V> {
 // over r2 for each k1.  w(m) is w_{3P}^m for the transform's sign.
 template <int P, typename V> struct DftComposite {
   template <int SIGN> __device__ static void run(V* a) {
-    using T = decltype(V::x);
-    constexpr int N = 3 * P;
 #pragma unroll
     for (int r2 = 0; r2 < P; ++r2) {
       V b[3] = {a[r2], a[P + r2], a[2 * P + r2]};
@@ -241,7 +239,11 @@ template <int P, typename V> struct DftComposite {
       a[P + r2] = b[1];
       a[2 * P + r2] = b[2];
     }
-    // a[k1 P + r2] holds the DFT3 output k1 of column r2
+    after_dft3<SIGN>(a);
+  }
+  // a[k1 P + r2] holds the DFT3 output k1 of column r2
+  template <int SIGN> __device__ static void after_dft3(V* a) {
+    constexpr int N = 3 * P;
 #pragma unroll
     for (int k1 = 1; k1 < 3; ++k1)
 #pragma unroll
@@ -258,7 +260,6 @@ template <int P, typename V> struct DftComposite {
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) a[k] = y[k];
-    (void)sizeof(T);
   }
 };
 template <typename V> struct Dft<6, V> : DftComposite<2, V> {};

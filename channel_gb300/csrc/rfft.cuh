@@ -228,18 +228,12 @@ __device__ __forceinline__ void rpass_last_any(V (&a)[E], int t, const V* __rest
   }
 }
 
-// Every pass but the last: a[] holds the input distribution on entry and the
-// last pass's inputs on return; buf is the group's padded exchange buffer
-// (rbuf_size elements).  after_first() runs between passes 1 and 2.  Every
-// thread of the group calls it.
-struct RNothing {
-  __device__ __forceinline__ void operator()() const {}
-};
-template <int E, int TPR, int SIGN, bool FULL = false, typename V, typename After = RNothing>
-__device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __restrict__ tw, After after_first = After()) {
+// The passes between the first and the last: a[] holds the outputs of pass 1
+// on entry and the last pass's inputs on return; buf is the group's padded
+// exchange buffer (rbuf_size elements).  Every thread of the group calls it.
+template <int E, int TPR, int SIGN, typename V>
+__device__ __forceinline__ void rfft_middle(V (&a)[E], V* buf, int t, const V* __restrict__ tw) {
   constexpr int NP = rplan_passes(E, TPR);
-  rpass_first<E, TPR, SIGN, FULL>(a);
-  after_first();
   if constexpr (NP >= 2) {
     rpass_store<E, TPR, 0, SIGN, true>(a, buf, t, tw);
     group_sync<TPR>();
@@ -259,6 +253,18 @@ __device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __r
     group_sync<TPR>();
   }
   static_assert(NP <= 4, "at most four passes");
+}
+
+// Every pass but the last, a[] holding the input distribution on entry.
+// after_first() runs between passes 1 and 2.
+struct RNothing {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <int E, int TPR, int SIGN, bool FULL = false, typename V, typename After = RNothing>
+__device__ __forceinline__ void rfft_head(V (&a)[E], V* buf, int t, const V* __restrict__ tw, After after_first = After()) {
+  rpass_first<E, TPR, SIGN, FULL>(a);
+  after_first();
+  rfft_middle<E, TPR, SIGN>(a, buf, t, tw);
 }
 
 // Whole transform, a[] holding the input distribution (x[t + TPR e]) on
@@ -289,20 +295,19 @@ template <> struct RLen<192> { static constexpr int E = 24, TPR = 8; };
 template <> struct RLen<384> { static constexpr int E = 24, TPR = 16; };
 template <> struct RLen<768> { static constexpr int E = 24, TPR = 32; };
 template <> struct RLen<1536> { static constexpr int E = 24, TPR = 64; };
-// Plans of the x-row kernel.  WREG: w's physical values stay in registers
-// next to the transform being computed (12 elements per thread, 8 for the
-// power-of-two lengths, so that three or four blocks share an SM); without
-// it w too sits in shared memory and a thread holds 24 elements (measured
-// faster at 768 points, where two 64-thread groups per row would need named
-// barriers at every exchange).
+// Plans of the x-row kernel, which holds w's physical values in registers
+// next to the transform being computed: 12 points per thread (8 for the
+// power-of-two lengths), so that three or four blocks share an SM.  At 768
+// points 24: with 12, two warps per row would need named barriers at every
+// exchange.
 template <int N> struct XLen;
-template <> struct XLen<32> { static constexpr int E = 8, TPR = 4; static constexpr bool WREG = true; };
-template <> struct XLen<48> { static constexpr int E = 12, TPR = 4; static constexpr bool WREG = true; };
-template <> struct XLen<64> { static constexpr int E = 8, TPR = 8; static constexpr bool WREG = true; };
-template <> struct XLen<96> { static constexpr int E = 12, TPR = 8; static constexpr bool WREG = true; };
-template <> struct XLen<192> { static constexpr int E = 12, TPR = 16; static constexpr bool WREG = true; };
-template <> struct XLen<384> { static constexpr int E = 12, TPR = 32; static constexpr bool WREG = true; };
-template <> struct XLen<768> { static constexpr int E = 24, TPR = 32; static constexpr bool WREG = false; };
+template <> struct XLen<32> { static constexpr int E = 8, TPR = 4; };
+template <> struct XLen<48> { static constexpr int E = 12, TPR = 4; };
+template <> struct XLen<64> { static constexpr int E = 8, TPR = 8; };
+template <> struct XLen<96> { static constexpr int E = 12, TPR = 8; };
+template <> struct XLen<192> { static constexpr int E = 12, TPR = 16; };
+template <> struct XLen<384> { static constexpr int E = 12, TPR = 32; };
+template <> struct XLen<768> { static constexpr int E = 24, TPR = 32; };
 
 // Plans of the fixed-point kernels (16-byte elements): 12 or 8 points per
 // thread.  Occupancy decides: 24 (16) points need fewer passes but 168

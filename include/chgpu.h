@@ -167,13 +167,14 @@ int chgpu_autotune(chgpu_handle* h);
  *          factorisation ahead, fused-kernel substitutions, 5: the
  *          factorisation ahead, eight threads per pair), step halves (1 or
  *          2)}.  z columns 0: the
- * register-blocked z kernels (compile-time plans for nzd = 32, 48, 64, 96,
- * 192, 384, 768, 1536); x-row variant 1-3: the generic kernel with its
- * registers capped for that many 256-thread blocks per SM, 4 and 5: the
- * register-blocked x-row kernel (nxd = 32 ... 768) with registers for 3 or
- * 4 resident blocks.  A handle starts with the register-blocked kernels
- * where they measured faster (FP32: z and x; FP64: z); the autotuner keeps
- * that choice and tunes within it, so its tiles do not change the results.
+ * register-blocked z kernels (compile-time plans: nzd = 32, 48, 64, 96, 192,
+ * 384, 768 and 1536, in FP64 and double-float also 128, 256, 512 and 1024);
+ * x-row variant 1-3: the generic kernel with its registers capped for that
+ * many 256-thread blocks per SM, 4 and 5: the register-blocked x-row kernel
+ * (the same lengths up to 768) with, in FP32, registers for 3 or 4 resident
+ * blocks.  A handle starts with the register-blocked kernels for the lengths
+ * that have a plan; the autotuner keeps that choice and tunes within it, so
+ * its tiles do not change the results.
  * Switching between generic and register-blocked kernels with
  * chgpu_set_tiles changes the rounding of the transforms (their
  * factorisations differ), not their accuracy. */
