@@ -24,7 +24,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-I", str(ROOT / "include")]
 SOURCES = ["capi.cu", "conv.cu", "convf_f32.cu", "convx_z_f64.cu",
-           "convx_z_dd.cu", "convx_x.cu", "solve.cu", "setup.cpp", "noalloc.cu", "stats.cu", "export.cu", "mlp.cu", "peaks.cu",
+           "convx_z_dd.cu", "convx_x.cu", "convx_tau.cu", "convx_tke.cu", "solve.cu", "setup.cpp", "noalloc.cu", "stats.cu", "export.cu", "mlp.cu", "peaks.cu",
            "closure.cu", "tke.cu"]
 
 

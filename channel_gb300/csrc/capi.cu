@@ -96,13 +96,12 @@ struct chgpu_handle {
   void* twz = nullptr;
   void* twx = nullptr;
   void* twh = nullptr;
-  // register-blocked transform kernels (convf.cuh; FP64 and double-float:
-  // the fixed-point ones of convx.cuh), used for the lengths with a
-  // compile-time plan: their per-pass twiddle tables
+  // register-blocked transform kernels (FP32: convf.cuh; FP64 and
+  // double-float: the fixed-point ones of convx.cuh), used for the lengths
+  // with a compile-time plan: their per-pass twiddle tables
   void* twzr = nullptr;
   void* twxr = nullptr;
-  void* twhx = nullptr;  // fixed-point pack roots
-  FxFactor fxfac{};
+  FxTables fx;  // in the mixed path only for the budget spectra
   double* rdy = nullptr;  // 1/dy per plane
   bool zfast = false, xfast = false;
   int xrvar = 4;  // FP32 register-blocked x-row variant: 4 (registers for 3 blocks per SM) or 5 (for 4)
@@ -405,27 +404,32 @@ int upload_fx_twiddles(chgpu_handle* h, void** dst, int E, int TPR) {
 }
 // tables of the fixed-point kernels for the lengths that have a plan: pass
 // twiddles, pack roots exp(-i pi k / nxd) then the same times g = factor/2 in
-// [1/2, 1) (FxFactor), 1/dy per plane
-int upload_fx_tables(chgpu_handle* h) {
+// [1/2, 1) (FxFactor)
+int upload_fx_tables(chgpu_handle* h, FxTables* T) {
   int E = 0, TPR = 0;
   if (fx_zlen_plan(h->d.nzd, &E, &TPR))
-    if (int rc = upload_fx_twiddles(h, &h->twzr, E, TPR)) return rc;
+    if (int rc = upload_fx_twiddles(h, &T->z, E, TPR)) return rc;
   const int M = h->d.nxd;
   if (fx_xlen_plan(M, &E, &TPR)) {
-    if (int rc = upload_fx_twiddles(h, &h->twxr, E, TPR)) return rc;
+    if (int rc = upload_fx_twiddles(h, &T->x, E, TPR)) return rc;
     const long double half = 0.5L / (2.0L * (long double)M * (long double)h->d.nzd);
     int ex = 0;
     const long double g = frexpl(half, &ex);
-    h->fxfac.exp = ex;
-    fx_weight(g, &h->fxfac.gh, &h->fxfac.gl);
+    T->fac.exp = ex;
+    fx_weight(g, &T->fac.gh, &T->fac.gl);
     const FxRoots root(2 * M);
     std::vector<int4> w(2 * (size_t)M);
     for (int k = 0; k < M; ++k) {
       w[k] = root(k);
       w[M + k] = root(k, g);
     }
-    if (int rc = upload_int4(h, &h->twhx, w)) return rc;
+    if (int rc = upload_int4(h, &T->pack, w)) return rc;
   }
+  return 0;
+}
+// those of the step's kernels, and 1/dy per plane
+int upload_fx_step_tables(chgpu_handle* h) {
+  if (int rc = upload_fx_tables(h, &h->fx)) return rc;
   std::vector<double> r(h->d.nplanes, 0.0);
   for (int iy = 1; iy <= h->p.ny - 1; ++iy) r[iy + 1] = 1.0 / h->tab.dy[iy];
   CK(h, cudaMalloc((void**)&h->rdy, sizeof(double) * r.size()));
@@ -512,8 +516,7 @@ ConvLaunch conv_launch(chgpu_handle* h, int compute_cfl, int products, int plane
   L.products = products;
   L.twzr = h->twzr;
   L.twxr = h->twxr;
-  L.twhx = h->twhx;
-  L.fxfac = h->fxfac;
+  L.fx = h->fx;
   L.rdy = h->rdy;
   L.zfast = h->zfast;
   L.xfast = h->xfast;
@@ -730,7 +733,7 @@ void release(chgpu_handle* h) {
   }
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->fac, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
-                  h->twz, h->twx, h->twh, h->twzr, h->twxr, h->twhx, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
+                  h->twz, h->twx, h->twh, h->twzr, h->twxr, h->fx.z, h->fx.x, h->fx.pack, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
                   h->cl_G, h->cl_Z, h->cl_P, h->cl_tau, h->cl_wd, h->cl_twz, h->cl_twx, h->cl_twh,
                   h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean,
                   h->tke_twz, h->tke_twx, h->tke_twh};
@@ -899,14 +902,14 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
       if ((rc = upload_stage_twiddles<cdd>(h, &h->twz, h->rz))) break;
       if ((rc = upload_stage_twiddles<cdd>(h, &h->twx, h->rx))) break;
       if ((rc = upload_pack_roots<cdd>(h, &h->twh, 2 * nxd, 0.5L * (long double)d.factor))) break;
-      if ((rc = upload_fx_tables(h))) break;
+      if ((rc = upload_fx_step_tables(h))) break;
       if ((rc = upload_derT<dd>(h))) break;
       if ((rc = upload_derL<double>(h))) break;
     } else {
       if ((rc = upload_stage_twiddles<double2>(h, &h->twz, h->rz))) break;
       if ((rc = upload_stage_twiddles<double2>(h, &h->twx, h->rx))) break;
       if ((rc = upload_pack_roots<double2>(h, &h->twh, 2 * nxd, 0.5L * (long double)d.factor))) break;
-      if ((rc = upload_fx_tables(h))) break;
+      if ((rc = upload_fx_step_tables(h))) break;
       if ((rc = upload_derT<double>(h))) break;
       if ((rc = upload_derL<double>(h))) break;
     }
@@ -1810,6 +1813,8 @@ int chgpu_tke_reset(chgpu_handle* h, const double* mean) {
     if (int rc = upload_stage_twiddles<double2>(h, &h->tke_twz, h->tke_rz)) return rc;
     if (int rc = upload_stage_twiddles<double2>(h, &h->tke_twx, h->tke_rx)) return rc;
     if (int rc = upload_pack_roots<double2>(h, &h->tke_twh, 2 * d.nxd, 0.5L * (long double)d.factor)) return rc;
+    if (h->prec == CHGPU_MIXED)
+      if (int rc = upload_fx_tables(h, &h->fx)) return rc;
     CK(h, tke_set_smem_limits(d.nzd, d.nxd));
     h->tke_ready = true;
   }
@@ -1872,6 +1877,7 @@ int chgpu_tke_accumulate(chgpu_handle* h, const double* pressure) {
   L.twh = (const double2*)h->tke_twh;
   L.rz = h->tke_rz;
   L.rx = h->tke_rx;
+  L.fx = h->fx;
   L.chunk = h->tke_chunk;
   launch_tke_snapshot(L, h->stream);
   CK(h, cudaGetLastError());

@@ -340,14 +340,14 @@ size_t conv_zinv_smem(int zcols, int nzd, int nzt, size_t ts) {
 size_t conv_x_smem(int xrows, int nxd, size_t ts) { return 3 * (size_t)pad32_size(3 * xrows * nxd) * ts; }
 
 template <> bool launch_convolutions_r<double>(const ConvLaunch& L, cudaStream_t s, int stage) {
-  return stage == 1 ? launch_fx_x(L, s) : launch_fx_z<double>(L, s, stage);
+  return stage != 1 ? launch_fx_z<double>(L, s, stage) : L.tau ? launch_fx_x_tau(L, s) : launch_fx_x(L, s);
 }
 // the double-float path's work buffers hold FP64 values between its three
 // fixed-point kernels, double-float ones between the generic kernels: all
 // three stages take the same family
 template <> bool launch_convolutions_r<dd>(const ConvLaunch& L, cudaStream_t s, int stage) {
-  if (!L.zfast || !L.xfast || L.tau) return false;
-  return stage == 0 ? launch_fx_z<double>(L, s, 0) : stage == 1 ? launch_fx_x(L, s) : launch_fx_z<dd>(L, s, 2);
+  if (!L.zfast || !L.xfast) return false;
+  return stage == 2 ? launch_fx_z<dd>(L, s, 2) : launch_convolutions_r<double>(L, s, stage);
 }
 
 template <typename T>
@@ -355,9 +355,9 @@ void launch_convolutions(const ConvLaunch& L, cudaStream_t s, int stage) {
   using V2 = typename C2<T>::t;
   const Dims& d = L.d;
   const int nxp = d.nx + 1;
-  // lengths with a register-blocked plan (the closure's stresses go through
-  // the x-row kernel below)
-  if ((stage == 1 ? (L.xfast && !L.tau) : L.zfast) && launch_convolutions_r<T>(L, s, stage)) return;
+  // lengths with a register-blocked plan (in FP32 the closure's stresses go
+  // through the x-row kernel below)
+  if ((stage == 1 ? L.xfast : L.zfast) && launch_convolutions_r<T>(L, s, stage)) return;
   if (stage == 0) {
     const int ncol = L.ix_hi - L.ix_lo;
     dim3 grid((ncol + L.zcols - 1) / L.zcols, L.nplanes, 3);
@@ -434,6 +434,7 @@ cudaError_t conv_set_smem_limits(int prec, int nzd, int nxd) {
   }
   if ((e = fx_z_smem_limits<double>(nzd))) return e;
   if ((e = fx_x_smem_limits(nxd))) return e;
+  if ((e = fx_x_tau_smem_limits(nxd))) return e;
   if (prec == CHGPU_FP64) return generic_limits<double>(optin);
   if ((e = fx_z_smem_limits<dd>(nzd))) return e;
   return generic_limits<dd>(optin);

@@ -5,7 +5,7 @@ namespace chgpu {
 
 bool launch_fx_x(const ConvLaunch& L, cudaStream_t s) {
   switch (L.d.nxd) {
-#define CHGPU_LEN(N) case N: fx_launch_x<N>(L, s); return true;
+#define CHGPU_LEN(N) case N: fx_launch_x<N, false>(L, s); return true;
     CHGPU_FX_XLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
     default: return false;
@@ -13,7 +13,7 @@ bool launch_fx_x(const ConvLaunch& L, cudaStream_t s) {
 }
 cudaError_t fx_x_smem_limits(int nxd) {
   switch (nxd) {
-#define CHGPU_LEN(N) case N: return fx_limits_x<N>();
+#define CHGPU_LEN(N) case N: return fx_limits_x<N, false>();
     CHGPU_FX_XLENGTHS(CHGPU_LEN)
 #undef CHGPU_LEN
     default: return cudaSuccess;

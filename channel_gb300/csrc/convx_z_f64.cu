@@ -20,4 +20,13 @@ template <> cudaError_t fx_z_smem_limits<double>(int nzd) {
   }
 }
 
+bool launch_fx_tke_z(const TkeLaunch& L, int p0, int planes, bool inverse, cudaStream_t s) {
+  switch (L.d.nzd) {
+#define CHGPU_LEN(N) case N: fx_launch_tke_z<N>(L, p0, planes, inverse, s); return true;
+    CHGPU_FX_ZLENGTHS(CHGPU_LEN)
+#undef CHGPU_LEN
+    default: return false;
+  }
+}
+
 }  // namespace chgpu

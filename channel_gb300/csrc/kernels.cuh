@@ -33,6 +33,13 @@ struct FxFactor {
   int gh, gl, exp;
 };
 
+// Tables of the fixed-point kernels: pass twiddles of the z and x lengths,
+// pack roots of the x length, factor/2; null for a length without a plan.
+struct FxTables {
+  void *z = nullptr, *x = nullptr, *pack = nullptr;
+  FxFactor fac{};
+};
+
 struct ConvLaunch {
   Dims d;
   RadixDev rz, rx;
@@ -59,10 +66,8 @@ struct ConvLaunch {
   const void* twzr;
   const void* twxr;
   int zfast, xfast;
-  // the fixed-point kernels of the FP64 and double-float paths: pack roots,
-  // factor/2, 1/dy per plane
-  const void* twhx;
-  FxFactor fxfac;
+  // the fixed-point kernels of the FP64 and double-float paths: 1/dy per plane
+  FxTables fx;
   const double* rdy;
 };
 
@@ -85,10 +90,12 @@ template <typename T> bool launch_fx_z(const ConvLaunch& L, cudaStream_t s, int 
 template <> bool launch_fx_z<double>(const ConvLaunch& L, cudaStream_t s, int stage);
 template <> bool launch_fx_z<dd>(const ConvLaunch& L, cudaStream_t s, int stage);
 bool launch_fx_x(const ConvLaunch& L, cudaStream_t s);
+bool launch_fx_x_tau(const ConvLaunch& L, cudaStream_t s);  // with the closure's stresses (convx_tau.cu)
 template <typename T> cudaError_t fx_z_smem_limits(int nzd);
 template <> cudaError_t fx_z_smem_limits<double>(int nzd);
 template <> cudaError_t fx_z_smem_limits<dd>(int nzd);
 cudaError_t fx_x_smem_limits(int nxd);
+cudaError_t fx_x_tau_smem_limits(int nxd);
 #define CHGPU_FX_ZLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536)
 #define CHGPU_FX_XLENGTHS(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768)
 // dynamic shared memory of the z-transform and x-row kernels (padded buffers)
@@ -184,8 +191,14 @@ struct TkeLaunch {
   const double2* twx;
   const double2* twh;
   RadixDev rz, rx;
+  FxTables fx;  // of the fixed-point kernels
   int chunk;  // planes per chunk
 };
+// the transforms of `planes` planes from p0 on by the fixed-point kernels
+// (convx_z_f64.cu, convx_tke.cu); false when the length has no plan
+bool launch_fx_tke_z(const TkeLaunch& L, int p0, int planes, bool inverse, cudaStream_t s);
+bool launch_fx_tke_x(const TkeLaunch& L, int planes, cudaStream_t s);
+cudaError_t fx_tke_x_smem_limits(int nxd);
 void launch_tke_snapshot(const TkeLaunch& L, cudaStream_t s);
 cudaError_t tke_set_smem_limits(int nzd, int nxd);
 size_t tke_z_smem(int nzd);

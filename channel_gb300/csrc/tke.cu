@@ -18,7 +18,10 @@
 //                  pressure field, pstrain and PHIptrsp for the six pairs
 //                  uu, vv, ww, uv, vw, uw (:161-180, :230-233), added to
 //                  the running sums acc[term][pair][plane][kz].
-// Everything is FP64 (the reference's arithmetic), in every precision path.
+// Everything is FP64 (the reference's arithmetic), in every precision path;
+// lengths with a compile-time plan take the fixed-point kernels of convx.cuh
+// instead of the three here (a sample at 127x192x127: z-inverses 11.4 -> 1.09
+// ms, x rows 16.1 -> 3.36, z-forward 2.83 -> 0.26, of 33.7 -> 8.05 in all).
 #include <cuda_runtime.h>
 
 #include "chgpu_internal.h"
@@ -216,6 +219,8 @@ cudaError_t tke_set_smem_limits(int nzd, int nxd) {
     e = cudaFuncSetAttribute(k_tke_zfwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tke_z_smem(nzd));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_tke_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tke_x_smem(nxd));
+  if (e == cudaSuccess) e = fx_z_smem_limits<double>(nzd);
+  if (e == cudaSuccess) e = fx_tke_x_smem_limits(nxd);
   return e;
 }
 
@@ -228,10 +233,14 @@ void launch_tke_snapshot(const TkeLaunch& L, cudaStream_t s) {
   const int nxp = d.nx + 1;
   for (int p0 = 0; p0 < d.nplanes; p0 += L.chunk) {
     const int C = d.nplanes - p0 < L.chunk ? d.nplanes - p0 : L.chunk;
-    k_tke_zinv<<<dim3(nxp, C, 12), 256, tke_z_smem(d.nzd), s>>>(L.W, L.Zt, L.twz, d, L.rz, p0, L.chunk);
-    k_tke_x<<<dim3(d.nzd, C), 256, tke_x_smem(d.nxd), s>>>(L.Zt, L.Xt, L.twx, L.twh, d, L.rx, 0.5 * d.factor,
-                                                          L.chunk);
-    k_tke_zfwd<<<dim3(nxp, C, 3), 256, tke_z_smem(d.nzd), s>>>(L.Xt, L.N3, L.twz, d, L.rz, p0, L.chunk);
+    // the fixed-point kernels for the lengths with a plan
+    if (!launch_fx_tke_z(L, p0, C, true, s))
+      k_tke_zinv<<<dim3(nxp, C, 12), 256, tke_z_smem(d.nzd), s>>>(L.W, L.Zt, L.twz, d, L.rz, p0, L.chunk);
+    if (!launch_fx_tke_x(L, C, s))
+      k_tke_x<<<dim3(d.nzd, C), 256, tke_x_smem(d.nxd), s>>>(L.Zt, L.Xt, L.twx, L.twh, d, L.rx, 0.5 * d.factor,
+                                                            L.chunk);
+    if (!launch_fx_tke_z(L, p0, C, false, s))
+      k_tke_zfwd<<<dim3(nxp, C, 3), 256, tke_z_smem(d.nzd), s>>>(L.Xt, L.N3, L.twz, d, L.rz, p0, L.chunk);
   }
   const int S = d.nplanes * d.nzt;
   k_tke_accum<<<(S + 127) / 128, 128, 0, s>>>(L.W, L.N3, L.P, L.acc, L.mean + 3 * d.nplanes, d);
