@@ -144,6 +144,7 @@ struct chgpu_handle {
   // Reynolds-stress budget spectra (allocated by the first chgpu_tke_reset)
   double2 *tke_W = nullptr, *tke_N = nullptr, *tke_P = nullptr, *tke_Zt = nullptr, *tke_Xt = nullptr;
   double *tke_acc = nullptr, *tke_mean = nullptr;
+  double* tke_sp = nullptr;  // chgpu_tke_result: spectra, work, profiles
   void *tke_twz = nullptr, *tke_twx = nullptr, *tke_twh = nullptr;
   RadixDev tke_rz{}, tke_rx{};
   int tke_chunk = 0;
@@ -735,7 +736,7 @@ void release(chgpu_handle* h) {
   void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->fac, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
                   h->twz, h->twx, h->twh, h->twzr, h->twxr, h->fx.z, h->fx.x, h->fx.pack, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
                   h->cl_G, h->cl_Z, h->cl_P, h->cl_tau, h->cl_wd, h->cl_twz, h->cl_twx, h->cl_twh,
-                  h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean,
+                  h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean, h->tke_sp,
                   h->tke_twz, h->tke_twx, h->tke_twh};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -1805,6 +1806,7 @@ int chgpu_tke_reset(chgpu_handle* h, const double* mean) {
     CK(h, cudaMalloc((void**)&h->tke_Xt, sizeof(double2) * 3 * C * nxp * d.nzd));
     CK(h, cudaMalloc((void**)&h->tke_acc, sizeof(double) * 36 * (size_t)np * d.nzt));
     CK(h, cudaMalloc((void**)&h->tke_mean, sizeof(double) * 5 * (size_t)np));
+    CK(h, cudaMalloc((void**)&h->tke_sp, sizeof(double) * (78 * (size_t)d.nzt + 60) * np));
     Radix rz = make_radix(d.nzd, false), rx = make_radix(d.nxd, false);
     h->tke_rz.n = rz.n; h->tke_rz.nst = rz.nst; std::memcpy(h->tke_rz.r, rz.r, sizeof rz.r);
     h->tke_rx.n = rx.n; h->tke_rx.nst = rx.nst; std::memcpy(h->tke_rx.r, rx.r, sizeof rx.r);
@@ -1895,49 +1897,19 @@ int chgpu_tke_result(chgpu_handle* h, int timestwo, double* mean7, double* spect
   const Dims& d = h->d;
   const int np = d.nplanes, nzt = d.nzt;
   const size_t S = (size_t)np * nzt;
-  std::vector<double> acc(36 * S);
-  CK(h, cudaMemcpyAsync(acc.data(), h->tke_acc, sizeof(double) * acc.size(), cudaMemcpyDeviceToHost, h->stream));
-  CK(h, cudaStreamSynchronize(h->stream));
-  const double N = (double)h->tke_n;
-  // spectra(irs, term, iz, iy) in the reference's order (irs fastest); the
-  // accumulated terms var, prod, psdiss, ttrsp, pstrain, PHIptrsp sit at
-  // term 0, 1, 2, 3, 5, 9 (uiuj_spectra.f90:13-14, :70)
-  static const int kAccTerm[6] = {0, 1, 2, 3, 5, 9};
-  std::vector<double> sp((size_t)60 * S, 0.0);
-  auto SP = [&](int irs, int term, int izp, int plane) -> double& {
-    return sp[(size_t)irs + 6 * ((size_t)term + 10 * ((size_t)izp + (size_t)nzt * plane))];
-  };
-  for (int q = 0; q < 6; ++q)
-    for (int irs = 0; irs < 6; ++irs)
-      for (int plane = 0; plane < np; ++plane)
-        for (int izp = 0; izp < nzt; ++izp)
-          SP(irs, kAccTerm[q], izp, plane) = acc[(size_t)(q * 6 + irs) * S + (size_t)plane * nzt + izp] / N;
-  // flux derivatives (:243-259): PHIvdiff = ni d/dy var, vdiff = ni d2/dy2 var, ptrsp = d/dy PHIptrsp
-  std::vector<double> f0(np), f1(np);
-  for (int izp = 0; izp < nzt; ++izp)
-    for (int irs = 0; irs < 6; ++irs) {
-      for (int q = 0; q < np; ++q) f0[q] = SP(irs, 0, izp, q);
-      real_deriv(h->tab, f0.data(), f1.data(), 1);
-      for (int q = 0; q < np; ++q) SP(irs, 8, izp, q) = f1[q] * d.ni;
-      real_deriv(h->tab, f0.data(), f1.data(), 2);
-      for (int q = 0; q < np; ++q) SP(irs, 4, izp, q) = f1[q] * d.ni;
-      for (int q = 0; q < np; ++q) f0[q] = SP(irs, 9, izp, q);
-      real_deriv(h->tab, f0.data(), f1.data(), 1);
-      for (int q = 0; q < np; ++q) SP(irs, 6, izp, q) = f1[q];
-    }
-  if (timestwo)  // -two (:262)
-    for (int plane = 0; plane < np; ++plane)
-      for (int izp = 0; izp < nzt; ++izp)
-        for (int irs = 0; irs < 6; ++irs) SP(irs, 0, izp, plane) *= 2.0;
-  if (spectra) std::memcpy(spectra, sp.data(), sizeof(double) * sp.size());
+  TkeRows rows;
+  const double* w[2][4] = {{h->tab.d14m1, h->tab.d140, h->tab.d14n, h->tab.d14np1},
+                           {h->tab.d24m1, h->tab.d240, h->tab.d24n, h->tab.d24np1}};
+  for (int o = 0; o < 2; ++o)
+    for (int r = 0; r < 4; ++r) std::memcpy(rows.w[o][r], w[o][r], sizeof rows.w[o][r]);
+  double *sp = h->tke_sp, *work = sp + 60 * S, *prof = work + 18 * S;
+  launch_tke_result(h->tke_acc, sp, work, prof, h->der, h->d0lu, rows, d, (double)h->tke_n, timestwo, h->stream);
+  CK(h, cudaGetLastError());
+  h->launches += 3;
+  if (spectra) CK(h, cudaMemcpyAsync(spectra, sp, sizeof(double) * 60 * S, cudaMemcpyDeviceToHost, h->stream));
   if (profiles)
-    for (int plane = 0; plane < np; ++plane)
-      for (int term = 0; term < 10; ++term)
-        for (int irs = 0; irs < 6; ++irs) {
-          double s = 0.0;
-          for (int izp = 0; izp < nzt; ++izp) s += SP(irs, term, izp, plane);
-          profiles[(size_t)irs + 6 * ((size_t)term + 10 * (size_t)plane)] = s;
-        }
+    CK(h, cudaMemcpyAsync(profiles, prof, sizeof(double) * 60 * np, cudaMemcpyDeviceToHost, h->stream));
+  CK(h, cudaStreamSynchronize(h->stream));
   if (mean7)
     for (int plane = 0; plane < np; ++plane)
       for (int q = 0; q < 7; ++q) mean7[(size_t)q + 7 * (size_t)plane] = h->tke_meanh[(size_t)q * np + plane];

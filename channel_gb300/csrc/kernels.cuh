@@ -200,6 +200,15 @@ bool launch_fx_tke_z(const TkeLaunch& L, int p0, int planes, bool inverse, cudaS
 bool launch_fx_tke_x(const TkeLaunch& L, int planes, cudaStream_t s);
 cudaError_t fx_tke_x_smem_limits(int nxd);
 void launch_tke_snapshot(const TkeLaunch& L, cudaStream_t s);
+// wall rows of the first and second derivative: iy = -1, 0, ny, ny+1
+struct TkeRows {
+  double w[2][4][5];
+};
+// the spectra sp (60 per plane and kz), the profiles prof (60 per plane) of n
+// samples; work: 18 per plane and kz
+void launch_tke_result(const double* acc, double* sp, double* work, double* prof, const double* der,
+                       const double* d0lu, const TkeRows& rows, const Dims& d, double n, int timestwo,
+                       cudaStream_t s);
 cudaError_t tke_set_smem_limits(int nzd, int nxd);
 size_t tke_z_smem(int nzd);
 size_t tke_x_smem(int nxd);

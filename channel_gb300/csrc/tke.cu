@@ -12,7 +12,7 @@
 //                  physical grid and brought back to the kept modes with
 //                  `factor`, in chunks of planes (the ttrsp block, :182-227;
 //                  the sum over k is taken before the forward transform,
-//                  which the linearity of the transform and of cprod allows).
+//                  which the linearity of the transform and of the product allows).
 //   k_tke_accum  : one thread per (plane, kz), the sum over kx with weight
 //                  c = 1 (kx = 0), 2 of var, prod, psdiss, ttrsp and, with a
 //                  pressure field, pstrain and PHIptrsp for the six pairs
@@ -31,8 +31,6 @@
 namespace chgpu {
 
 namespace {
-
-__device__ __forceinline__ double cprod(double2 a, double2 b) { return a.x * b.x + a.y * b.y; }  // Re(conj(a) b)
 
 __global__ void k_tke_prep(const double2* __restrict__ V, double2* __restrict__ W, const double* __restrict__ mean,
                            Dims d) {
@@ -152,9 +150,14 @@ __global__ void __launch_bounds__(256) k_tke_zfwd(const double2* __restrict__ Xt
   }
 }
 
-// terms accumulated per snapshot (the rest follow at the end by y derivatives)
-constexpr int kTkeTerms = 6;  // var, prod, psdiss, ttrsp, pstrain, PHIptrsp
-
+// The terms accumulated per snapshot: var, prod, psdiss, ttrsp, pstrain,
+// PHIptrsp (the rest follow at the end by y derivatives).
+//
+// Bound by the FP64 pipe: with the weights c and the factors -1, -2 ni applied
+// to the sums over kx, and prod formed from the sums of var, a mode takes 66
+// multiply-adds (18 more with a pressure) where applying them per mode took
+// about 160; 1.63 -> 0.86 ms at 127x192x127 (1.5 GB).
+template <bool PRESSURE>
 __global__ void __launch_bounds__(128) k_tke_accum(const double2* __restrict__ W, const double2* __restrict__ N3,
                                                    const double2* __restrict__ P, double* __restrict__ acc,
                                                    const double* __restrict__ mgrad, Dims d) {
@@ -163,18 +166,32 @@ __global__ void __launch_bounds__(128) k_tke_accum(const double2* __restrict__ W
   if (t >= S) return;
   const int plane = t / d.nzt, izp = t - plane * d.nzt;
   const size_t FS = (size_t)d.nplanes * d.nmodes;
-  const double ni = d.ni;
-  const double Uy = mgrad[plane], Wy = mgrad[d.nplanes + plane];
-  // mean velocity gradient M[j][k] (get_mean_grad): M[0][1] = dU/dy, M[2][1] = dW/dy
-  const double Mj1[3] = {Uy, 0.0, Wy};
-  double a[kTkeTerms][6];
-#pragma unroll
-  for (int q = 0; q < kTkeTerms; ++q)
-#pragma unroll
-    for (int r = 0; r < 6; ++r) a[q][r] = 0.0;
   constexpr int PI_[6] = {0, 1, 2, 0, 1, 0}, PJ_[6] = {0, 1, 2, 1, 2, 2};
-  for (int ix = 0; ix <= d.nx; ++ix) {
-    const double c = ix == 0 ? 1.0 : 2.0;
+  // sums over kx of u_i u_j, sum_k g_ik g_jk, N_i u_j, p (g_ij + g_ji), p u_i
+  double uu[6], gg[6], nu[3][3], pg[PRESSURE ? 6 : 1], pu[PRESSURE ? 3 : 1];
+#pragma unroll
+  for (int r = 0; r < 6; ++r) uu[r] = gg[r] = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) nu[i][j] = 0.0;
+#pragma unroll
+  for (int r = 0; r < (PRESSURE ? 6 : 1); ++r) pg[r] = 0.0;
+#pragma unroll
+  for (int i = 0; i < (PRESSURE ? 3 : 1); ++i) pu[i] = 0.0;
+  for (int ix = d.nx; ix >= 0; --ix) {
+    if (ix == 0) {  // kx > 0 stands for -kx too
+#pragma unroll
+      for (int r = 0; r < 6; ++r) uu[r] *= 2.0, gg[r] *= 2.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) nu[i][j] *= 2.0;
+#pragma unroll
+      for (int r = 0; r < (PRESSURE ? 6 : 1); ++r) pg[r] *= 2.0;
+#pragma unroll
+      for (int i = 0; i < (PRESSURE ? 3 : 1); ++i) pu[i] *= 2.0;
+    }
     const size_t base = (size_t)plane * d.nmodes + (size_t)ix * d.nzt + izp;
     double2 u[3], n[3], gr[3][3];
 #pragma unroll
@@ -184,31 +201,145 @@ __global__ void __launch_bounds__(128) k_tke_accum(const double2* __restrict__ W
 #pragma unroll
       for (int k = 0; k < 3; ++k) gr[i][k] = W[(size_t)(3 + 3 * i + k) * FS + base];
     }
-    const double2 p = P ? P[base] : make_double2(0.0, 0.0);
+    auto add = [](double& s, double2 a, double2 b) { s = fma(a.x, b.x, fma(a.y, b.y, s)); };  // s += Re(conj(a) b)
 #pragma unroll
     for (int r = 0; r < 6; ++r) {
-      const int i = PI_[r], j = PJ_[r];
-      a[0][r] = a[0][r] + c * cprod(u[i], u[j]);
-      // the reference sums over k with the mean gradient's zero entries too
-      a[1][r] = a[1][r] - c * (cprod(u[i], u[1]) * Mj1[j] + cprod(u[j], u[1]) * Mj1[i]);
+      add(uu[r], u[PI_[r]], u[PJ_[r]]);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) a[2][r] = a[2][r] - 2.0 * ni * c * cprod(gr[i][k], gr[j][k]);
-      a[3][r] = a[3][r] - c * cprod(n[i], u[j]) - c * cprod(n[j], u[i]);
-      if (P) {
-        a[4][r] = a[4][r] + c * cprod(p, gr[i][j] + gr[j][i]);
-        if (r == 1) a[5][r] = a[5][r] - c * (cprod(p, u[1]) + cprod(u[1], p));
-        if (r == 3) a[5][r] = a[5][r] - c * cprod(p, u[0]);
-        if (r == 4) a[5][r] = a[5][r] - c * cprod(p, u[2]);
-      }
+      for (int k = 0; k < 3; ++k) add(gg[r], gr[PI_[r]][k], gr[PJ_[r]][k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) add(nu[i][j], n[i], u[j]);
+    if constexpr (PRESSURE) {
+      const double2 p = P[base];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) add(pg[r], p, gr[PI_[r]][PJ_[r]] + gr[PJ_[r]][PI_[r]]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) add(pu[i], p, u[i]);
     }
   }
+  auto put = [&](int q, int r, double v) { acc[(size_t)(q * 6 + r) * S + t] += v; };
+  // mean velocity gradient M[j][1] (get_mean_grad): dU/dy, 0, dW/dy; the sums u_i v
+  const double M[3] = {mgrad[plane], 0.0, mgrad[d.nplanes + plane]}, uv[3] = {uu[3], uu[1], uu[4]};
 #pragma unroll
-  for (int q = 0; q < kTkeTerms; ++q)
-#pragma unroll
-    for (int r = 0; r < 6; ++r) acc[(size_t)(q * 6 + r) * S + t] += a[q][r];
+  for (int r = 0; r < 6; ++r) {
+    const int i = PI_[r], j = PJ_[r];
+    put(0, r, uu[r]);
+    put(1, r, -(uv[i] * M[j] + uv[j] * M[i]));
+    put(2, r, -2.0 * d.ni * gg[r]);
+    put(3, r, -(nu[i][j] + nu[j][i]));
+    if constexpr (PRESSURE) {
+      put(4, r, pg[r]);
+      if (r == 1) put(5, r, -2.0 * pu[1]);
+      if (r == 3) put(5, r, -pu[0]);
+      if (r == 4) put(5, r, -pu[2]);
+    }
+  }
+}
+
+// The spectra in the reference's order sp[plane][kz][term 0..9][pair] from the
+// sums of n samples: the accumulated terms var, prod, psdiss, ttrsp, pstrain,
+// PHIptrsp sit at term 0, 1, 2, 3, 5, 9 (uiuj_spectra.f90:13-14, :70), 7 stays
+// zero, k_tke_fluxes writes 4, 6 and 8.
+__global__ void k_tke_terms(const double* __restrict__ acc, double* __restrict__ sp, double n, int timestwo, size_t S) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 60 * S) return;
+  const size_t col = t / 60;
+  const int e = (int)(t - 60 * col), term = e / 6, irs = e - 6 * term;
+  if (term == 4 || term == 6 || term == 8) return;
+  const int q = term <= 3 ? term : term == 5 ? 4 : term == 9 ? 5 : -1;
+  double v = q >= 0 ? acc[(size_t)(q * 6 + irs) * S + col] / n : 0.0;
+  if (term == 0 && timestwo) v *= 2.0;  // -two (:262)
+  sp[t] = v;
+}
+
+// The flux derivatives (:243-259), one thread per (term, pair, kz): PHIvdiff =
+// ni d/dy var (term 8), vdiff = ni d2/dy2 var (4), ptrsp = d/dy PHIptrsp (6),
+// by the compact stencils and the factored D0mat (COMPLEXderiv, dnsdata.f90:
+// 339-414) with the first sweep parked in x[term * 6 + pair][plane][kz].
+__global__ void __launch_bounds__(64) k_tke_fluxes(const double* __restrict__ acc, double* __restrict__ x,
+                                                   double* __restrict__ sp, const double* __restrict__ der,
+                                                   const double* __restrict__ d0lu, TkeRows rows, double n, Dims d) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 18 * d.nzt) return;
+  const int c = t / d.nzt, izp = t - c * d.nzt, which = c / 6, irs = c - 6 * which;
+  const int ny = d.ny;
+  const size_t S = (size_t)d.nplanes * d.nzt, st = d.nzt;
+  const double* f = acc + (size_t)((which == 2 ? 5 : 0) * 6 + irs) * S + st + izp;  // f[iy * st]
+  double* xs = x + (size_t)c * S + st + izp;
+  const int term = which == 0 ? 8 : which == 1 ? 4 : 6, dk = which == 1 ? 10 : 5;
+  const double scale = which == 2 ? 1.0 : d.ni;
+  double* out = sp + ((size_t)izp * 10 + term) * 6 + irs;  // + (iy + 1) * 60 st
+  auto F = [&](int iy) { return f[(ptrdiff_t)iy * (ptrdiff_t)st] / n; };
+  auto dot5 = [&](int iy0, const double* w) {
+    double a = w[0] * F(iy0);
+    for (int j = 1; j < 5; ++j) a += w[j] * F(iy0 + j);
+    return a;
+  };
+  const double(&w)[4][5] = rows.w[which == 1];
+  const double fm1 = dot5(-1, w[0]), f0 = dot5(-1, w[1]), fn = dot5(ny - 3, w[2]), fn1 = dot5(ny - 3, w[3]);
+  double x1 = 0.0, x2 = 0.0;
+  // the window F(iy - 2) ... F(iy + 2), its next value loaded ahead
+  double v0 = F(ny - 3), v1 = F(ny - 2), v2 = F(ny - 1), v3 = F(ny), v4 = F(ny + 1);
+  for (int iy = ny - 1; iy >= 1; --iy) {
+    const double next = iy > 1 ? F(iy - 3) : 0.0;
+    const double* dr = der + (size_t)iy * 20;
+    double s = dr[dk] * v0 + dr[dk + 1] * v1 + dr[dk + 2] * v2 + dr[dk + 3] * v3 + dr[dk + 4] * v4;
+    if (iy == ny - 1) s -= dr[3] * fn + dr[4] * fn1;
+    if (iy == ny - 2) s -= dr[4] * fn;
+    if (iy == 1) s -= dr[1] * f0 + dr[0] * fm1;
+    if (iy == 2) s -= dr[0] * f0;
+    const double* lu = d0lu + (size_t)(iy - 1) * 5;
+    const double v = lu[2] * (s - (lu[3] * x1 + lu[4] * x2));
+    x2 = x1;
+    x1 = v;
+    xs[(size_t)iy * st] = v;
+    v4 = v3; v3 = v2; v2 = v1; v1 = v0; v0 = next;
+  }
+  auto put = [&](int iy, double v) { out[(size_t)(iy + 1) * 60 * st] = v * scale; };
+  put(-1, fm1);
+  put(0, f0);
+  double bm2 = fm1, bm1 = f0, cur = xs[st];
+  for (int iy = 1; iy <= ny - 1; ++iy) {
+    const double next = iy < ny - 1 ? xs[(size_t)(iy + 1) * st] : 0.0;
+    const double* lu = d0lu + (size_t)(iy - 1) * 5;
+    const double v = cur - (lu[0] * bm2 + lu[1] * bm1);
+    put(iy, v);
+    bm2 = bm1;
+    bm1 = v;
+    cur = next;
+  }
+  put(ny, fn);
+  put(ny + 1, fn1);
+}
+
+// profiles[plane][term][pair]: the sum over kz
+__global__ void k_tke_profiles(const double* __restrict__ sp, double* __restrict__ prof, int nplanes, int nzt) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 60 * nplanes) return;
+  const int plane = t / 60, e = t - 60 * plane;
+  const double* src = sp + (size_t)plane * nzt * 60 + e;
+  double s = 0.0;
+#pragma unroll 8
+  for (int izp = 0; izp < nzt; ++izp) s += src[(size_t)izp * 60];
+  prof[t] = s;
 }
 
 }  // namespace
+
+// 24 MB of spectra at 127x192x127: 0.7 to 1.3 ms with their copy to the host's
+// memory (the derivatives' serial sweeps 0.40 of it), 14 ms when the host worked
+// on the copied sums.
+void launch_tke_result(const double* acc, double* sp, double* work, double* prof, const double* der,
+                       const double* d0lu, const TkeRows& rows, const Dims& d, double n, int timestwo,
+                       cudaStream_t s) {
+  const size_t S = (size_t)d.nplanes * d.nzt;
+  k_tke_terms<<<(unsigned)((60 * S + 255) / 256), 256, 0, s>>>(acc, sp, n, timestwo, S);
+  k_tke_fluxes<<<(18 * d.nzt + 63) / 64, 64, 0, s>>>(acc, work, sp, der, d0lu, rows, n, d);
+  k_tke_profiles<<<(60 * d.nplanes + 127) / 128, 128, 0, s>>>(sp, prof, d.nplanes, d.nzt);
+}
 
 size_t tke_z_smem(int nzd) { return 2 * (size_t)pad32_size(nzd) * sizeof(double2); }
 size_t tke_x_smem(int nxd) { return (3 * (size_t)pad32_size(4 * nxd) + pad32_size(3 * nxd)) * sizeof(double2); }
@@ -243,7 +374,10 @@ void launch_tke_snapshot(const TkeLaunch& L, cudaStream_t s) {
       k_tke_zfwd<<<dim3(nxp, C, 3), 256, tke_z_smem(d.nzd), s>>>(L.Xt, L.N3, L.twz, d, L.rz, p0, L.chunk);
   }
   const int S = d.nplanes * d.nzt;
-  k_tke_accum<<<(S + 127) / 128, 128, 0, s>>>(L.W, L.N3, L.P, L.acc, L.mean + 3 * d.nplanes, d);
+  if (L.P)
+    k_tke_accum<true><<<(S + 127) / 128, 128, 0, s>>>(L.W, L.N3, L.P, L.acc, L.mean + 3 * d.nplanes, d);
+  else
+    k_tke_accum<false><<<(S + 127) / 128, 128, 0, s>>>(L.W, L.N3, nullptr, L.acc, L.mean + 3 * d.nplanes, d);
 }
 
 }  // namespace chgpu
