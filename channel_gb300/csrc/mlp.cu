@@ -104,7 +104,10 @@ __device__ __forceinline__ unsigned short bf16_bits(float x) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
 __device__ __forceinline__ unsigned pack2(float a, float b) {
-  return (unsigned)bf16_bits(a) | ((unsigned)bf16_bits(b) << 16);
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);  // one conversion for both
+  unsigned r;
+  memcpy(&r, &v, sizeof r);
+  return r;
 }
 // 8 consecutive K elements of one row: one 16-byte store
 __device__ __forceinline__ void store8(unsigned char* dst, const float* x) {
@@ -114,7 +117,16 @@ __device__ __forceinline__ void store1(unsigned char* dst, float x) {
   *reinterpret_cast<unsigned short*>(dst) = bf16_bits(x);
 }
 
-__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+// 1 / (1 + exp(-z)): the approximate reciprocal and one Newton-Raphson step,
+// which the operand's range [1, 6.1e37] lets go without the branch of a
+// general division, so that the independent activations of a lane interleave.
+// The same bits as the division for z in [-80, 80] (0 of 3 10^8 values differ).
+__device__ __forceinline__ float sigmoid(float z) {
+  const float x = 1.0f + expf(fminf(-z, 87.0f));
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(y, fmaf(-x, y, 1.0f), y);
+}
 
 // ---------------------------------------------------------------------------
 // operand packing
@@ -177,7 +189,7 @@ __device__ __forceinline__ void write_input_row(unsigned char* xp, unsigned char
 // written point-major (next layer's A) and, when ht is set, transposed
 __device__ __forceinline__ void hidden_epilogue(unsigned tz, const float* bias, unsigned char* hp, unsigned char* ht,
                                                 int p) {
-#pragma unroll
+#pragma unroll 1  // 16 activations of code: unrolled, the layers' epilogues overflow the instruction cache
   for (int j = 0; j < 4; ++j) {
     float v[16];
     tm_ld16(tz + 16 * j, v);
@@ -416,12 +428,18 @@ struct PlaneIO {
   __device__ void store(long long idx, int o, float v) const { tau[o * comp_stride + idx + 2 * plane_pts] = v; }
 };
 
+// Bound by instruction issue, about 20 instructions an activation and 192
+// activations a point, and by how many blocks overlap their waits for the
+// tensor cores.  Over 2.6 M points 0.97 -> 0.46 ms: the activation without
+// branches 0.79, one epilogue's code for all layers (three unrolled ones
+// missed the instruction cache) and paired BF16 conversions 0.61, six blocks
+// per SM (the input tile in the activations' place) 0.46.
 template <typename IO>
 __global__ void __launch_bounds__(128) k_mlp_infer(const unsigned char* __restrict__ packed, IO io,
                                                    const Norm* __restrict__ nmp, int* __restrict__ err, int errbit) {
   extern __shared__ __align__(1024) unsigned char sm[];
-  __shared__ __align__(8) unsigned long long bar;
-  __shared__ unsigned tbase_s;
+  unsigned long long& bar = *reinterpret_cast<unsigned long long*>(sm + SI_BAR);
+  unsigned& tbase_s = *reinterpret_cast<unsigned*>(sm + SI_BAR + 8);
   const int p = threadIdx.x, warp = p >> 5;
   const Norm& nm = *nmp;  // read through the cache where used
   if (p == 0) mbar_init(&bar, 1);
@@ -440,7 +458,7 @@ __global__ void __launch_bounds__(128) k_mlp_infer(const unsigned char* __restri
   bool ok = __syncthreads_and(mbar_wait(&bar, phase, kBulkWaitPolls));
   phase ^= 1u;
   const float* bias = reinterpret_cast<const float*>(sm + SI_BIAS);
-  unsigned char *X = sm + SI_X, *H = sm + SI_H;
+  unsigned char *H = sm + SI_H, *X = H;
   constexpr unsigned i64 = idesc_bf16(128, 64), i16 = idesc_bf16(128, 16);
   const long long n = io.count();
   const long long tiles = (n + 127) / 128;
@@ -451,15 +469,16 @@ __global__ void __launch_bounds__(128) k_mlp_infer(const unsigned char* __restri
     else
       for (int k = 0; k < NIN; ++k) f[k] = 0.0f;
     write_input_row(X, nullptr, p, f);
-    ok = stage(&bar, phase, [&] { mma_chain(tbase + I_Z, X, 256, sm + P_W1, 256, 1, i64, false); });
+    static_assert(P_W3 - P_W2 == 8192, "consecutive operands");
+#pragma unroll 1
+    for (int l = 0; ok && l < 3; ++l) {  // the first bias is a column of W1
+      ok = stage(&bar, phase, [&] {
+        if (l == 0) mma_chain(tbase + I_Z, X, 256, sm + P_W1, 256, 1, i64, false);
+        else mma_chain(tbase + I_Z, H, 1024, sm + P_W2 + (l - 1) * 8192, 1024, 4, i64, false);
+      });
+      if (ok) hidden_epilogue(tl + I_Z, l == 0 ? nullptr : bias + 64 * (l - 1), H, nullptr, p);
+    }
     if (!ok) break;
-    hidden_epilogue(tl + I_Z, nullptr, H, nullptr, p);
-    ok = stage(&bar, phase, [&] { mma_chain(tbase + I_Z, H, 1024, sm + P_W2, 1024, 4, i64, false); });
-    if (!ok) break;
-    hidden_epilogue(tl + I_Z, bias, H, nullptr, p);
-    ok = stage(&bar, phase, [&] { mma_chain(tbase + I_Z, H, 1024, sm + P_W3, 1024, 4, i64, false); });
-    if (!ok) break;
-    hidden_epilogue(tl + I_Z, bias + 64, H, nullptr, p);
     ok = stage(&bar, phase, [&] { mma_chain(tbase + I_Z, H, 1024, sm + P_W4, 1024, 4, i16, false); });
     if (!ok) break;
     float v[16];
@@ -525,6 +544,12 @@ int mlp_set_smem_limits() {
       cudaFuncSetAttribute(mlp::k_mlp_infer<mlp::PlaneIO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            mlp::S_INFER_END) != cudaSuccess)
     return -1;
+  // for kInferBlocks resident blocks
+  if (cudaFuncSetAttribute(mlp::k_mlp_infer<mlp::SoaIO>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(mlp::k_mlp_infer<mlp::PlaneIO>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) !=
+          cudaSuccess)
+    return -1;
   return 0;
 }
 void launch_mlp_pack(const float* theta, unsigned char* packed, cudaStream_t s) {
@@ -539,14 +564,14 @@ void launch_mlp_train(const unsigned char* packed, const float* feat, const floa
 void launch_mlp_infer(const unsigned char* packed, const float* feat, long long n, const mlp::Norm* nm, float* out,
                       int* err, int nsm, cudaStream_t s) {
   const long long tiles = (n + 127) / 128;
-  const int grid = (int)(tiles < 4LL * nsm ? tiles : 4LL * nsm);
+  const int grid = (int)(tiles < (long long)mlp::kInferBlocks * nsm ? tiles : (long long)mlp::kInferBlocks * nsm);
   if (grid > 0) mlp::k_mlp_infer<<<grid, 128, mlp::S_INFER_END, s>>>(packed, mlp::SoaIO{feat, out, n}, nm, err, 1);
 }
 void launch_mlp_closure(const chgpu_mlp* m, const float* phys, float* tau, const float* wd, long long plane_pts,
                         int nplanes, int ny, int* err, int errbit, int nsm, cudaStream_t s) {
   const long long n = (long long)(ny - 1) * plane_pts;
   const long long tiles = (n + 127) / 128;
-  const int grid = (int)(tiles < 4LL * nsm ? tiles : 4LL * nsm);
+  const int grid = (int)(tiles < (long long)mlp::kInferBlocks * nsm ? tiles : (long long)mlp::kInferBlocks * nsm);
   mlp::PlaneIO io{phys, tau, wd, plane_pts, (long long)nplanes * plane_pts, n};
   if (grid > 0) mlp::k_mlp_infer<<<grid, 128, mlp::S_INFER_END, s>>>(m->packed, io, m->nm_dev, err, errbit);
 }

@@ -46,13 +46,15 @@ constexpr int G_XT = 0, G_H1T = 2, G_ONE1 = 10, G_H2T = 11, G_ONE2 = 19, G_H3T =
 constexpr int G_DYT = 29, G_DZ3T = 31, G_DZ2T = 39, G_DZ1T = 47, G_END = 55;
 constexpr int S_END = S_T + G_END * 2048;  // 193 536 bytes
 // shared memory of the inference kernel: the forward operands W1..W4 (the
-// first P_W4T bytes of the packed block), the biases, the input tile and one
-// activation tile (each layer's epilogue overwrites the operand its product
-// has finished reading)
+// first P_W4T bytes of the packed block), the biases, and one tile for the
+// input and the activations (each layer's epilogue overwrites the operand its
+// product has finished reading)
 constexpr int SI_BIAS = P_W4T;                 // 20480
-constexpr int SI_X = 21504;                    // [128 x 16]
-constexpr int SI_H = SI_X + 4096;              // [128 x 64]
-constexpr int S_INFER_END = SI_H + 16384;      // 41 984 bytes
+constexpr int SI_BAR = SI_BIAS + 576;          // the mbarrier, the tensor-memory address
+constexpr int SI_H = SI_BIAS + 640;            // [128 x 64]; the input tile [128 x 16] first
+constexpr int S_INFER_END = SI_H + 16384;      // 37 504 bytes
+constexpr int kInferBlocks = 6;                // that fit an SM's shared memory (1 KB reserved per block)
+static_assert(PACKED_BYTES - P_BIAS <= 576 && kInferBlocks * (S_INFER_END + 1024) <= 233472, "inference layout");
 
 // tensor-memory columns (FP32, 128 lanes)
 constexpr unsigned C_Z1 = 0, C_Z2 = 64, C_Z3 = 128, C_Y4 = 192, C_DH = 208;
