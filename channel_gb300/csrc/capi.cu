@@ -72,7 +72,8 @@ struct chgpu_handle {
   // mode and real / imaginary component)
   int solve_form = 1;
   cudaStream_t stream2 = nullptr, stream3 = nullptr;
-  cudaEvent_t ev_vv = nullptr, ev_solved = nullptr, ev_fac_fork = nullptr, ev_factored = nullptr;
+  cudaEvent_t ev_vv = nullptr, ev_solved = nullptr, ev_fac_fork = nullptr, ev_factored = nullptr,
+              ev_factored_rest = nullptr;
   cudaEvent_t ev_copy_fork = nullptr, ev_copy_join = nullptr;  // the two-stream field upload
   // device buffers
   double2* V = nullptr;
@@ -84,6 +85,9 @@ struct chgpu_handle {
   double2* F = nullptr;  // body force, plane-major like V
   bool use_F = false;
   double* fac = nullptr;
+  // sets of factors in fac: one per substep for the sizes whose default form
+  // factors ahead (at most 65 535 pairs), else one
+  int fac_slots = 1;
   double* der = nullptr;
   void* derT = nullptr;
   void* derL = nullptr;
@@ -534,6 +538,8 @@ SolveLaunch solve_launch(chgpu_handle* h, const double* ode) {
   L.rhs = h->rhs;
   L.F = h->use_F ? h->F : nullptr;
   L.fac = h->fac;
+  L.slot = 0;
+  L.slot_stride = (size_t)kFacPerRow * (h->d.ny - 1) * h->d.npairs;
   L.der = h->der;
   L.derT = h->derT;
   L.derL = h->derL;
@@ -603,11 +609,21 @@ void run_rhs(chgpu_handle* h, const double* ode, cudaStream_t s = nullptr, int m
 
 // rhs_in_field: read the right-hand sides from V (the reference's in-place
 // convention) instead of the separate buffer k_rhs writes.
-// k_factor of one substep on the third stream, after everything enqueued on
-// the main stream so far (the previous substep's k_solve, which reads fac,
-// and for a step's first substep the outstats that set dt) and, with two
-// halves, after half B's solve; k_solve waits for ev_factored.
-void enqueue_factor(chgpu_handle* h, double ode1, bool after_half_b) {
+// k_factor of substep k on the third stream, after everything enqueued on the
+// main stream so far (the previous substep's k_solve, which reads fac, and for
+// a step's first substep the outstats that set dt) and, with two halves, after
+// half B's solve; k_solve waits for ev_factored.
+//
+// With a set of factors per substep the step's lambdas, all known at its
+// start, are factored then: the first substep's, and behind it the other two
+// in one launch, which have until the second substep's solve.  One set: each
+// substep's factorisation starts with it and has to end with its transforms,
+// with which it shares the SMs.  Mixed steps 1.14 -> 1.10 ms at 47x96x47, 3.05
+// -> 2.92 at 83x120x85, 7.36 -> 7.22 at 127x192x127 (all three in one launch
+// 1.11, 2.90, 7.38); FP64 at 32x64x32 0.87 -> 0.77.
+void enqueue_factor(chgpu_handle* h, int k, bool after_half_b) {
+  if (h->fac_slots == 3 && k > 0) return;
+  const double ode1 = RK[k][0];
   SolveLaunch L = solve_launch(h, nullptr);
   L.ode[0] = ode1;
   L.lambda_from_dt = 1;
@@ -617,10 +633,17 @@ void enqueue_factor(chgpu_handle* h, double ode1, bool after_half_b) {
   launch_factor(L, h->stream3);
   cudaEventRecord(h->ev_factored, h->stream3);
   h->launches += 1;
+  if (h->fac_slots == 3) {
+    L.slot = 1;
+    L.ode[0] = RK[1][0];
+    launch_factor(L, h->stream3, 2, RK[2][0]);
+    cudaEventRecord(h->ev_factored_rest, h->stream3);
+    h->launches += 1;
+  }
 }
 
 void run_linsolve(chgpu_handle* h, double ode1, double lambda, int from_dt, bool rhs_in_field,
-                  cudaStream_t s = nullptr, int q_lo = 0, int q_hi = -1, bool factored = false) {
+                  cudaStream_t s = nullptr, int q_lo = 0, int q_hi = -1, bool factored = false, int substep = 0) {
   SolveLaunch L = solve_launch(h, nullptr);
   L.ode[0] = ode1;
   L.lambda = lambda;
@@ -641,14 +664,17 @@ void run_linsolve(chgpu_handle* h, double ode1, double lambda, int from_dt, bool
   if (!s) s = h->stream;
   L.split_solve = h->solve_form == 1 ? 0 : (h->solve_form == 4 ? 2 : (h->solve_form == 5 ? 3 : 1));
   L.factored = factored && h->solve_form >= 2 ? 1 : 0;
-  if (L.factored) cudaStreamWaitEvent(s, h->ev_factored, 0);
+  if (L.factored) {
+    L.slot = h->fac_slots == 3 ? substep : 0;
+    cudaStreamWaitEvent(s, L.slot == 0 ? h->ev_factored : h->ev_factored_rest, 0);
+  }
   timed(h, 4, [&] { launch_linsolve(L, s); });
   h->launches += h->solve_form >= 2 && !L.factored ? 2 : 1;
 }
 
-void run_outstats(chgpu_handle* h) {
+void run_outstats(chgpu_handle* h, bool step = false) {
   SolveLaunch L = solve_launch(h, nullptr);
-  timed(h, 5, [&] { launch_outstats(L, h->stream); });
+  timed(h, 5, [&] { launch_outstats(L, step ? RK : nullptr, h->stream); });
   h->launches += 1;
 }
 
@@ -672,13 +698,11 @@ void enqueue_step(chgpu_handle* h) {
   const int KA = (h->d.nx + 1 + 1) / 2, nxp = h->d.nx + 1;
   const int mA = KA * h->d.nzt, qA = KA * (h->d.nz + 1);
   for (int k = 0; k < 3; ++k) {
-    if (ahead) enqueue_factor(h, RK[k][0], split && k > 0);
-    timed(h, 5, [&] { launch_advance_time(h->sc, 2.0 / RK[k][0], k == 0, h->stream); });
-    h->launches += 1;
+    if (ahead) enqueue_factor(h, k, split && k > 0);
     if (!split) {
       run_convolutions(h, k == 2, 1, 0, h->d.nplanes);
       run_rhs(h, RK[k]);
-      run_linsolve(h, RK[k][0], 0.0, 1, false, nullptr, 0, -1, ahead);
+      run_linsolve(h, RK[k][0], 0.0, 1, false, nullptr, 0, -1, ahead, k);
       continue;
     }
     if (k == 0) {
@@ -695,12 +719,12 @@ void enqueue_step(chgpu_handle* h) {
     cudaEventRecord(h->ev_vv, h->stream);
     cudaStreamWaitEvent(h->stream2, h->ev_vv, 0);
     run_rhs(h, RK[k], h->stream2, mA, h->d.nmodes);
-    run_linsolve(h, RK[k][0], 0.0, 1, false, h->stream2, qA, h->d.npairs, ahead);
+    run_linsolve(h, RK[k][0], 0.0, 1, false, h->stream2, qA, h->d.npairs, ahead, k);
     cudaEventRecord(h->ev_solved, h->stream2);
-    run_linsolve(h, RK[k][0], 0.0, 1, false, h->stream, 0, qA, ahead);
+    run_linsolve(h, RK[k][0], 0.0, 1, false, h->stream, 0, qA, ahead, k);
   }
   if (split) cudaStreamWaitEvent(h->stream, h->ev_solved, 0);
-  run_outstats(h);
+  run_outstats(h, true);
 }
 
 void fill_stats(const chgpu_handle* h, chgpu_stats* st) {
@@ -753,6 +777,7 @@ void release(chgpu_handle* h) {
   if (h->ev_copy_fork) cudaEventDestroy(h->ev_copy_fork);
   if (h->ev_copy_join) cudaEventDestroy(h->ev_copy_join);
   if (h->ev_factored) cudaEventDestroy(h->ev_factored);
+  if (h->ev_factored_rest) cudaEventDestroy(h->ev_factored_rest);
   if (h->stream2) cudaStreamDestroy(h->stream2);
   if (h->stream3) cudaStreamDestroy(h->stream3);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -832,6 +857,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   }
   h->halves = d.npairs >= 65536 ? 2 : 1;
   h->solve_form = default_solve_form(d.npairs);
+  h->fac_slots = h->solve_form >= 3 ? 3 : 1;
   h->rz.n = rz.n; h->rz.nst = rz.nst; std::memcpy(h->rz.r, rz.r, sizeof rz.r);
   h->rx.n = rx.n; h->rx.nst = rx.nst; std::memcpy(h->rx.r, rx.r, sizeof rx.r);
   set_twiddle_offsets(h->rz);
@@ -867,6 +893,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream3, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fac_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_factored, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_factored_rest, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_copy_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_copy_join, cudaEventDisableTiming);
     if (e != cudaSuccess) { rc = cuda_fail(h, e, "cudaStreamCreate"); break; }
@@ -881,7 +908,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     if ((rc = dev_alloc((void**)&h->rhs, sizeof(double2) * 2 * (p->ny - 1) * nmodes, "rhs"))) break;
     if ((rc = dev_alloc((void**)&h->fac,
                         sizeof(double) * kFacPerRow * (p->ny - 1) *
-                            (size_t)d.npairs,
+                            (size_t)d.npairs * h->fac_slots,
                         "factors")))
       break;
     if ((rc = dev_alloc((void**)&h->der, sizeof(double) * t.der.size(), "der"))) break;

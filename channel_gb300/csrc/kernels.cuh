@@ -143,14 +143,17 @@ struct SolveLaunch {
   int split_solve;    // 0: the fused k_linsolve; 1: k_factor then k_solve (fac holds kFacPerRow per row);
                       // 2: k_factor then k_linsolve reading the factors (two threads per pair);
                       // 3: k_factor then k_solve with eight threads per pair
+  int slot;            // which of the handle's sets of factors
+  size_t slot_stride;  // doubles per set
   int factored;       // split form: fac already holds this substep's factors (k_factor ran ahead), k_solve only
 };
 
 template <typename T> void launch_rhs(const SolveLaunch& L, cudaStream_t s);
 void launch_linsolve(const SolveLaunch& L, cudaStream_t s);
-void launch_factor(const SolveLaunch& L, cudaStream_t s);  // k_factor alone, pairs q_lo..q_hi
-void launch_advance_time(DevScalars* sc, double coef, int new_step, cudaStream_t s);
-void launch_outstats(const SolveLaunch& L, cudaStream_t s);
+// k_factor alone, pairs q_lo..q_hi, into slot L.slot with L.ode[0] and, for two slots, the next with ode1_next
+void launch_factor(const SolveLaunch& L, cudaStream_t s, int slots = 1, double ode1_next = 0.0);
+// rk: the substeps' coefficients at the end of a step, else null
+void launch_outstats(const SolveLaunch& L, const double (*rk)[3], cudaStream_t s);
 void launch_flowrate(const SolveLaunch& L, cudaStream_t s);
 void launch_transpose(const double2* in, double2* out, int rows, int cols, int batch, cudaStream_t s);
 // physical-space export (export.cu)

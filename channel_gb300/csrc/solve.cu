@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(64, 8) k_linsolve(double2* __restrict__ V, con
                                                  BcRows bc, Dims d, double lambda_in, double ode1,
                                                  int lambda_from_dt, DevScalars* __restrict__ sc,
                                                  const dd* __restrict__ lindd, const double* __restrict__ nud,
-                                                 int q_lo, int q_hi) {
+                                                 int q_lo, int q_hi, int slot) {
   const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
   const int q = q_lo + blockIdx.x * 32 + lane;
   const bool active = q < q_hi;
@@ -797,10 +797,10 @@ __global__ void __launch_bounds__(64, 8) k_linsolve(double2* __restrict__ V, con
       }
       if constexpr (FACTORED) {
         if (role == 1 && is00) {  // the wall terms k_factor stored (linsolve_blocking.inc:26-27,40-41)
-          if (iy == 1) b[0] = b[0] - make_double2(sc->wallrhs[0], sc->wallrhs[1]);
-          if (iy == 2) b[0] = b[0] - make_double2(sc->wallrhs[2], sc->wallrhs[3]);
-          if (iy == ny - 2) b[0] = b[0] - make_double2(sc->wallrhs[4], sc->wallrhs[5]);
-          if (iy == ny - 1) b[0] = b[0] - make_double2(sc->wallrhs[6], sc->wallrhs[7]);
+          if (iy == 1) b[0] = b[0] - make_double2(sc->wallrhs[slot][0], sc->wallrhs[slot][1]);
+          if (iy == 2) b[0] = b[0] - make_double2(sc->wallrhs[slot][2], sc->wallrhs[slot][3]);
+          if (iy == ny - 2) b[0] = b[0] - make_double2(sc->wallrhs[slot][4], sc->wallrhs[slot][5]);
+          if (iy == ny - 1) b[0] = b[0] - make_double2(sc->wallrhs[slot][6], sc->wallrhs[slot][7]);
         }
       } else {
         // warp-uniform: each warp assembles only its own matrix; the products
@@ -987,21 +987,29 @@ __global__ void __launch_bounds__(64, 8) k_linsolve(double2* __restrict__ V, con
 // reciprocal pivot and upper entries LeftLU5divStep1 reads).  The eta thread
 // of the mean mode also stores the wall-velocity terms of its right-hand side
 // (rows 1, 2, ny-2, ny-1; linsolve_blocking.inc:26-27,40-41).
+// blockIdx.y: with factors for several substeps at once, the slot of fac (and
+// of sc->wallrhs) after slot0, with its substep's coefficient.
 // Registers capped for 8 resident 64-thread blocks per SM.
+struct FactorOdes {
+  double a, b;
+};
 __global__ void __launch_bounds__(64, 8) k_factor(double* __restrict__ fac, const double* __restrict__ der,
-                                                  BcRows bc, Dims d, double lambda_in, double ode1,
+                                                  BcRows bc, Dims d, double lambda_in, FactorOdes ode1,
                                                   int lambda_from_dt, DevScalars* __restrict__ sc,
-                                                  const double* __restrict__ nud, int q_lo, int q_hi) {
+                                                  const double* __restrict__ nud, int q_lo, int q_hi, int slot0,
+                                                  size_t slot_stride) {
   const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
   const int q = q_lo + blockIdx.x * 32 + lane;
   if (q >= q_hi) return;
+  const int slot = slot0 + blockIdx.y;
+  fac += slot * slot_stride;
   const int ny = d.ny, nz = d.nz;
   const int ix = q / (nz + 1);
   const int a = q - ix * (nz + 1);
   const bool is00 = (ix == 0 && a == 0);
   const double ka = ix * d.alfa0, kb = a * d.beta0;
   const double k2 = ka * ka + kb * kb;
-  const double lambda = lambda_from_dt ? ode1 / sc->deltat : lambda_in;
+  const double lambda = lambda_from_dt ? (blockIdx.y ? ode1.b : ode1.a) / sc->deltat : lambda_in;
   const size_t P = d.npairs;
   double bot[5], botm1[5], top[5], topp1[5];
 #pragma unroll
@@ -1039,10 +1047,10 @@ __global__ void __launch_bounds__(64, 8) k_factor(double* __restrict__ fac, cons
     if (iy == 1) bc_bot1(A, bot, botm1);
     if (iy == 2) bc_bot2(A, bot);
     if (wallrhs) {  // subtracted from the right-hand side of these rows by k_solve
-      if (iy == 1) { sc->wallrhs[0] = A[1] * bval0 / bot[1]; sc->wallrhs[1] = A[1] * 0.0 / bot[1]; }
-      if (iy == 2) { sc->wallrhs[2] = A[0] * bval0 / bot[1]; sc->wallrhs[3] = A[0] * 0.0 / bot[1]; }
-      if (iy == ny - 2) { sc->wallrhs[4] = A[4] * bvaln / top[3]; sc->wallrhs[5] = A[4] * 0.0 / top[3]; }
-      if (iy == ny - 1) { sc->wallrhs[6] = A[3] * bvaln / top[3]; sc->wallrhs[7] = A[3] * 0.0 / top[3]; }
+      if (iy == 1) { sc->wallrhs[slot][0] = A[1] * bval0 / bot[1]; sc->wallrhs[slot][1] = A[1] * 0.0 / bot[1]; }
+      if (iy == 2) { sc->wallrhs[slot][2] = A[0] * bval0 / bot[1]; sc->wallrhs[slot][3] = A[0] * 0.0 / bot[1]; }
+      if (iy == ny - 2) { sc->wallrhs[slot][4] = A[4] * bvaln / top[3]; sc->wallrhs[slot][5] = A[4] * 0.0 / top[3]; }
+      if (iy == ny - 1) { sc->wallrhs[slot][6] = A[3] * bvaln / top[3]; sc->wallrhs[slot][7] = A[3] * 0.0 / top[3]; }
     }
     if (iy == ny - 1) { A[3] = 0; A[4] = 0; }  // rbparmat_blocking.f90:29
     if (iy == ny - 2) A[4] = 0;
@@ -1332,7 +1340,7 @@ __global__ void __launch_bounds__(64 * NP, 8 / NP) k_solve(double2* __restrict__
                                                           const double* __restrict__ d0lu,
                                                           const double* __restrict__ yint, BcRows bc, Dims d,
                                                           DevScalars* __restrict__ sc, const dd* __restrict__ lindd,
-                                                          int q_lo, int q_hi) {
+                                                          int q_lo, int q_hi, int slot) {
   static_assert(NP >= 2, "four warps solve");
   using P = Part<RI>;
   using B = typename P::B;
@@ -1380,10 +1388,10 @@ __global__ void __launch_bounds__(64 * NP, 8 / NP) k_solve(double2* __restrict__
     };
     // the packed wall velocity (linsolve_blocking.inc:26-27,40-41)
     auto wall_terms = [&](int iy, B b) -> B {
-      if (iy == 1) b = b - P::pair(sc->wallrhs, c);
-      if (iy == 2) b = b - P::pair(sc->wallrhs + 2, c);
-      if (iy == ny - 2) b = b - P::pair(sc->wallrhs + 4, c);
-      if (iy == ny - 1) b = b - P::pair(sc->wallrhs + 6, c);
+      if (iy == 1) b = b - P::pair(sc->wallrhs[slot], c);
+      if (iy == 2) b = b - P::pair(sc->wallrhs[slot] + 2, c);
+      if (iy == ny - 2) b = b - P::pair(sc->wallrhs[slot] + 4, c);
+      if (iy == ny - 1) b = b - P::pair(sc->wallrhs[slot] + 6, c);
       return b;
     };
     // operands ahead of the recurrence: kAhead rows in registers where a warp
@@ -1585,20 +1593,21 @@ __global__ void __launch_bounds__(64 * NP, 8 / NP) k_solve(double2* __restrict__
   else deriv_uw_parts<double, RI, NP>(V, der, d0lu, lindd, bc, d, mt, ka, kz, k2, c, part, takes, mean_flow);
 }
 
-void launch_factor(const SolveLaunch& L, cudaStream_t s) {
+void launch_factor(const SolveLaunch& L, cudaStream_t s, int slots, double ode1_next) {
   if (L.q_hi <= L.q_lo) return;
-  const unsigned grid = (unsigned)((L.q_hi - L.q_lo + 31) / 32);
-  k_factor<<<grid, 64, 0, s>>>(L.fac, L.der, L.bc, L.d, L.lambda, L.ode[0], L.lambda_from_dt, L.sc, L.nud, L.q_lo,
-                               L.q_hi);
+  const dim3 grid((unsigned)((L.q_hi - L.q_lo + 31) / 32), slots);
+  k_factor<<<grid, 64, 0, s>>>(L.fac, L.der, L.bc, L.d, L.lambda, FactorOdes{L.ode[0], ode1_next}, L.lambda_from_dt,
+                               L.sc, L.nud, L.q_lo, L.q_hi, L.slot, L.slot_stride);
 }
 
 void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
   if (L.q_hi <= L.q_lo) return;
+  double* fac = L.fac + L.slot * L.slot_stride;
   const unsigned grid = (unsigned)((L.q_hi - L.q_lo + 31) / 32);
   if (!L.split_solve) {
-    k_linsolve<false><<<grid, 64, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint,
+    k_linsolve<false><<<grid, 64, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu, L.yint,
                                           L.bc, L.d, L.lambda, L.ode[0], L.lambda_from_dt, L.sc, (const dd*)L.lindd,
-                                          L.nud, L.q_lo, L.q_hi);
+                                          L.nud, L.q_lo, L.q_hi, L.slot);
     return;
   }
   if (!L.factored) launch_factor(L, s);
@@ -1607,34 +1616,41 @@ void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
     // of 152 SMs), else two (four 128-thread blocks)
     const unsigned g16 = (unsigned)((L.q_hi - L.q_lo + 15) / 16);
     auto kern = g16 <= 304 ? k_solve<true, 4> : k_solve<true, 2>;
-    kern<<<g16, g16 <= 304 ? 256 : 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu,
-                                                L.yint, L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi);
+    kern<<<g16, g16 <= 304 ? 256 : 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu,
+                                                L.yint, L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi, L.slot);
     return;
   }
   if (L.split_solve == 2) {
-    k_linsolve<true><<<grid, 64, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint,
+    k_linsolve<true><<<grid, 64, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu, L.yint,
                                          L.bc, L.d, L.lambda, L.ode[0], L.lambda_from_dt, L.sc, (const dd*)L.lindd,
-                                         L.nud, L.q_lo, L.q_hi);
+                                         L.nud, L.q_lo, L.q_hi, L.slot);
     return;
   }
-  k_solve<false, 2><<<grid, 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, L.fac, L.der, L.d0lu, L.yint,
-                                         L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi);
+  k_solve<false, 2><<<grid, 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu, L.yint,
+                                         L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi, L.slot);
 }
 
 // ---------------------------------------------------------------------------
 // small scalar kernels
 // ---------------------------------------------------------------------------
-__global__ void k_advance_time(DevScalars* sc, double coef, int new_step) {
-  if (new_step) sc->istep += 1;
-  sc->time = sc->time + coef * sc->deltat;  // channel.f90:128,141,154
-}
+// the three advances of the time that a step ends with
+struct StepTime {
+  int steps;  // 0: none
+  double coef[3];
+};
 
-void launch_advance_time(DevScalars* sc, double coef, int new_step, cudaStream_t s) {
-  k_advance_time<<<1, 1, 0, s>>>(sc, coef, new_step);
-}
-
-// outstats without file output (dnsdata.f90:861-879)
-__global__ void k_outstats(const double2* __restrict__ V, Dims d, BcRows bc, DevScalars* sc) {
+// outstats without file output (dnsdata.f90:861-879).  A step's time advances
+// here, substep by substep (channel.f90:128,141,154): nothing reads it before,
+// and a kernel for each is three more links in the step's chain of launches
+// (1.18 -> 1.14 ms per mixed step at 47x96x47).
+__global__ void k_outstats(const double2* __restrict__ V, Dims d, BcRows bc, StepTime st, DevScalars* sc) {
+  if (st.steps) {
+    sc->istep += st.steps;
+    double t = sc->time;
+    const double dt = sc->deltat;
+    for (int k = 0; k < 3; ++k) t = t + st.coef[k] * dt;
+    sc->time = t;
+  }
   const double rg = sc->cfl;
   sc->cfl = 0.0;
   if (d.cflmax > 0) {
@@ -1672,7 +1688,14 @@ __global__ void k_outstats(const double2* __restrict__ V, Dims d, BcRows bc, Dev
   if (bad) sc->error |= 1;
 }
 
-void launch_outstats(const SolveLaunch& L, cudaStream_t s) { k_outstats<<<1, 1, 0, s>>>(L.V, L.d, L.bc, L.sc); }
+void launch_outstats(const SolveLaunch& L, const double (*rk)[3], cudaStream_t s) {
+  StepTime st{};
+  if (rk) {
+    st.steps = 1;
+    for (int k = 0; k < 3; ++k) st.coef[k] = 2.0 / rk[k][0];
+  }
+  k_outstats<<<1, 1, 0, s>>>(L.V, L.d, L.bc, st, L.sc);
+}
 
 // initial flow rate and CPI gradient (channel.f90:101-115)
 __global__ void k_flowrate(const double2* __restrict__ V, const double* __restrict__ yint, Dims d, DevScalars* sc) {
