@@ -1,5 +1,7 @@
 // The nonlinear terms of every y-plane: `convolutions` of the reference
-// (dnsdata.f90:487-602) as three batched shared-memory FFT kernels.
+// (dnsdata.f90:487-602) as three batched shared-memory FFT kernels, for the
+// transform lengths without a compile-time plan (the others: convf.cuh in
+// FP32, convx.cuh in FP64 and double-float).
 //
 //   k_zinv : z-backward transform of u,v,w per (plane, column kx), with the
 //            3/2 zero band inserted while loading (dnsdata.f90:504-510).
@@ -14,7 +16,8 @@
 //            keeping |kz|<=nz (:590, truncation read by buildrhs :609).
 //            Writes VV[p][plane][mode].
 //
-// T is the arithmetic type: double (plain FP64 step) or float (mixed step).
+// T is the arithmetic type: double (FP64 step), dd (double-float step) or
+// float (mixed step).
 #include <cuda_runtime.h>
 
 #include <algorithm>

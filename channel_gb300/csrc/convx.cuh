@@ -24,16 +24,16 @@
 // V, Zb and Pb are FP64; VV is FP64 or, in the double-float path (whose
 // stencils read it), double-float.
 //
-// What bounds them (GB300, counters at 255x64x255): k_xrow_x instruction issue
-// with the 12 warps per SM that its rows' shared memory allows (46% of the
-// issue slots; fixed-latency and shared-memory waits the rest); the z kernels
-// the same, and the FP64 pipe's conversions of their inputs and outputs (60%
-// busy).  Not memory: 2 TB/s in k_zinv_x.  Against the FP64-pipe transforms
-// they replace, the FP64 step went from 44.9 to 15.3 ms at 127x192x127 (k_xrow
-// 4.7, k_zfwd 1.55, k_zinv 0.85 of it; with the right-hand sides' change) and
-// from 262 to 82 ms at 255x256x255 (28.3, 9.4, 5.1); the double-float step
-// from 16.7 to 14.4 ms at 127x192x127.  In-place packing by pairs of entries,
-// one code path for the three inverse rows: k_xrow_x 38.7 -> 28.3 ms.
+// What bounds them (GB300, counters at 255x64x255): latency at 12 (k_xrow_x,
+// by its rows' shared memory) to 15 warps per SM, with 45-54% of the issue
+// slots and 57-59% of the integer multiply-add pipe taken; in the z kernels the
+// conversions of their inputs and outputs also take half of the FP64 pipe.  Not
+// memory: 2 TB/s in the z kernels.  Against the FP64-pipe transforms they
+// replace, ms per step: k_zinv, k_xrow, k_zfwd 3.77, 23.2, 7.47 -> 0.85, 4.7,
+// 1.56 at 127x192x127, 108, 853, 214 -> 24, 186, 47 at 383x384x383; the
+// double-float ones 41, 291, 70 -> 24, 186, 57.  In-place packing by pairs of
+// entries, one code path for the three inverse rows: k_xrow_x 38.7 -> 28.8 ms at
+// 255x256x255.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -1,8 +1,9 @@
 // Double-float arithmetic ("dd"): a real held as an unevaluated sum hi + lo
 // of two FP32 numbers with |lo| <= ulp(hi)/2, giving about 48 significant
 // bits on the FP32 pipes.  On GB300 the FP32 pipes are 58x wider than the
-// FP64 pipe (measured 69.9 vs 1.20 TFLOP/s), so transforms in this format
-// run several times faster than in FP64 while keeping errors near 1e-14.
+// FP64 pipe (measured 69.9 vs 1.20 TFLOP/s), so stencils in this format run
+// several times faster than in FP64 while keeping errors near 1e-14 (the
+// transforms are faster still in 64-bit fixed point, fx.cuh).
 //
 // Building blocks are the error-free transformations of Knuth (two-sum) and
 // Dekker (fast two-sum), with the product error taken from an FMA (Dekker,

@@ -682,7 +682,7 @@ __device__ __forceinline__ void deriv_uw(double2* __restrict__ V, const double* 
       }
       // u = (i kx v' - i kz eta)/k2, w = (i kz v' + i kx eta)/k2; in FP64 with
       // explicit fused multiply-adds, so that the per-component kernel
-      // (deriv_uw_c) rounds exactly alike
+      // (deriv_uw_parts) rounds exactly alike
       C u, w;
       if constexpr (std::is_same<R, double>::value) {
         u.x = fma(bu, et.y, -(au * vp.y));

@@ -31,10 +31,13 @@ extern "C" {
 #define CHGPU_E_NONFINITE -4 /* NaN/Inf met in the flow field or CFL */
 #define CHGPU_E_STATE -5     /* call out of order (e.g. step before upload) */
 
-#define CHGPU_FP64 0  /* every stage in FP64 */
+#define CHGPU_FP64 0  /* every stage in FP64 or better: the transforms and products of the
+                       * lengths with a compile-time plan in 64-bit fixed point scaled by column
+                       * and row, with FP64 values between the kernels */
 #define CHGPU_MIXED 1 /* FFTs, products, nonlinear stencils in FP32; solves FP64 */
-#define CHGPU_FP64DD 2 /* FFTs, products, nonlinear stencils in double-float (two FP32
-                        * numbers, ~48 bits) on the FP32 pipes; everything else FP64 */
+#define CHGPU_FP64DD 2 /* nonlinear stencils (and the transforms of lengths without a plan) in
+                        * double-float (two FP32 numbers, ~48 bits) on the FP32 pipes;
+                        * everything else as CHGPU_FP64 */
 
 /* dns.in after read_dnsin (dnsdata.f90:98-125). `ni` holds 1/Re, the value
  * read_dnsin leaves in `ni`. Logical flags are 0/1. */
