@@ -199,8 +199,14 @@ __global__ void __launch_bounds__(256, MINB) k_xrow(const typename C2<T>::t* __r
 // (the c2r of k_xrow), for the closure's velocity gradients.  Blocks:
 // (groups of nrows z rows, planes, groups of 3 fields).  Writes
 // out[c][plane][jz][m], the pairs x = 2m, 2m+1 packed as in the transform.
+//
+// Bound by the latency of its five passes over shared memory: registers for
+// 1024 threads per SM (86 left 512), in blocks of 128 threads where those cover
+// the first stage's radix-16 butterflies, else of 256.  Closure steps, before,
+// with 128, with 256 threads: 47x96x47 4.57, 4.24, 4.28 ms; 63x64x40 mixed 2.14,
+// 2.02, 2.03; 127x64x127 12.53, 12.40, 11.98; 200x40x60 mixed 5.78, 6.22, 5.73.
 template <typename T>
-__global__ void __launch_bounds__(256) k_xphys(const typename C2<T>::t* __restrict__ Zb, typename C2<T>::t* __restrict__ out,
+__global__ void __launch_bounds__(256, 4) k_xphys(const typename C2<T>::t* __restrict__ Zb, typename C2<T>::t* __restrict__ out,
                                                const typename C2<T>::t* __restrict__ twx,
                                                const typename C2<T>::t* __restrict__ twh, Dims d, RadixDev rx,
                                                int nrows, int plane0) {
@@ -393,7 +399,8 @@ void launch_physical_fields(const double2* src, int ncomp, float2* zb, float2* o
   k_zinv<float><<<gz, 256, conv_zinv_smem(zcols, d.nzd, d.nzt, sizeof(float2)), s>>>(src, zb, twz, d, rz, zcols, 0, 0,
                                                                                       nxp, sc);
   dim3 gx(d.nzd / xrows, d.nplanes, ncomp / 3);
-  k_xphys<float><<<gx, 256, conv_x_smem(xrows, d.nxd, sizeof(float2)), s>>>(zb, out, twx, twh, d, rx, xrows, 0);
+  const int threads = 3 * xrows * d.nxd / 16 <= 128 ? 128 : 256;
+  k_xphys<float><<<gx, threads, conv_x_smem(xrows, d.nxd, sizeof(float2)), s>>>(zb, out, twx, twh, d, rx, xrows, 0);
 }
 
 template void launch_convolutions<double>(const ConvLaunch&, cudaStream_t, int);
