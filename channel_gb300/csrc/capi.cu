@@ -382,6 +382,14 @@ bool fx_xlen_plan(int n, int* E, int* TPR) {
     default: return false;
   }
 }
+// generic kernels: columns per z block that fit its shared-memory budget
+int max_zcols(int nzd, int nzt, size_t ts) {
+  int n = 8;
+  while (n > 1 && conv_zinv_smem(n, nzd, nzt, ts) > 100 * 1024) --n;
+  return n;
+}
+// ... and threads of an x block: 128 where they have its radix-16 butterflies
+int xrow_threads(int xrows, int nxd) { return 3 * xrows * nxd / 16 <= 128 ? 128 : 256; }
 // register-blocked plan of a z or x length in this precision's kernels
 bool zplan(int prec, int n, int* E, int* TPR) {
   return prec == CHGPU_MIXED ? rlen_plan(n, E, TPR) : fx_zlen_plan(n, E, TPR);
@@ -566,7 +574,8 @@ void enqueue_closure(chgpu_handle* h) {
   const Dims& d = h->d;
   launch_gradients(h->V, h->cl_G, h->der, h->d0lu, h->bc, d, h->stream);
   launch_physical_fields(h->cl_G, 9, h->cl_Z, h->cl_P, (const float2*)h->cl_twz, (const float2*)h->cl_twx,
-                         (const float2*)h->cl_twh, d, h->rz, h->rx, h->zcols, h->xrows, h->sc, h->stream);
+                         (const float2*)h->cl_twh, d, h->rz, h->rx, max_zcols(d.nzd, d.nzt, sizeof(float2)), h->xrows, h->sc,
+                         h->stream);
   launch_mlp_closure(h->cl_mlp, reinterpret_cast<const float*>(h->cl_P), reinterpret_cast<float*>(h->cl_tau),
                      h->cl_wd, (long long)d.nzd * 2 * d.nxd, d.nplanes, d.ny, &h->sc->error, 4, h->nsm, h->stream);
   h->launches += 5;
@@ -865,8 +874,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   // tiles: columns per z-transform block and rows per x block, from the
   // shared-memory budget (two ping-pong buffers; nine row buffers)
   const size_t ts = tsize(h);
-  h->zcols = 8;
-  while (h->zcols > 1 && conv_zinv_smem(h->zcols, nzd, d.nzt, ts) > 100 * 1024) --h->zcols;
+  h->zcols = max_zcols(nzd, d.nzt, ts);
   // rows per x block: the most that keep two resident blocks per SM (228 KB
   // of shared memory per SM, 1 KB reserved per block); chgpu_autotune may
   // choose otherwise by timing
@@ -874,6 +882,16 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   h->xrows = 1;
   while (h->xrows < 4 && conv_x_smem(2 * h->xrows, nxd, ts) <= xbudget && nzd % (2 * h->xrows) == 0)
     h->xrows *= 2;
+  // FP32: blocks of 1024 points of z columns and 64 threads, and 128 threads for
+  // x rows where those have its radix-16 butterflies (ms per step of k_zinv +
+  // k_zfwd, k_xrow, before and with this rule: 83x120x85 0.367, 0.908 -> 0.308,
+  // 0.674; 70x96x40 0.183, 0.345 -> 0.139, 0.263; 170x64x170 0.886 -> 0.746, and
+  // its x rows 1.59 with 256 threads, 1.78 with 128)
+  if (h->prec == CHGPU_MIXED) {
+    h->zcols = std::min(h->zcols, std::max(1, 1024 / nzd));
+    h->zthreads = 64;
+    h->xthreads = xrow_threads(h->xrows, nxd);
+  }
   if (conv_x_smem(h->xrows, nxd, ts) > 227 * 1024 || conv_zinv_smem(1, nzd, d.nzt, ts) > 227 * 1024) {
     delete h;
     return fail(nullptr, CHGPU_E_PARAM, "transform length too large for one thread block");
@@ -1485,10 +1503,11 @@ int chgpu_autotune(chgpu_handle* h) {
   // kernels' tiles are tuned where those run (switching between the two
   // would change the rounding of the step, so the tuner keeps the choice)
   if (!h->zfast) {
-    h->zthreads = 256;
+    auto threads_of = [&](int zc) { return std::max(64, std::min(256, (zc * nzd / 16 + 31) / 32 * 32)); };
     for (int zc = 1; zc <= 8; zc *= 2) {
       if (conv_zinv_smem(zc, nzd, h->d.nzt, ts) > lim) break;
       h->zcols = zc;
+      h->zthreads = threads_of(zc);  // one per radix-16 butterfly
       if (int rc = time_z(&ms)) return rc;
       if (ms < best) {
         best = ms;
@@ -1496,8 +1515,8 @@ int chgpu_autotune(chgpu_handle* h) {
       }
   }
   h->zcols = best_z;
-  int best_zt = 256;
-  for (int zt : {128, 192}) {
+  int best_zt = threads_of(best_z);
+  for (int zt : {64, 128, 192, 256}) {
     h->zthreads = zt;
     if (int rc = time_z(&ms)) return rc;
     if (ms < best) {
@@ -1526,12 +1545,12 @@ int chgpu_autotune(chgpu_handle* h) {
   if (!h->xfast) {
     int best_r = h->xrows, best_b = h->xminb;
     best = 1e30f;
-    h->xthreads = 256;
     for (int xb = 1; xb <= 3; ++xb)
       for (int xr = 1; xr <= 4; xr *= 2) {
         if (nzd % xr != 0 || conv_x_smem(xr, nxd, ts) > lim) continue;
         h->xrows = xr;
         h->xminb = xb;
+        h->xthreads = xrow_threads(xr, nxd);
         if (int rc = time_conv_stage(h, 1, reps, &ms)) return rc;
         if (ms < best) {
           best = ms;
@@ -1541,8 +1560,8 @@ int chgpu_autotune(chgpu_handle* h) {
       }
     h->xrows = best_r;
     h->xminb = best_b;
-    int best_xt = 256;
-    for (int xt : {128, 192}) {
+    int best_xt = xrow_threads(best_r, nxd);
+    for (int xt : {128, 192, 256}) {
       h->xthreads = xt;
       if (int rc = time_conv_stage(h, 1, reps, &ms)) return rc;
       if (ms < best) {
@@ -2117,7 +2136,8 @@ int chgpu_closure_features(chgpu_handle* h, float* feat) {
   const Dims& d = h->d;
   launch_gradients(h->V, h->cl_G, h->der, h->d0lu, h->bc, d, h->stream);
   launch_physical_fields(h->cl_G, 9, h->cl_Z, h->cl_P, (const float2*)h->cl_twz, (const float2*)h->cl_twx,
-                         (const float2*)h->cl_twh, d, h->rz, h->rx, h->zcols, h->xrows, h->sc, h->stream);
+                         (const float2*)h->cl_twh, d, h->rz, h->rx, max_zcols(d.nzd, d.nzt, sizeof(float2)), h->xrows, h->sc,
+                         h->stream);
   h->launches += 4;
   CK(h, cudaGetLastError());
   if (int rc = copy_closure_points(h, 9, feat)) return rc;
@@ -2142,7 +2162,8 @@ int chgpu_closure_physical(chgpu_handle* h, const double* spec, int ncomp, float
   CK(h, cudaMemcpyAsync(stage, spec, sizeof(double2) * n, cudaMemcpyHostToDevice, h->stream));
   launch_transpose(stage, h->cl_G, d.nmodes, d.nplanes, ncomp, h->stream);
   launch_physical_fields(h->cl_G, ncomp, h->cl_Z, h->cl_P, (const float2*)h->cl_twz, (const float2*)h->cl_twx,
-                         (const float2*)h->cl_twh, d, h->rz, h->rx, h->zcols, h->xrows, h->sc, h->stream);
+                         (const float2*)h->cl_twh, d, h->rz, h->rx, max_zcols(d.nzd, d.nzt, sizeof(float2)), h->xrows, h->sc,
+                         h->stream);
   h->launches += 3;
   CK(h, cudaGetLastError());
   if (int rc = copy_closure_points(h, ncomp, out)) return rc;
