@@ -140,20 +140,9 @@ CHGPU_FX_CONST FxC fx_cos24(int e) {
   const int f = ((e % 24) + 24) % 24, g = f > 12 ? 24 - f : f;
   return g > 6 ? fx_neg(fx_cos24_first(12 - g)) : fx_cos24_first(g);
 }
-// cos(22.5 e degrees) for 0 <= e <= 4
-CHGPU_FX_CONST FxC fx_cos16_first(int e) {
-  return e == 0   ? FxC{1, 0, 1ll << 62}
-         : e == 1 ? FxC{1, -1404174782535421627ll, 4260642322793532497ll}
-         : e == 2 ? fx_sqrt1_2()
-         : e == 3 ? FxC{0, 7059263338087549767ll, 1764815834521887442ll}
-                  : FxC{0, 0, 0};
-}
-CHGPU_FX_CONST FxC fx_cos16(int e) {
-  const int f = ((e % 16) + 16) % 16, g = f > 8 ? 16 - f : f;
-  return g > 4 ? fx_neg(fx_cos16_first(8 - g)) : fx_cos16_first(g);
-}
-CHGPU_FX_CONST FxC fx_cosN(int N, int m) { return N == 16 ? fx_cos16(m) : fx_cos24(m * (24 / N)); }
-CHGPU_FX_CONST FxC fx_sinN(int N, int m) { return N == 16 ? fx_cos16(m - 4) : fx_cos24(m * (24 / N) - 6); }
+// N dividing 24
+CHGPU_FX_CONST FxC fx_cosN(int N, int m) { return fx_cos24(m * (24 / N)); }
+CHGPU_FX_CONST FxC fx_sinN(int N, int m) { return fx_cos24(m * (24 / N) - 6); }
 
 // a (c + i s) at full scale, c and s compile-time constants
 __device__ __forceinline__ fx2 fx_cmulc(fx2 a, FxC c, FxC s) {
@@ -189,7 +178,7 @@ template <int SR, int SI> __device__ __forceinline__ fx2 fx_mul_diag(fx2 a) {
   return fx2{fx_mad(p, p, h, l), fx_mad(q, q, h, l)};
 }
 
-// register DFTs (the splits of Dft<8>, Dft<16> and DftComposite, cplx.cuh)
+// register DFTs (the splits of Dft<8> and DftComposite, cplx.cuh)
 template <> struct Dft<3, fx2> {
   template <int SIGN> __device__ __forceinline__ static void run(fx2* a) {
     const fx2 t = a[1] + a[2], d = a[1] - a[2];
@@ -218,48 +207,6 @@ template <> struct Dft<8, fx2> {
 #pragma unroll
     for (int k = 0; k < 8; ++k) a[k] = y[k];
   }
-};
-// 16 points as DFT4 over r1, twiddles w16^(r2 k1), DFT4 over r2 (r = 4 r1 +
-// r2, k = k1 + 4 k2).  QUARTER: the twiddles at quarter scale, the output a
-// quarter of the DFT.
-template <int SIGN, bool QUARTER> __device__ __forceinline__ void fx_dft16(fx2* a) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) dft4<SIGN>(a[q], a[q + 4], a[q + 8], a[q + 12]);
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1)
-#pragma unroll
-    for (int r2 = 0; r2 < 4; ++r2) {
-      fx2& v = a[r2 + 4 * k1];
-      const int m = r2 * k1;
-      if (m == 0) {
-        if (QUARTER) v = fx_quarter(v);
-      } else if (QUARTER) {
-        v = fx_cmulc_q(v, fx_cos16(m), SIGN > 0 ? fx_sinN(16, m) : fx_neg(fx_sinN(16, m)));
-      } else if (m == 4) {
-        v = mul_is<SIGN>(v);
-      } else if (m == 2) {
-        v = fx_mul_diag<1, SIGN>(v);
-      } else if (m == 6) {
-        v = fx_mul_diag<-1, SIGN>(v);
-      } else {
-        v = fx_cmulc(v, fx_cos16(m), SIGN > 0 ? fx_sinN(16, m) : fx_neg(fx_sinN(16, m)));
-      }
-    }
-  fx2 y[16];
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) {
-    fx2 b0 = a[4 * k1], b1 = a[4 * k1 + 1], b2 = a[4 * k1 + 2], b3 = a[4 * k1 + 3];
-    dft4<SIGN>(b0, b1, b2, b3);
-    y[k1] = b0;
-    y[k1 + 4] = b1;
-    y[k1 + 8] = b2;
-    y[k1 + 12] = b3;
-  }
-#pragma unroll
-  for (int k = 0; k < 16; ++k) a[k] = y[k];
-}
-template <> struct Dft<16, fx2> {
-  template <int SIGN> __device__ __forceinline__ static void run(fx2* a) { fx_dft16<SIGN, false>(a); }
 };
 // 3 P points as DFT3 over r1, twiddles w_{3P}^(r2 k1), DFT_P over r2
 template <int P, int SIGN, bool QUARTER> __device__ __forceinline__ void fx_dft3p(fx2* a) {
@@ -298,21 +245,21 @@ template <int P, int SIGN, bool QUARTER> __device__ __forceinline__ void fx_dft3
 #pragma unroll
   for (int k = 0; k < N; ++k) a[k] = y[k];
 }
-// First pass of a transform: forward transforms of 16 and 24 points per
-// thread are scaled by a quarter inside, whose two bits let the input use
-// the word's full width; backward ones run at full scale.
-__host__ __device__ constexpr bool fx_first_quarter(int E, int SIGN) { return SIGN < 0 && (E == 16 || E == 24); }
+// First pass of a transform: forward transforms of 24 points per thread are
+// scaled by a quarter inside, whose two bits let the input use the word's full
+// width; backward ones run at full scale.
+__host__ __device__ constexpr bool fx_first_quarter(int E, int SIGN) { return SIGN < 0 && E == 24; }
 template <int E, int SIGN, bool QUARTER> __device__ __forceinline__ void fx_first(fx2* a) {
   if constexpr (E == 24) fx_dft3p<8, SIGN, QUARTER>(a);
   else if constexpr (E == 12) fx_dft3p<4, SIGN, false>(a);
-  else if constexpr (E == 16) fx_dft16<SIGN, QUARTER>(a);
   else Dft<E, fx2>::template run<SIGN>(a);
 }
 
 // ---------------------------------------------------------------------------
 // scales
 // ---------------------------------------------------------------------------
-// What the kernels read and write: FP64 pairs or double-float pairs.
+// What the kernels read and write: FP64 pairs; double-float pairs are written
+// only.
 template <typename T> struct FxIo;
 template <> struct FxIo<double> {
   using V2 = double2;
@@ -335,15 +282,7 @@ template <> struct FxIo<double> {
 };
 template <> struct FxIo<dd> {
   using V2 = cdd;
-  static constexpr int kBias = 127, kExpMax = 255;
-  __device__ static int expo(dd v) { return (__float_as_int(v.hi) >> 23) & 0xff; }
-  __device__ static int lead(dd v) { return (((__float_as_int(v.hi) & 0x7fffff) | 0x800000) >> 5) + 1; }  // + 1: the low word
   __device__ static float pow2(int s) { return __int_as_float((127 + s) << 23); }  // -126 <= s <= 127
-  __device__ static long long in(dd v, int S) {
-    const int s1 = S >> 1;
-    const float f1 = pow2(s1), f2 = pow2(S - s1);
-    return __float2ll_rn(v.hi * f1 * f2) + __float2ll_rn(v.lo * f1 * f2);
-  }
   __device__ static dd out(long long f, int S) {
     const float h = __ll2float_rn(f), l = __ll2float_rn(f - __float2ll_rn(h));
     const int s1 = (-S) >> 1;

@@ -330,20 +330,20 @@ template <> struct FxLen<1024> { static constexpr int E = 8, TPR = 128; };
 template <> struct FxLen<1536> { static constexpr int E = 24, TPR = 64; };
 
 // Passes of a forward fixed-point transform at quarter scale (fx.cuh): every
-// one after the first, and inside the first of 16 and 24 points.
+// one after the first, and inside the first of 24 points.
 __host__ __device__ constexpr int fx_quarters(int E, int TPR) {
   return rplan_passes(E, TPR) - 1 + (fx_first_quarter(E, -1) ? 1 : 0);
 }
 // Growth of the moduli over the passes from `first` on at quarter scale, as
 // its largest value on the way and at the end; before them a factor g (a first
-// pass of 24 (16) points with its inner quarter: 3 (4), then 8/4 (4/4)).
+// pass of 24 points with its inner quarter: 3, then 8/4).
 struct FxGrowth {
   double most, last;
 };
 __host__ __device__ constexpr FxGrowth fx_growth(int E, int TPR, bool with_first) {
-  double g = !with_first ? 1.0 : E == 24 ? 3.0 : E == 16 ? 4.0 : (double)E;
+  double g = !with_first ? 1.0 : E == 24 ? 3.0 : (double)E;
   double mx = g;
-  if (with_first && fx_first_quarter(E, -1)) g *= E == 24 ? 2.0 : 1.0;
+  if (with_first && fx_first_quarter(E, -1)) g *= 2.0;
   if (g > mx) mx = g;
   for (int p = 1; p < rplan_passes(E, TPR); ++p) {
     g *= rplan_radix(E, TPR, p) / 4.0;
