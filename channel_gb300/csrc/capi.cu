@@ -208,11 +208,24 @@ std::vector<V2> roots(int n) {  // forward roots exp(-2 pi i m/n), from the math
   return w;
 }
 
-// der and the wavenumber units in the nonlinear-term type: [(ny+1)*20] then alfa0, beta0
+// der and the wavenumber units in the nonlinear-term type: [(ny+1)*20] then
+// alfa0, beta0, then [(ny+1)*15] the stencils d0, d1, d2 as they act on
+// differences of neighbours (k_rhs): C_0 ... C_3, C_j = -(c_0 + ... + c_j), and
+// the coefficients' sum
 template <typename T>
 int upload_derT(chgpu_handle* h) {
   const std::vector<double>& der = h->tab.der;
-  std::vector<T> t(der.size() + 2);
+  const size_t rows = der.size() / 20;
+  std::vector<T> t(der.size() + 2 + 15 * rows);
+  for (size_t r = 0; r < rows; ++r)
+    for (int k = 0; k < 3; ++k) {
+      T* c = &t[der.size() + 2 + 15 * r + 5 * k];
+      long double s = 0.0L;
+      for (int j = 0; j < 5; ++j) {
+        s += (long double)der[20 * r + 5 * k + j];
+        c[j] = from_ld<T>(j < 4 ? -s : s);
+      }
+    }
   for (size_t i = 0; i < der.size(); ++i) t[i] = from_ld<T>((long double)der[i]);
   t[der.size()] = from_ld<T>((long double)h->p.alfa0);
   t[der.size() + 1] = from_ld<T>((long double)h->p.beta0);

@@ -127,7 +127,7 @@ struct SolveLaunch {
   int rhs_plane_off;       // row iy lives at plane iy+rhs_plane_off
   double* fac;
   const double* der;
-  const void* derT;  // der in the nonlinear-term type, then alfa0, beta0
+  const void* derT;  // der in the nonlinear-term type, then alfa0, beta0, the stencils of differences
   const void* derL;  // der in the linear-term type, then alfa0, beta0, ni
   const double* d0lu;
   const double* yint;

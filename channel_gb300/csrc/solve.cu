@@ -89,9 +89,6 @@ template <> __device__ __forceinline__ float store_as<float>(dd x) { return __fa
 template <typename T> struct HistT { using t = typename C2<T>::t; };
 template <> struct HistT<dd> { using t = double2; };
 
-// resident 128-thread blocks per SM the registers are capped for
-template <typename T> struct RhsBlocks { static constexpr int value = 3; };
-
 // rb (at most kRhsMaxRows) consecutive rows per thread: the five-row windows
 // slide down the rows,
 // so each row is loaded (and, in the mixed path, converted to
@@ -102,15 +99,24 @@ template <typename T> struct RhsBlocks { static constexpr int value = 3; };
 //   expl_v = D1 P + (D2 + k2 D0) Q,  P = k2 vv - kx^2 uu - 2 kx kz uw - kz^2 ww,  Q = i (kx uv + kz vw)
 //   expl_eta = D0 R + D1 S,          R = kx kz (uu - ww) + (kz^2 - kx^2) uw,      S = i (kx vw - kz uv)
 // (dnsdata.f90:636-640, 654 expanded; the mean mode's S = (-uv, -vw), :653),
-// and eta's linear terms act on w = i kz V1 - i kx V3.  Per mode and row: 114
-// FP64 operations where the 13 stencils of the products and the stencils of
-// V1 and V3 took 217; the FP64 pipe bounds the kernel, 80% busy (39.2 -> 23.9
-// ms per step at 255x256x255; double-float, whose linear terms are FP64, 17.4
-// -> 13.0).  The FP32 path keeps the stencils of each product and field, whose
-// FP32 rounding the mixed step's results carry.
+// and eta's linear terms act on w = i kz V1 - i kx V3.  The FP64 pipe bounds the
+// kernel: ms per step at 255x256x255 against the 13 stencils of the products and
+// the stencils of V1 and V3, 39.2 -> 26.2; double-float, whose linear terms are
+// FP64, 17.4 -> 13.5.  The FP32 path keeps the stencils of each product and
+// field, whose FP32 rounding the mixed step's results carry.
+//
+// D1 and D2 nearly cancel from row to row, so Q and S rounded in their windows
+// make more noise than stencils of the products do (2.5 and 1.5 times, the
+// kernel at 23.9 and 13.0 ms).  Theirs hold the differences from row to row,
+// formed from those of uv and vw, which are exact between neighbours within a
+// factor of two:
+//   sum_j c_j F_j = (sum_j c_j) F_4 + sum_{j<4} C_j (F_{j+1} - F_j),  C_j = -(c_0 + ... + c_j).
+// Relative L2 rounding error of expl_v, expl_eta at 79x101x75: 4.9e-16, 1.3e-15
+// from the products' stencils, 1.6e-16, 2.4e-16 so; 2.6e-15, 2.8e-16 and 6.1e-16,
+// 1.1e-16 at 9x192x12.
 constexpr int kRhsMaxRows = 32;
 template <typename T>
-__global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2* __restrict__ V, const typename C2<T>::t* __restrict__ VV,
+__global__ void __launch_bounds__(128, 3) k_rhs(const double2* __restrict__ V, const typename C2<T>::t* __restrict__ VV,
                                              typename HistT<T>::t* __restrict__ old, double2* __restrict__ rhs,
                                              const typename LinT<T>::t* __restrict__ derL, const T* __restrict__ derT,
                                              Dims d, double ode1, double ode2, double ode3,
@@ -158,7 +164,8 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   const int ix = m / d.nzt;
   const int iz = m - ix * d.nzt - d.nz;
   const bool mean = ix == 0 && iz == 0;
-  // wavenumbers (derT holds der in T, then alfa0, beta0; derL likewise in L, then ni)
+  // wavenumbers (derT holds der in T, then alfa0, beta0 and the
+  // stencils of differences; derL der in L, then alfa0, beta0, ni)
   const size_t tail = (size_t)(d.ny + 1) * 20;
   const T ta = T((float)ix) * derT[tail], tb = T((float)iz) * derT[tail + 1];
   const T tk2 = ta * ta + tb * tb;
@@ -199,19 +206,31 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
       cp_async_commit();
     }
   };
-  // windows over rows iy-2..iy+2: the six product spectra (plane = row + 1)
-  // or their combinations P, Q, R, S, and the field as V2 and w
-  constexpr int NW = COMB ? 4 : 6;
+  // windows over rows iy-2..iy+2: the six product spectra (plane = row + 1), or
+  // P and R, the four differences dq and ds of Q and S and their values at iy+2
+  // (from uv and vw there and one row before), and the field as V2 and w
+  constexpr int NW = COMB ? 2 : 6;
   V2 vv[NW][5];
+  V2 dq[COMB ? 4 : 1], ds[COMB ? 4 : 1], q4, s4, uv, vw;
   LV v2[5], w[5], v3[COMB ? 1 : 5];  // w: V1 in the FP32 path
+  auto comb_q = [&](V2 a, V2 b) { return mk<V2>(-fmaT(ta, a.y, tb * b.y), fmaT(ta, a.x, tb * b.x)); };
+  auto comb_s = [&](V2 a, V2 b) {
+    return mean ? mk<V2>(-a.x, -b.x) : mk<V2>(fmaT(tb, a.y, -(ta * b.y)), fmaT(ta, b.x, -(tb * a.x)));
+  };
   auto put_products = [&](int j, const V2 (&p)[6]) {
     if constexpr (COMB) {  // uu, vv, ww, uv, vw, uw
       vv[0][j] = mk<V2>(fmaT(tk2, p[1].x, fmaT(-taa, p[0].x, fmaT(-tab2, p[5].x, -(tbb * p[2].x)))),
                         fmaT(tk2, p[1].y, fmaT(-taa, p[0].y, fmaT(-tab2, p[5].y, -(tbb * p[2].y)))));
-      vv[1][j] = mk<V2>(-fmaT(ta, p[3].y, tb * p[4].y), fmaT(ta, p[3].x, tb * p[4].x));
-      vv[2][j] = mk<V2>(fmaT(tab, p[0].x - p[2].x, tba * p[5].x), fmaT(tab, p[0].y - p[2].y, tba * p[5].y));
-      vv[3][j] = mean ? mk<V2>(-p[3].x, -p[4].x)
-                      : mk<V2>(fmaT(tb, p[3].y, -(ta * p[4].y)), fmaT(ta, p[4].x, -(tb * p[3].x)));
+      vv[1][j] = mk<V2>(fmaT(tab, p[0].x - p[2].x, tba * p[5].x), fmaT(tab, p[0].y - p[2].y, tba * p[5].y));
+      if (j > 1) {  // slot 1: the first row, which has no difference
+        const V2 du = p[3] - uv, dw = p[4] - vw;
+        dq[j - 1] = comb_q(du, dw);
+        ds[j - 1] = comb_s(du, dw);
+      }
+      uv = p[3];
+      vw = p[4];
+      q4 = comb_q(uv, vw);
+      s4 = comb_s(uv, vw);
     } else {
 #pragma unroll
       for (int k = 0; k < 6; ++k) vv[k][j] = p[k];
@@ -246,6 +265,12 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   for (int j = 0; j < 4; ++j) {
 #pragma unroll
     for (int k = 0; k < NW; ++k) vv[k][j] = vv[k][j + 1];
+    if constexpr (COMB) {
+      if (j < 3) {
+        dq[j] = dq[j + 1];
+        ds[j] = ds[j + 1];
+      }
+    }
     v2[j] = v2[j + 1];
     w[j] = w[j + 1];
     if constexpr (!COMB) v3[j] = v3[j + 1];
@@ -279,7 +304,7 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   for (int j = 0; j < 5; ++j) {
     e0[j] = drT[j];
     e1[j] = drT[5 + j];
-    e2[j] = drT[10 + j];
+    if constexpr (!COMB) e2[j] = drT[10 + j];
   }
   // DD(f,k) (dnsdata.f90:609-610) on window k at rows iy-2..iy+2
   auto DD = [&](const T* c, int k) -> V2 {
@@ -290,16 +315,32 @@ __global__ void __launch_bounds__(128, RhsBlocks<T>::value) k_rhs(const double2*
   };
   V2 explv, ee;  // the explicit terms of D2v and eta (of the mean mode: U, W without the pressure gradient)
   if constexpr (COMB) {
-    auto axpy = [&](V2 s, const T* c, int k) -> V2 {
+    auto axpy = [](T c, V2 x, V2 s) { return mk<V2>(fmaT(c, x.x, s.x), fmaT(c, x.y, s.y)); };
+    // s = the first term of the stencil c of window k, the others added from
+    // the ends in, the largest last
+    auto values = [&](V2 s, const T* c, int k) {
+      s = axpy(c[4], vv[k][4], s);
+      s = axpy(c[1], vv[k][1], s);
+      s = axpy(c[3], vv[k][3], s);
+      return axpy(c[2], vv[k][2], s);
+    };
+    // s + the stencil c of a window's differences df
+    auto differences = [&](V2 s, const T* c, const V2* df) {
 #pragma unroll
-      for (int j = 0; j < 5; ++j) s = mk<V2>(fmaT(c[j], vv[k][j].x, s.x), fmaT(c[j], vv[k][j].y, s.y));
+      for (int j = 0; j < 4; ++j) s = axpy(c[j], df[j], s);
       return s;
     };
-    T e20[5];
+    const T* df = derT + tail + 2 + (size_t)iy * 15;  // C_0 ... C_3 and the sum, of d0, d1, d2
+    T c1[5], c20[5];
 #pragma unroll
-    for (int j = 0; j < 5; ++j) e20[j] = fmaT(tk2, e0[j], e2[j]);
-    explv = axpy(DD(e1, 0), e20, 1);
-    ee = axpy(DD(e0, 2), e1, 3);
+    for (int j = 0; j < 5; ++j) {
+      c1[j] = df[5 + j];
+      c20[j] = fmaT(tk2, df[j], df[10 + j]);
+    }
+    explv = values(mk<V2>(e1[0] * vv[0][0].x, e1[0] * vv[0][0].y), e1, 0);
+    explv = axpy(c20[4], q4, differences(explv, c20, dq));
+    ee = differences(mk<V2>(c1[4] * s4.x, c1[4] * s4.y), c1, ds);
+    ee = values(axpy(e0[0], vv[1][0], ee), e0, 1);
   } else {
     const V2 DD0_6 = DD(e0, 5), DD1_6 = DD(e1, 5);
     // rhsu = -i ta DD0(uu) - DD1(uv) - i tb DD0(uw) (dnsdata.f90:636-638), and
