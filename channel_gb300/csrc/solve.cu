@@ -168,13 +168,16 @@ __global__ void __launch_bounds__(128, 3) k_rhs(const double2* __restrict__ V, c
   // stencils of differences; derL der in L, then alfa0, beta0, ni)
   const size_t tail = (size_t)(d.ny + 1) * 20;
   const T ta = T((float)ix) * derT[tail], tb = T((float)iz) * derT[tail + 1];
-  const T tk2 = ta * ta + tb * tb;
+  // (FP64: one explicit rounding each, or the copies of these that the compiler
+  // makes for the start-up rows and for the loop may be contracted differently,
+  // and the result depend on rb)
+  const T tk2 = COMB ? fmaT(ta, ta, tb * tb) : ta * ta + tb * tb;
   const L a = L((float)ix) * derL[tailL], b = L((float)iz) * derL[tailL + 1];
-  const L k2 = a * a + b * b;
+  const L k2 = COMB ? fmaT(a, a, b * b) : a * a + b * b;
   const L lode2 = Num<L>::from_double(ode2), lode3 = Num<L>::from_double(ode3);
   // coefficients of P and R
   const T taa = COMB ? ta * ta : T(), tbb = COMB ? tb * tb : T(), tab = COMB ? ta * tb : T();
-  const T tab2 = tab + tab, tba = COMB ? tbb - taa : T();
+  const T tab2 = tab + tab, tba = COMB ? fmaT(tb, tb, -taa) : T();
   // STAGED (FP32 path): the next D rows' products (plane iy+3), field rows
   // iy+2 and RK history at iy are copied into a per-thread ring in shared
   // memory while the current row is computed (cp.async), instead of loaded

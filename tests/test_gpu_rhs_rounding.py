@@ -121,3 +121,25 @@ def test_explicit_terms_round_no_worse_than_the_reference_stencils(gpu_lib, nx, 
     for got, ref, terms in ((G[1], ev, ((1, 1, P), (2, 1, Q), (0, k2, Q))), (G[0], ee, ((0, 1, R), (1, 1, S)))):
         err, bar = rounding(split(got), terms, der, n), rounding(split(ref), terms, der, n)
         assert err <= unit * bar, (err, bar)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp64dd", "mixed"])
+@pytest.mark.parametrize("nx,ny,nz", [(32, 48, 16), (24, 64, 24), (40, 96, 20)])
+def test_rows_per_thread_do_not_change_the_results(gpu_lib, nx, ny, nz, prec):
+    """The step in two halves runs k_rhs on half the modes and so with other rows per thread: the same bits, also at
+    wavenumbers whose squares and products are rounded."""
+    from channel_gb300 import Channel, DnsIn
+
+    p = DnsIn(nx=nx, ny=ny, nz=nz, alfa0=1.1234567, beta0=3.0987, re=2000.0, a=1.6, ymin=0.0, ymax=2.0,
+              meanflowx=4.0 / 3.0, deltat=0.002, cflmax=0.0, nstep=1)
+    out = []
+    for halves in (1, 2):
+        with Channel(p, prec) as g:
+            g.set_step_halves(halves)
+            g.upload(field(p, 2))
+            g.start()
+            for _ in range(2):
+                line = g.step()
+            out.append((g.download(), line))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
