@@ -23,6 +23,7 @@
 #include "../../include/chgpu_closure.h"
 #include "chgpu_internal.h"
 #include "kernels.cuh"
+#include "launch_rules.h"
 #include "rfft.cuh"
 #include "mlp.cuh"
 
@@ -155,7 +156,9 @@ struct chgpu_handle {
   long long tke_n = 0;
   bool tke_ready = false, tke_pressure = false;
   std::vector<double> tke_meanh;  // U, W, dU/dy, dW/dy, d2U/dy2, d2W/dy2, P per plane
-  int nsm = 0;
+  int nsm = 1;  // SMs of the device
+  // how many times this handle's pairs those of all members of its ensemble are
+  double together = 1.0;
   // per-kernel timing
   bool profiling = false;
   std::vector<cudaEvent_t> ev_pool;
@@ -561,6 +564,8 @@ SolveLaunch solve_launch(chgpu_handle* h, const double* ode) {
   L.fac = h->fac;
   L.slot = 0;
   L.slot_stride = (size_t)kFacPerRow * (h->d.ny - 1) * h->d.npairs;
+  L.nsm = h->nsm;
+  L.together = h->together;
   L.der = h->der;
   L.derT = h->derT;
   L.derL = h->derL;
@@ -811,15 +816,6 @@ extern "C" {
 
 const char* chgpu_last_error(const chgpu_handle* h) { return h ? h->err.c_str() : g_create_error.c_str(); }
 
-namespace {
-// Solve form of a handle that has not been tuned: eight threads per pair
-// while its blocks are one wave (16 pairs per 128-thread block, four blocks
-// on each of 152 SMs; ms per mixed step against four threads per pair:
-// 32x64x32 0.51 / 0.66, 47x96x47 1.07 / 1.28, 83x120x85 2.70 / 2.83, but
-// 127x192x127 6.97 / 6.45), then four threads, then the fused kernel
-int default_solve_form(int pairs) { return pairs <= 16 * 4 * 152 ? 5 : pairs < 65536 ? 3 : 1; }
-}  // namespace
-
 int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   if (!p || !out) return fail(nullptr, CHGPU_E_PARAM, "chgpu_create: null argument");
   *out = nullptr;
@@ -878,7 +874,9 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     h->xrvar = nxd % 3 == 0 ? 5 : 4;
   }
   h->halves = d.npairs >= 65536 ? 2 : 1;
-  h->solve_form = default_solve_form(d.npairs);
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev);
+  h->solve_form = default_solve_form(d.npairs, h->nsm);
   h->fac_slots = h->solve_form >= 3 ? 3 : 1;
   h->rz.n = rz.n; h->rz.nst = rz.nst; std::memcpy(h->rz.r, rz.r, sizeof rz.r);
   h->rx.n = rx.n; h->rx.nst = rx.nst; std::memcpy(h->rx.r, rx.r, sizeof rx.r);
@@ -1285,13 +1283,16 @@ int chgpu_ensemble_create(const chgpu_params* params, int n, chgpu_ensemble** ou
       return ens_fail(nullptr, rc, msg);
     }
   }
-  // the members share the GPU: their solve form is that of their pairs
-  // together (64 minimal channels, 42 472 pairs, mixed: 8.7 ms per step with
-  // four threads per pair, 10.3 with the eight that each would take alone)
+  // the members share the GPU: their solve form and the sizes of their blocks
+  // are those of their pairs together (64 minimal channels, 42 472 pairs,
+  // mixed: 8.7 ms per step with four threads per pair, 10.3 with the eight that
+  // each would take alone)
   long long pairs = 0;
   for (chgpu_handle* h : e->m) pairs += h->d.npairs;
-  const int form = default_solve_form((int)std::min<long long>(pairs, 65535));
-  for (chgpu_handle* h : e->m) h->solve_form = std::min(h->solve_form, form);
+  for (chgpu_handle* h : e->m) {
+    h->solve_form = std::min(h->solve_form, default_solve_form(std::min<long long>(pairs, 65535), h->nsm));
+    h->together = (double)pairs / h->d.npairs;
+  }
   cudaError_t c = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   if (c == cudaSuccess) c = cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming);
   for (int i = 0; i < n && c == cudaSuccess; ++i) c = cudaEventCreateWithFlags(&e->join[i], cudaEventDisableTiming);
@@ -2056,9 +2057,6 @@ int closure_alloc_all(chgpu_handle* h) {
   const size_t phys = (size_t)9 * np * d.nzd * d.nxd * sizeof(float2);
   // cl_P also stages host spectra (up to 9 fields, complex128) for chgpu_closure_physical
   const size_t stage = (size_t)9 * np * nm * sizeof(double2);
-  int dev = 0;
-  CK(h, cudaGetDevice(&dev));
-  CK(h, cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev));
   if (mlp_set_smem_limits() != 0) return fail(h, CHGPU_E_CUDA, "closure: shared-memory limit refused");
   auto alloc = [&](void** ptr, size_t bytes) -> int {
     cudaError_t e = cudaMalloc(ptr, bytes);

@@ -145,6 +145,10 @@ struct SolveLaunch {
                       // 3: k_factor then k_solve with eight threads per pair
   int slot;            // which of the handle's sets of factors
   size_t slot_stride;  // doubles per set
+  // the launch's share of the GPU, for the choices of blocks: its SMs, and how
+  // many times this handle's modes those of all handles that step together are
+  int nsm = 1;
+  double together = 1.0;
   int factored;       // split form: fac already holds this substep's factors (k_factor ran ahead), k_solve only
 };
 

@@ -33,6 +33,7 @@
 #include "chgpu_internal.h"
 #include "cplx.cuh"
 #include "kernels.cuh"
+#include "launch_rules.h"
 
 namespace chgpu {
 
@@ -114,7 +115,6 @@ template <> struct HistT<dd> { using t = double2; };
 // Relative L2 rounding error of expl_v, expl_eta at 79x101x75: 4.9e-16, 1.3e-15
 // from the products' stencils, 1.6e-16, 2.4e-16 so; 2.6e-15, 2.8e-16 and 6.1e-16,
 // 1.1e-16 at 9x192x12.
-constexpr int kRhsMaxRows = 32;
 template <typename T>
 __global__ void __launch_bounds__(128, 3) k_rhs(const double2* __restrict__ V, const typename C2<T>::t* __restrict__ VV,
                                              typename HistT<T>::t* __restrict__ old, double2* __restrict__ rhs,
@@ -432,34 +432,9 @@ __global__ void __launch_bounds__(128, 3) k_rhs(const double2* __restrict__ V, c
   }  // rows
 }
 
-// Rows per thread: the count that minimises the time of the fullest of 152
-// SMs, three blocks at a time.  A block's time is its rows plus the four
-// start-up rows of the windows (1 row's worth; 2 in the FP32 path, which
-// waits on their loads); three resident blocks take 3 units a row, one or two
-// kRhsPart (measured at 32x64x32 and 47x96x47: the FP64 pipe is nearly
-// filled by one block, the FP32 path's latency is not).  Against a fixed 16:
-// FP64 0.285 -> 0.157 ms a step at 32x64x32, 0.487 -> 0.382 at 47x96x47,
-// 1.29 -> 1.06 at 79x101x75; mixed 0.138 -> 0.067, 0.184 -> 0.136, 0.35 -> 0.30.
-template <typename T> struct RhsPart { static constexpr double one = 1.6, two = 2.4; };
-template <> struct RhsPart<double> { static constexpr double one = 1.25, two = 2.1; };
-template <> struct RhsPart<float> { static constexpr double one = 1.95, two = 2.6; };
-template <typename T>
-int rhs_rows(int modes, int ny) {
-  const int cols = (modes + 127) / 128;
-  const int start = std::is_same<T, float>::value ? 2 : 1;
-  int best = kRhsMaxRows;
-  double cost = 1e300;
-  for (int rb = kRhsMaxRows; rb >= 2; --rb) {
-    const long long blocks = (long long)cols * ((ny - 1 + rb - 1) / rb), per_sm = (blocks + 151) / 152;
-    const int part = (int)(per_sm % 3);
-    const double units = 3.0 * (double)(per_sm / 3) + (part == 1 ? RhsPart<T>::one : part == 2 ? RhsPart<T>::two : 0.0);
-    if (units * (rb + start) < cost) {
-      cost = units * (rb + start);
-      best = rb;
-    }
-  }
-  return best;
-}
+template <typename T> constexpr RhsCost rhs_cost() { return kRhsCostDD; }
+template <> constexpr RhsCost rhs_cost<double>() { return kRhsCostFP64; }
+template <> constexpr RhsCost rhs_cost<float>() { return kRhsCostFP32; }
 
 template <typename T>
 void launch_rhs(const SolveLaunch& L, cudaStream_t s) {
@@ -467,7 +442,7 @@ void launch_rhs(const SolveLaunch& L, cudaStream_t s) {
   using O2 = typename HistT<T>::t;
   using LT = typename LinT<T>::t;
   if (L.m_hi <= L.m_lo) return;
-  const int rb = rhs_rows<T>(L.m_hi - L.m_lo, L.d.ny);
+  const int rb = rhs_rows(rhs_cost<T>(), L.m_hi - L.m_lo, L.d.ny, L.nsm, L.together);
   dim3 grid((L.m_hi - L.m_lo + 127) / 128, (L.d.ny - 1 + rb - 1) / rb);
   k_rhs<T><<<grid, 128, 0, s>>>(L.V, (const V2*)L.VV, (O2*)L.old, L.rhs, (const LT*)L.derL, (const T*)L.derT, L.d,
                                 L.ode[0], L.ode[1], L.ode[2], L.sc, L.F, L.m_lo, L.m_hi, rb);
@@ -1656,11 +1631,10 @@ void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
   }
   if (!L.factored) launch_factor(L, s);
   if (L.split_solve == 3) {
-    // four parts where that still is one wave (two 256-thread blocks on each
-    // of 152 SMs), else two (four 128-thread blocks)
     const unsigned g16 = (unsigned)((L.q_hi - L.q_lo + 15) / 16);
-    auto kern = g16 <= 304 ? k_solve<true, 4> : k_solve<true, 2>;
-    kern<<<g16, g16 <= 304 ? 256 : 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu,
+    const bool four = solve_in_four_parts((int)g16, L.nsm, L.together);
+    auto kern = four ? k_solve<true, 4> : k_solve<true, 2>;
+    kern<<<g16, four ? 256 : 128, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu,
                                                 L.yint, L.bc, L.d, L.sc, (const dd*)L.lindd, L.q_lo, L.q_hi, L.slot);
     return;
   }
