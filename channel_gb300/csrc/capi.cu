@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -86,9 +87,7 @@ struct chgpu_handle {
   double2* F = nullptr;  // body force, plane-major like V
   bool use_F = false;
   double* fac = nullptr;
-  // sets of factors in fac: one per substep for the sizes whose default form
-  // factors ahead (at most 65 535 pairs), else one
-  int fac_slots = 1;
+  double* fac_rest = nullptr;  // the second and third substeps' sets of factors, or none (take_fac_rest)
   double* der = nullptr;
   void* derT = nullptr;
   void* derL = nullptr;
@@ -149,7 +148,6 @@ struct chgpu_handle {
   // Reynolds-stress budget spectra (allocated by the first chgpu_tke_reset)
   double2 *tke_W = nullptr, *tke_N = nullptr, *tke_P = nullptr, *tke_Zt = nullptr, *tke_Xt = nullptr;
   double *tke_acc = nullptr, *tke_mean = nullptr;
-  double* tke_sp = nullptr;  // chgpu_tke_result: spectra, work, profiles
   void *tke_twz = nullptr, *tke_twx = nullptr, *tke_twh = nullptr;
   RadixDev tke_rz{}, tke_rx{};
   int tke_chunk = 0;
@@ -179,6 +177,7 @@ int fail(chgpu_handle* h, int code, const std::string& msg) {
 }
 
 int cuda_fail(chgpu_handle* h, cudaError_t e, const char* where) {
+  cudaGetLastError();  // reported here, not once more by the next call
   return fail(h, e == cudaErrorMemoryAllocation ? CHGPU_E_NOMEM : CHGPU_E_CUDA,
               std::string(where) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
 }
@@ -188,6 +187,62 @@ int cuda_fail(chgpu_handle* h, cudaError_t e, const char* where) {
     cudaError_t e_ = (call);                                \
     if (e_ != cudaSuccess) return cuda_fail((h), e_, #call); \
   } while (0)
+
+// One set of factors of the two systems, in doubles.
+size_t fac_set(const chgpu_handle* h) { return (size_t)kFacPerRow * (h->d.ny - 1) * h->d.npairs; }
+double* fac_slot(const chgpu_handle* h, int slot) {
+  return slot == 0 ? h->fac : h->fac_rest + (slot - 1) * fac_set(h);
+}
+
+// The sets of factors of the second and third substeps, for the sizes whose
+// default form factors ahead.  A step needs only one set, so these are given up
+// whenever memory is short: all handles together take a 64th of the device's
+// memory at most (a fifth of a handle's own buffers would go into them) and one
+// handle a 16th of what is free, an allocation that fails takes them back
+// (dev_malloc), and the forms that factor each substep by itself do without.
+std::atomic<size_t> g_fac_rest_bytes{0};
+
+void drop_graph(chgpu_handle* h) {  // the captured step holds the old launch sequence
+  if (h->graph) {
+    cudaStreamSynchronize(h->stream);
+    cudaGraphExecDestroy(h->graph);
+    h->graph = nullptr;
+  }
+  ++h->version;  // an ensemble captures its members again
+}
+void drop_fac_rest(chgpu_handle* h) {
+  if (!h->fac_rest) return;
+  cudaDeviceSynchronize();  // no step that reads them is in flight, the ensemble's neither
+  drop_graph(h);
+  cudaFree(h->fac_rest);
+  h->fac_rest = nullptr;
+  g_fac_rest_bytes -= 2 * sizeof(double) * fac_set(h);
+}
+void take_fac_rest(chgpu_handle* h) {
+  if (h->solve_form < 3) drop_fac_rest(h);
+  if (h->solve_form < 3 || h->d.npairs >= 65536 || h->fac_rest) return;
+  const size_t bytes = 2 * sizeof(double) * fac_set(h);
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if ((g_fac_rest_bytes += bytes) <= total / 64 && bytes <= free / 16) {
+    if (cudaMalloc((void**)&h->fac_rest, bytes) == cudaSuccess) return;
+    cudaGetLastError();
+    h->fac_rest = nullptr;
+  }
+  g_fac_rest_bytes -= bytes;
+}
+cudaError_t dev_malloc(chgpu_handle* h, void** ptr, size_t bytes) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && h->fac_rest) {
+    cudaGetLastError();
+    drop_fac_rest(h);
+    e = cudaMalloc(ptr, bytes);
+  }
+  return e;
+}
 
 // element size of the transform buffers and spectra (and of the RK history)
 size_t tsize(const chgpu_handle* h) { return h->prec == CHGPU_MIXED ? sizeof(float2) : sizeof(double2); }
@@ -232,7 +287,7 @@ int upload_derT(chgpu_handle* h) {
   for (size_t i = 0; i < der.size(); ++i) t[i] = from_ld<T>((long double)der[i]);
   t[der.size()] = from_ld<T>((long double)h->p.alfa0);
   t[der.size() + 1] = from_ld<T>((long double)h->p.beta0);
-  CK(h, cudaMalloc(&h->derT, sizeof(T) * t.size()));
+  CK(h, dev_malloc(h, &h->derT, sizeof(T) * t.size()));
   CK(h, cudaMemcpy(h->derT, t.data(), sizeof(T) * t.size(), cudaMemcpyHostToDevice));
   // constants of the x-row pass: factor/2, 1/dx, 1/dz (dnsdata.f90:124), 1/dy(iy) per plane (:155)
   std::vector<T> c(3 + h->d.nplanes, T());
@@ -240,7 +295,7 @@ int upload_derT(chgpu_handle* h) {
   c[1] = from_ld<T>((long double)h->d.rdx);
   c[2] = from_ld<T>((long double)h->d.rdz);
   for (int iy = 1; iy <= h->p.ny - 1; ++iy) c[3 + iy + 1] = from_ld<T>(1.0L / (long double)h->tab.dy[iy]);
-  CK(h, cudaMalloc(&h->cst, sizeof(T) * c.size()));
+  CK(h, dev_malloc(h, &h->cst, sizeof(T) * c.size()));
   CK(h, cudaMemcpy(h->cst, c.data(), sizeof(T) * c.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -255,7 +310,7 @@ int upload_derL(chgpu_handle* h) {
   t[der.size()] = from_ld<L>((long double)h->p.alfa0);
   t[der.size() + 1] = from_ld<L>((long double)h->p.beta0);
   t[der.size() + 2] = from_ld<L>((long double)h->p.ni);
-  CK(h, cudaMalloc(&h->derL, sizeof(L) * t.size()));
+  CK(h, dev_malloc(h, &h->derL, sizeof(L) * t.size()));
   CK(h, cudaMemcpy(h->derL, t.data(), sizeof(L) * t.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -324,7 +379,7 @@ int upload_stage_twiddles(chgpu_handle* h, void** dst, const RadixDev& rad) {
       }
     Ns *= R;
   }
-  CK(h, cudaMalloc(dst, sizeof(V2) * w.size()));
+  CK(h, dev_malloc(h, dst, sizeof(V2) * w.size()));
   CK(h, cudaMemcpy(*dst, w.data(), sizeof(V2) * w.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -342,7 +397,7 @@ int upload_pack_roots(chgpu_handle* h, void** dst, int n, long double scale) {
     w[n + m].x = from_ld<T>(scale * cosl(ang));
     w[n + m].y = from_ld<T>(-scale * sinl(ang));
   }
-  CK(h, cudaMalloc(dst, sizeof(V2) * w.size()));
+  CK(h, dev_malloc(h, dst, sizeof(V2) * w.size()));
   CK(h, cudaMemcpy(*dst, w.data(), sizeof(V2) * w.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -415,7 +470,7 @@ bool xplan(int prec, int n, int* E, int* TPR) {
 }
 
 int upload_int4(chgpu_handle* h, void** dst, const std::vector<int4>& w) {
-  CK(h, cudaMalloc(dst, sizeof(int4) * w.size()));
+  CK(h, dev_malloc(h, dst, sizeof(int4) * w.size()));
   CK(h, cudaMemcpy(*dst, w.data(), sizeof(int4) * w.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -461,7 +516,7 @@ int upload_fx_step_tables(chgpu_handle* h) {
   if (int rc = upload_fx_tables(h, &h->fx)) return rc;
   std::vector<double> r(h->d.nplanes, 0.0);
   for (int iy = 1; iy <= h->p.ny - 1; ++iy) r[iy + 1] = 1.0 / h->tab.dy[iy];
-  CK(h, cudaMalloc((void**)&h->rdy, sizeof(double) * r.size()));
+  CK(h, dev_malloc(h, (void**)&h->rdy, sizeof(double) * r.size()));
   CK(h, cudaMemcpy(h->rdy, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -487,7 +542,7 @@ int upload_rplan_twiddles(chgpu_handle* h, void** dst, int n, bool xplan = false
         e.y = from_ld<T>(-sinl(ang));
       }
   }
-  CK(h, cudaMalloc(dst, sizeof(V2) * w.size()));
+  CK(h, dev_malloc(h, dst, sizeof(V2) * w.size()));
   CK(h, cudaMemcpy(*dst, w.data(), sizeof(V2) * w.size(), cudaMemcpyHostToDevice));
   return 0;
 }
@@ -563,7 +618,7 @@ SolveLaunch solve_launch(chgpu_handle* h, const double* ode) {
   L.F = h->use_F ? h->F : nullptr;
   L.fac = h->fac;
   L.slot = 0;
-  L.slot_stride = (size_t)kFacPerRow * (h->d.ny - 1) * h->d.npairs;
+  L.slot_stride = fac_set(h);
   L.nsm = h->nsm;
   L.together = h->together;
   L.der = h->der;
@@ -649,7 +704,7 @@ void run_rhs(chgpu_handle* h, const double* ode, cudaStream_t s = nullptr, int m
 // -> 2.92 at 83x120x85, 7.36 -> 7.22 at 127x192x127 (all three in one launch
 // 1.11, 2.90, 7.38); FP64 at 32x64x32 0.87 -> 0.77.
 void enqueue_factor(chgpu_handle* h, int k, bool after_half_b) {
-  if (h->fac_slots == 3 && k > 0) return;
+  if (h->fac_rest && k > 0) return;
   const double ode1 = RK[k][0];
   SolveLaunch L = solve_launch(h, nullptr);
   L.ode[0] = ode1;
@@ -660,8 +715,9 @@ void enqueue_factor(chgpu_handle* h, int k, bool after_half_b) {
   launch_factor(L, h->stream3);
   cudaEventRecord(h->ev_factored, h->stream3);
   h->launches += 1;
-  if (h->fac_slots == 3) {
+  if (h->fac_rest) {
     L.slot = 1;
+    L.fac = fac_slot(h, 1);
     L.ode[0] = RK[1][0];
     launch_factor(L, h->stream3, 2, RK[2][0]);
     cudaEventRecord(h->ev_factored_rest, h->stream3);
@@ -692,7 +748,8 @@ void run_linsolve(chgpu_handle* h, double ode1, double lambda, int from_dt, bool
   L.split_solve = h->solve_form == 1 ? 0 : (h->solve_form == 4 ? 2 : (h->solve_form == 5 ? 3 : 1));
   L.factored = factored && h->solve_form >= 2 ? 1 : 0;
   if (L.factored) {
-    L.slot = h->fac_slots == 3 ? substep : 0;
+    L.slot = h->fac_rest ? substep : 0;
+    L.fac = fac_slot(h, L.slot);
     cudaStreamWaitEvent(s, L.slot == 0 ? h->ev_factored : h->ev_factored_rest, 0);
   }
   timed(h, 4, [&] { launch_linsolve(L, s); });
@@ -778,6 +835,7 @@ int pull_scalars(chgpu_handle* h) {
 }
 
 void release(chgpu_handle* h) {
+  drop_fac_rest(h);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   for (auto& pe : h->ev_pending) {
     cudaEventDestroy(pe.second.first);
@@ -787,7 +845,7 @@ void release(chgpu_handle* h) {
   void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->fac, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
                   h->twz, h->twx, h->twh, h->twzr, h->twxr, h->fx.z, h->fx.x, h->fx.pack, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
                   h->cl_G, h->cl_Z, h->cl_P, h->cl_tau, h->cl_wd, h->cl_twz, h->cl_twx, h->cl_twh,
-                  h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean, h->tke_sp,
+                  h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean,
                   h->tke_twz, h->tke_twx, h->tke_twh};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -877,7 +935,6 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev);
   h->solve_form = default_solve_form(d.npairs, h->nsm);
-  h->fac_slots = h->solve_form >= 3 ? 3 : 1;
   h->rz.n = rz.n; h->rz.nst = rz.nst; std::memcpy(h->rz.r, rz.r, sizeof rz.r);
   h->rx.n = rx.n; h->rx.nst = rx.nst; std::memcpy(h->rx.r, rx.r, sizeof rx.r);
   set_twiddle_offsets(h->rz);
@@ -935,11 +992,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     if ((rc = dev_alloc(&h->Pb, std::max(ts * 6 * nplanes * nxp * nzd, sizeof(double2) * 3 * nplanes * nmodes),
                         "x work buffer"))) break;
     if ((rc = dev_alloc((void**)&h->rhs, sizeof(double2) * 2 * (p->ny - 1) * nmodes, "rhs"))) break;
-    if ((rc = dev_alloc((void**)&h->fac,
-                        sizeof(double) * kFacPerRow * (p->ny - 1) *
-                            (size_t)d.npairs * h->fac_slots,
-                        "factors")))
-      break;
+    if ((rc = dev_alloc((void**)&h->fac, sizeof(double) * fac_set(h), "factors"))) break;
     if ((rc = dev_alloc((void**)&h->der, sizeof(double) * t.der.size(), "der"))) break;
     if ((rc = dev_alloc((void**)&h->d0lu, sizeof(double) * t.d0lu.size(), "D0mat"))) break;
     if ((rc = dev_alloc((void**)&h->yint, sizeof(double) * std::max<size_t>(3, t.yint.size()), "yint"))) break;
@@ -1021,6 +1074,7 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     delete h;
     return rc;
   }
+  take_fac_rest(h);
   *out = h;
   return 0;
 }
@@ -1276,7 +1330,12 @@ int chgpu_ensemble_create(const chgpu_params* params, int n, chgpu_ensemble** ou
   e->m.assign(n, nullptr);
   e->join.assign(n, nullptr);
   for (int i = 0; i < n; ++i) {
-    if (int rc = chgpu_create(&params[i], &e->m[i])) {
+    int rc = chgpu_create(&params[i], &e->m[i]);
+    if (rc == CHGPU_E_NOMEM) {  // without the other members' optional buffers
+      for (int k = 0; k < i; ++k) drop_fac_rest(e->m[k]);
+      rc = chgpu_create(&params[i], &e->m[i]);
+    }
+    if (rc) {
       const std::string msg = "member " + std::to_string(i) + ": " + chgpu_last_error(nullptr);
       ens_release(e);
       delete e;
@@ -1435,8 +1494,8 @@ int tune_solve_and_halves(chgpu_handle* h) {
   const size_t vbytes = sizeof(double2) * 3 * (size_t)d.nplanes * d.nmodes;
   const size_t obytes = tsize(h) * 2 * (size_t)(d.ny - 1) * d.nmodes;
   void *sv = nullptr, *so = nullptr, *ss = nullptr;
-  if (cudaMalloc(&sv, vbytes) != cudaSuccess || cudaMalloc(&so, obytes) != cudaSuccess ||
-      cudaMalloc(&ss, sizeof(DevScalars)) != cudaSuccess) {
+  if (dev_malloc(h, &sv, vbytes) != cudaSuccess || dev_malloc(h, &so, obytes) != cudaSuccess ||
+      dev_malloc(h, &ss, sizeof(DevScalars)) != cudaSuccess) {
     // no room for the saved state: keep the current choice
     cudaGetLastError();
     if (sv) cudaFree(sv);
@@ -1587,11 +1646,8 @@ int chgpu_autotune(chgpu_handle* h) {
   }
   if (int rc = tune_solve_and_halves(h)) return rc;
   h->tuned = true;
-  ++h->version;
-  if (h->graph) {  // the captured step holds the old launch shapes
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
+  drop_graph(h);  // the captured step holds the old launch shapes
+  take_fac_rest(h);
   return 0;
 }
 
@@ -1620,11 +1676,8 @@ int chgpu_set_tiles(chgpu_handle* h, const int tiles[CHGPU_NTILES]) {
   h->xthreads = xt;
   h->solve_form = sf;
   h->halves = hv;
-  ++h->version;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
+  drop_graph(h);
+  take_fac_rest(h);
   return 0;
 }
 
@@ -1641,11 +1694,7 @@ int chgpu_set_step_halves(chgpu_handle* h, int halves) {
   if (!h || (halves != 1 && halves != 2)) return fail(h, CHGPU_E_PARAM, "chgpu_set_step_halves: 1 or 2");
   if (h->halves != halves) {
     h->halves = halves;
-    ++h->version;
-    if (h->graph) {
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-    }
+    drop_graph(h);
   }
   return 0;
 }
@@ -1705,11 +1754,11 @@ int export_setup(chgpu_handle* h) {
   // planes per chunk: W and P of a chunk within 256 MiB
   const size_t per_plane = (size_t)3 * (h->d.nx + 1) * Nz * sizeof(double2) + (size_t)3 * Nz * Nx * sizeof(double);
   h->ex_chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)h->d.ny + 1, (1ull << 28) / per_plane));
-  CK(h, cudaMalloc((void**)&h->ex_W, (size_t)3 * h->ex_chunk * (h->d.nx + 1) * Nz * sizeof(double2)));
-  CK(h, cudaMalloc((void**)&h->ex_P, (size_t)3 * h->ex_chunk * Nz * Nx * sizeof(double)));
+  CK(h, dev_malloc(h, (void**)&h->ex_W, (size_t)3 * h->ex_chunk * (h->d.nx + 1) * Nz * sizeof(double2)));
+  CK(h, dev_malloc(h, (void**)&h->ex_P, (size_t)3 * h->ex_chunk * Nz * Nx * sizeof(double)));
   const std::vector<double2> wz = roots<double2>(Nz), wx = roots<double2>(Nx);
-  CK(h, cudaMalloc((void**)&h->ex_twz, sizeof(double2) * Nz));
-  CK(h, cudaMalloc((void**)&h->ex_twx, sizeof(double2) * Nx));
+  CK(h, dev_malloc(h, (void**)&h->ex_twz, sizeof(double2) * Nz));
+  CK(h, dev_malloc(h, (void**)&h->ex_twx, sizeof(double2) * Nx));
   CK(h, cudaMemcpy(h->ex_twz, wz.data(), sizeof(double2) * Nz, cudaMemcpyHostToDevice));
   CK(h, cudaMemcpy(h->ex_twx, wx.data(), sizeof(double2) * Nx, cudaMemcpyHostToDevice));
   return 0;
@@ -1742,7 +1791,7 @@ int chgpu_export_physical(chgpu_handle* h, const chgpu_export_opts* o, double* o
     if (h->ex_out) CK(h, cudaFree(h->ex_out));
     h->ex_out = nullptr;
     h->ex_out_cap = 0;
-    CK(h, cudaMalloc((void**)&h->ex_out, need * sizeof(double)));
+    CK(h, dev_malloc(h, (void**)&h->ex_out, need * sizeof(double)));
     h->ex_out_cap = need;
   }
   ExportLaunch L{};
@@ -1785,7 +1834,7 @@ int chgpu_set_body_force(chgpu_handle* h, const double* F) {
     h->use_F = false;
   } else {
     const size_t n = (size_t)3 * h->d.nplanes * h->d.nmodes;
-    if (!h->F) CK(h, cudaMalloc((void**)&h->F, sizeof(double2) * n));
+    if (!h->F) CK(h, dev_malloc(h, (void**)&h->F, sizeof(double2) * n));
     double2* stage = reinterpret_cast<double2*>(h->Pb);
     CK(h, cudaMemcpyAsync(stage, F, sizeof(double2) * n, cudaMemcpyHostToDevice, h->stream));
     launch_transpose(stage, h->F, h->d.nmodes, h->d.nplanes, 3, h->stream);
@@ -1795,18 +1844,14 @@ int chgpu_set_body_force(chgpu_handle* h, const double* F) {
     CK(h, cudaStreamSynchronize(h->stream));
     h->use_F = true;
   }
-  if (was != h->use_F) ++h->version;
-  if (was != h->use_F && h->graph) {  // the captured step holds the old launch parameters
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
+  if (was != h->use_F) drop_graph(h);
   return 0;
 }
 
 int chgpu_stats_reset(chgpu_handle* h) {
   if (!h) return fail(h, CHGPU_E_PARAM, "null handle");
   const size_t n = (size_t)4 * 3 * h->d.nplanes;
-  if (!h->stats_acc) CK(h, cudaMalloc((void**)&h->stats_acc, sizeof(double) * n));
+  if (!h->stats_acc) CK(h, dev_malloc(h, (void**)&h->stats_acc, sizeof(double) * n));
   CK(h, cudaMemsetAsync(h->stats_acc, 0, sizeof(double) * n, h->stream));
   h->stats_n = 0;
   return 0;
@@ -1859,14 +1904,15 @@ int chgpu_tke_reset(chgpu_handle* h, const double* mean) {
     const size_t per_plane = 12 * nxp * (size_t)d.nzd * sizeof(double2);
     h->tke_chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)np, ((size_t)2 << 30) / per_plane));
     const size_t C = (size_t)h->tke_chunk;
-    CK(h, cudaMalloc((void**)&h->tke_W, sizeof(double2) * 12 * FS));
-    CK(h, cudaMalloc((void**)&h->tke_N, sizeof(double2) * 3 * FS));
-    CK(h, cudaMalloc((void**)&h->tke_P, sizeof(double2) * FS));
-    CK(h, cudaMalloc((void**)&h->tke_Zt, sizeof(double2) * 12 * C * nxp * d.nzd));
-    CK(h, cudaMalloc((void**)&h->tke_Xt, sizeof(double2) * 3 * C * nxp * d.nzd));
-    CK(h, cudaMalloc((void**)&h->tke_acc, sizeof(double) * 36 * (size_t)np * d.nzt));
-    CK(h, cudaMalloc((void**)&h->tke_mean, sizeof(double) * 5 * (size_t)np));
-    CK(h, cudaMalloc((void**)&h->tke_sp, sizeof(double) * (78 * (size_t)d.nzt + 60) * np));
+    // between samples W also holds the spectra, the work space and the profiles of chgpu_tke_result
+    CK(h, dev_malloc(h, (void**)&h->tke_W,
+                     std::max(sizeof(double2) * 12 * FS, sizeof(double) * (78 * (size_t)d.nzt + 60) * np)));
+    CK(h, dev_malloc(h, (void**)&h->tke_N, sizeof(double2) * 3 * FS));
+    CK(h, dev_malloc(h, (void**)&h->tke_P, sizeof(double2) * FS));
+    CK(h, dev_malloc(h, (void**)&h->tke_Zt, sizeof(double2) * 12 * C * nxp * d.nzd));
+    CK(h, dev_malloc(h, (void**)&h->tke_Xt, sizeof(double2) * 3 * C * nxp * d.nzd));
+    CK(h, dev_malloc(h, (void**)&h->tke_acc, sizeof(double) * 36 * (size_t)np * d.nzt));
+    CK(h, dev_malloc(h, (void**)&h->tke_mean, sizeof(double) * 5 * (size_t)np));
     Radix rz = make_radix(d.nzd, false), rx = make_radix(d.nxd, false);
     h->tke_rz.n = rz.n; h->tke_rz.nst = rz.nst; std::memcpy(h->tke_rz.r, rz.r, sizeof rz.r);
     h->tke_rx.n = rx.n; h->tke_rx.nst = rx.nst; std::memcpy(h->tke_rx.r, rx.r, sizeof rx.r);
@@ -1962,7 +2008,7 @@ int chgpu_tke_result(chgpu_handle* h, int timestwo, double* mean7, double* spect
                            {h->tab.d24m1, h->tab.d240, h->tab.d24n, h->tab.d24np1}};
   for (int o = 0; o < 2; ++o)
     for (int r = 0; r < 4; ++r) std::memcpy(rows.w[o][r], w[o][r], sizeof rows.w[o][r]);
-  double *sp = h->tke_sp, *work = sp + 60 * S, *prof = work + 18 * S;
+  double *sp = reinterpret_cast<double*>(h->tke_W), *work = sp + 60 * S, *prof = work + 18 * S;
   launch_tke_result(h->tke_acc, sp, work, prof, h->der, h->d0lu, rows, d, (double)h->tke_n, timestwo, h->stream);
   CK(h, cudaGetLastError());
   h->launches += 3;
@@ -1982,7 +2028,7 @@ int chgpu_snapshot_async(chgpu_handle* h) {
   if (h->snap_pending) return fail(h, CHGPU_E_STATE, "chgpu_snapshot_async: previous snapshot not collected");
   const size_t n = (size_t)3 * h->d.nplanes * h->d.nmodes;
   if (!h->snap_stage) {
-    CK(h, cudaMalloc((void**)&h->snap_stage, sizeof(double2) * n));
+    CK(h, dev_malloc(h, (void**)&h->snap_stage, sizeof(double2) * n));
     CK(h, cudaMallocHost((void**)&h->snap_host, sizeof(double2) * n));
     CK(h, cudaStreamCreateWithFlags(&h->snap_stream, cudaStreamNonBlocking));
     CK(h, cudaEventCreateWithFlags(&h->snap_read, cudaEventDisableTiming));
@@ -2023,15 +2069,6 @@ namespace {
 
 long long closure_plane_pts(const chgpu_handle* h) { return (long long)h->d.nzd * 2 * h->d.nxd; }
 
-void drop_graph(chgpu_handle* h) {  // the captured step holds the old launch sequence
-  if (h->graph) {
-    cudaStreamSynchronize(h->stream);
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
-  ++h->version;
-}
-
 void closure_free(chgpu_handle* h) {
   void** bufs[] = {(void**)&h->cl_G, (void**)&h->cl_Z, (void**)&h->cl_P, (void**)&h->cl_tau, (void**)&h->cl_wd,
                    &h->cl_twz, &h->cl_twx, &h->cl_twh};
@@ -2059,7 +2096,7 @@ int closure_alloc_all(chgpu_handle* h) {
   const size_t stage = (size_t)9 * np * nm * sizeof(double2);
   if (mlp_set_smem_limits() != 0) return fail(h, CHGPU_E_CUDA, "closure: shared-memory limit refused");
   auto alloc = [&](void** ptr, size_t bytes) -> int {
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    cudaError_t e = dev_malloc(h, ptr, bytes);
     return e == cudaSuccess ? 0 : fail(h, CHGPU_E_NOMEM, "closure: device allocation failed");
   };
   if (int rc = alloc((void**)&h->cl_G, (size_t)9 * np * nm * sizeof(double2))) return rc;

@@ -143,7 +143,7 @@ struct SolveLaunch {
   int split_solve;    // 0: the fused k_linsolve; 1: k_factor then k_solve (fac holds kFacPerRow per row);
                       // 2: k_factor then k_linsolve reading the factors (two threads per pair);
                       // 3: k_factor then k_solve with eight threads per pair
-  int slot;            // which of the handle's sets of factors
+  int slot;            // which of the handle's sets of factors fac is
   size_t slot_stride;  // doubles per set
   // the launch's share of the GPU, for the choices of blocks: its SMs, and how
   // many times this handle's modes those of all handles that step together are

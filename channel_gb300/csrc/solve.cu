@@ -1006,8 +1006,8 @@ __global__ void __launch_bounds__(64, 8) k_linsolve(double2* __restrict__ V, con
 // reciprocal pivot and upper entries LeftLU5divStep1 reads).  The eta thread
 // of the mean mode also stores the wall-velocity terms of its right-hand side
 // (rows 1, 2, ny-2, ny-1; linsolve_blocking.inc:26-27,40-41).
-// blockIdx.y: with factors for several substeps at once, the slot of fac (and
-// of sc->wallrhs) after slot0, with its substep's coefficient.
+// blockIdx.y: with factors for several substeps at once, the slot (of
+// sc->wallrhs) after slot0, fac's, with its substep's coefficient.
 // Registers capped for 8 resident 64-thread blocks per SM.
 struct FactorOdes {
   double a, b;
@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(64, 8) k_factor(double* __restrict__ fac, cons
   const int q = q_lo + blockIdx.x * 32 + lane;
   if (q >= q_hi) return;
   const int slot = slot0 + blockIdx.y;
-  fac += slot * slot_stride;
+  fac += blockIdx.y * slot_stride;
   const int ny = d.ny, nz = d.nz;
   const int ix = q / (nz + 1);
   const int a = q - ix * (nz + 1);
@@ -1621,7 +1621,7 @@ void launch_factor(const SolveLaunch& L, cudaStream_t s, int slots, double ode1_
 
 void launch_linsolve(const SolveLaunch& L, cudaStream_t s) {
   if (L.q_hi <= L.q_lo) return;
-  double* fac = L.fac + L.slot * L.slot_stride;
+  double* fac = L.fac;
   const unsigned grid = (unsigned)((L.q_hi - L.q_lo + 31) / 32);
   if (!L.split_solve) {
     k_linsolve<false><<<grid, 64, 0, s>>>(L.V, L.rhs_src, L.rhs_cstride, L.rhs_plane_off, fac, L.der, L.d0lu, L.yint,
