@@ -125,6 +125,29 @@ template <int E, int TPR, int NC> constexpr int fx_zminb() {
   return (E == 24 ? 384 : E == 12 ? 640 : 768) / (NC * TPR);
 }
 
+// Between two passes: the values of the group's transform shifted so that the
+// largest |re|, |im| is just below 2^BITS, or by `most` >= -62 to the left if
+// that is less.  Returns the shift to the left.
+template <int E, int TPR, int BITS>
+__device__ __forceinline__ int fx_renormalise(fx2 (&a)[E], int most, void* scratch, int t) {
+  int m = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int hx = fx_up(a[e].x), hy = fx_up(a[e].y);
+    m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
+  }
+  m = group_reduce<kRedOr, TPR>(m, scratch, t);
+  const int s = min(BITS - (64 - __clz(m)), most);
+  if (s >= 0) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) a[e] = fx2{a[e].x << s, a[e].y << s};
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], -s);
+  }
+  return s;
+}
+
 // Inverse x transform of one row, whose spectrum (FP64, kx = 0..nx) sits in
 // the slot F, by its TPR threads: the physical values a[e] at pair t + TPR e,
 // normalised so that the row's largest |re|, |im| is just below 2^kRowBits.
@@ -211,27 +234,12 @@ __device__ __forceinline__ void fx_forward_row(fx2 (&a)[E], fx2* X, int t, int n
   // 2^62 and the outputs 2^61 (for the unpacking)
   static_assert(E <= 12, "12 sqrt(2) 2^57.6 < 2^62");
   constexpr int kMid = fx_bits(fx_growth(E, TPR, false), 61);
-  int mid = 0;  // shift to the left between passes 1 and 2
-  rfft<E, TPR, -1, true>(a, X, t, tw, [&](int o, fx2 v) { X[o] = v; }, [&] {
-    int m = 0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int hx = fx_up(a[e].x), hy = fx_up(a[e].y);
-      m |= (hx ^ (hx >> 31)) | (hy ^ (hy >> 31));
-    }
-    m = group_reduce<kRedOr, TPR>(m, scratch, t);
-    mid = kMid - (64 - __clz(m));
-    if (mid >= 0) {
-#pragma unroll
-      for (int e = 0; e < E; ++e) a[e] = fx2{a[e].x << mid, a[e].y << mid};
-    } else {
-#pragma unroll
-      for (int e = 0; e < E; ++e) a[e] = fx_shr(a[e], -mid);
-    }
-  });
   // the passes after the first and the unpacking are at quarter scale
-  const int So = scale + mid - 2 * rplan_passes(E, TPR) - fac.exp;
-  const int mode = fx_mode<double>(So, nf);
+  int So = scale - 2 * rplan_passes(E, TPR) - fac.exp;
+  rfft<E, TPR, -1, true>(a, X, t, tw, [&](int o, fx2 v) { X[o] = v; }, [&] {
+    So += fx_renormalise<E, TPR, kMid>(a, 64, scratch, t);
+  });
+  const int mode = nf ? kNan : So < FxIo<double>::kSMin || So > FxIo<double>::kSMax ? 1 : 0;
   group_sync<TPR>();
   // r2c unpacking, kx = 0..nx (HFT, dnsdata.f90:586), at quarter scale, in
   // place and two entries at a time: with s = g (Z_k + conj Z_{M-k}) and
@@ -245,8 +253,8 @@ __device__ __forceinline__ void fx_forward_row(fx2 (&a)[E], fx2* X, int t, int n
     const fx2 sm{zk.x + zc.x, zk.y - zc.y}, df{zk.x - zc.x, zk.y + zc.y};
     const fx2 r = fx_cmul<-1>(fx2{df.y, -df.x}, fx_ldw(twh + M + k));
     const fx2 s{fx_mad(0, sm.x, fac.gh, fac.gl), fx_mad(0, sm.y, fac.gh, fac.gl)};
-    Xr[k] = fx_store<double>(s + r, So, mode);
-    if (kc <= nx && kc != k) Xr[kc] = fx_store<double>(fx2{s.x - r.x, r.y - s.y}, So, mode);
+    Xr[k] = fx_store_any(s + r, So, mode);
+    if (kc <= nx && kc != k) Xr[kc] = fx_store_any(fx2{s.x - r.x, r.y - s.y}, So, mode);
   }
 }
 
@@ -323,8 +331,8 @@ __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zinv_x(con
   for (int e = 0; e < E; ++e) B += fx_lead_at(raw[e].x, emax) + fx_lead_at(raw[e].y, emax);
   const unsigned B1 = (unsigned)group_reduce<kRedMax, TPR>((int)B, buf, t);
   B = (unsigned)group_reduce<kRedSum, TPR>((int)B, buf, t);
-  const int S1 = emax == 0 ? 0 : fx_scale_sum<double>(emax, B1, 62);
-  const int S = emax == 0 ? 0 : fx_scale_sum<double>(emax, B, 62);
+  const int S1 = emax == 0 ? 0 : fx_cap<double>(fx_scale_sum<double>(emax, B1, 62), 1);
+  const int S = emax == 0 ? 0 : fx_cap<double>(fx_scale_sum<double>(emax, B, 62), 1);
   fx2 a[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {  // conversions only where there is a mode: they fill half the FP64 pipe
@@ -333,12 +341,12 @@ __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zinv_x(con
     if (jz <= nz || jz >= N - nz) a[e] = fx_load<double>(raw[e], S1);
   }
   const int So = S - 2;  // one pass at quarter scale
-  const int mode = fx_mode<double>(So, emax == In::kExpMax);
+  const bool nan = fx_nan<double>(So, emax == In::kExpMax);
   double2* dst = Zb + (((size_t)c * win.planes + plane - win.first) * (d.nx + 1) + cx) * N;
   rfft<E, TPR, +1>(
       a, buf, t, tw,
       [&](int o, fx2 v) {
-        if (active) dst[o] = fx_store<double>(v, So, mode);
+        if (active) dst[o] = fx_store<double>(v, So, nan);
       },
       [&] {
 #pragma unroll
@@ -373,17 +381,18 @@ __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zfwd_x(con
   }
   emax = group_reduce<kRedMax, TPR>(emax, buf, t);
   // |re|, |im| < 2^(emax - bias + 1)
-  const int S = emax == 0 ? 0 : fx_forward_bits(E, TPR, 62) - (emax - Io::kBias + 1);
+  constexpr int kQuarters = fx_quarters(E, TPR);
+  const int S = emax == 0 ? 0 : fx_cap<T>(fx_forward_bits(E, TPR, 62) - (emax - Io::kBias + 1), kQuarters);
   fx2 a[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) a[e] = fx_load<double>(raw[e], S);
-  const int So = S - 2 * fx_quarters(E, TPR);
-  const int mode = fx_mode<T>(So, emax == Io::kExpMax);
+  const int So = S - 2 * kQuarters;
   V2* dst = VV + (((size_t)p * d.nplanes + plane) * nxp + cx) * nzt + nz;
+  const bool nan = fx_nan<T>(So, emax == Io::kExpMax);
   rfft<E, TPR, -1>(a, buf, t, tw, [&](int o, fx2 v) {
     if (!active) return;
-    if (o <= nz) dst[o] = fx_store<T>(v, So, mode);
-    else if (o >= N - nz) dst[o - N] = fx_store<T>(v, So, mode);
+    if (o <= nz) dst[o] = fx_store<T>(v, So, nan);
+    else if (o >= N - nz) dst[o - N] = fx_store<T>(v, So, nan);
   });
 }
 
@@ -464,9 +473,9 @@ __global__ void __launch_bounds__(NR * TPR, MINB) k_xrow_x(const double2* __rest
       const int s3[3] = {su, sv, sw};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const int md = fx_mode<double>(s3[c], (bad >> c) & 1);
-        inf = inf || md == 2;
-        r[c] = md ? 0.0 : r[c] * __hiloint2double((1023 - s3[c]) << 20, 0);
+        inf = inf || ((bad >> c) & 1);
+        const int s = max(-2000, min(-s3[c], 2000)), s1 = s >> 1;  // a velocity below 2^-960 may count as zero
+        r[c] = r[c] * FxIo<double>::pow2(s1) * FxIo<double>::pow2(s - s1);
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) {

@@ -267,7 +267,7 @@ template <> struct FxIo<double> {
   __device__ static int expo(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
   // leading 19 significand bits, in units of 2^(expo - kBias - 18)
   __device__ static int lead(double v) { return ((__double2hiint(v) & 0xfffff) | 0x100000) >> 2; }
-  // round(v 2^S); zero below one unit
+  // round(v 2^S); zero below one unit, and where v is below the normal range
   __device__ static long long in(double v, int S) {
     const int hi = __double2hiint(v), e = hi & 0x7ff00000, t = e + (S << 20);
     const double s = __hiloint2double((hi & (int)0x800fffff) | t, __double2loint(v));
@@ -277,7 +277,13 @@ template <> struct FxIo<double> {
     const double d = __ll2double_rn(f);
     return f == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (S << 20), __double2loint(d));
   }
-  static constexpr int kSMin = -900, kSMax = 1020;  // scales whose results are normal numbers
+  static constexpr int kSMin = -961, kSMax = 1022;  // scales at which out() holds for |f| <= 2^62
+  __device__ static double pow2(int s) { return __hiloint2double((1023 + s) << 20, 0); }  // -1022 <= s <= 1023
+  // the same at any scale, rounded once: subnormal, zero and infinite too
+  __device__ static double out_any(long long f, int S) {
+    const int s = max(-2000, min(-S, 2000)), s1 = s >> 1;
+    return __ll2double_rn(f) * pow2(s1) * pow2(s - s1);
+  }
   __device__ static double nan() { return __longlong_as_double(0x7ff8000000000000ll); }
 };
 template <> struct FxIo<dd> {
@@ -289,25 +295,38 @@ template <> struct FxIo<dd> {
     const float f1 = pow2(s1), f2 = pow2(-S - s1);
     return dd(h * f1 * f2, l * f1 * f2);
   }
-  static constexpr int kSMin = -60, kSMax = 180;
+  static constexpr int kSMin = -252, kSMax = 252;
   __device__ static dd nan() { return dd(__int_as_float(0x7fc00000), 0.f); }
 };
-// 0: a usual scale; 1: every value below the type's normal range (zeros are
-// written); 2: not finite, or above it (NaN is written)
-template <typename T> __device__ __forceinline__ int fx_mode(int S, bool bad) {
-  return bad || S < FxIo<T>::kSMin ? 2 : (S > FxIo<T>::kSMax ? 1 : 0);
+// The z kernels hold data that would take a larger scale than kSMax (below
+// 2^(bits - kSMax) throughout, zeros among them) at a smaller one, so that one unit
+// of the result is at least the smallest normal number 2^-1022 (double-float:
+// 2^-252, where every value rounds to zero).  NaN is written where the data are
+// not finite, and at scales below kSMin, whose column's or row's bound exceeds
+// the type's range: values within a factor 2^11 of overflow.
+template <typename T> __device__ __forceinline__ int fx_cap(int S, int quarters) {
+  return min(S, FxIo<T>::kSMax + 2 * quarters);
 }
-template <typename T> __device__ __forceinline__ typename FxIo<T>::V2 fx_store(fx2 v, int S, int mode) {
+template <typename T> __device__ __forceinline__ bool fx_nan(int S, bool bad) { return bad || S < FxIo<T>::kSMin; }
+template <typename T> __device__ __forceinline__ typename FxIo<T>::V2 fx_store(fx2 v, int S, bool nan) {
   using Io = FxIo<T>;
   typename Io::V2 r;
-  if (mode == 0) {
+  if (nan) {
+    r.x = Io::nan();
+    r.y = r.x;
+  } else {
     r.x = Io::out(v.x, S);
     r.y = Io::out(v.y, S);
-  } else {
-    r.x = mode == 2 ? Io::nan() : T();
-    r.y = r.x;
   }
   return r;
+}
+// The x rows' (FP64), whose scale a product's two factors have set: any scale,
+// NaN only for data that are not finite (-1).
+constexpr int kNan = -1;
+__device__ __forceinline__ double2 fx_store_any(fx2 v, int S, int mode) {  // mode 0: kSMin <= S <= kSMax; 1: another
+  using Io = FxIo<double>;
+  if (mode == 0) return make_double2(Io::out(v.x, S), Io::out(v.y, S));
+  return mode == kNan ? make_double2(Io::nan(), Io::nan()) : make_double2(Io::out_any(v.x, S), Io::out_any(v.y, S));
 }
 template <typename T> __device__ __forceinline__ fx2 fx_load(typename FxIo<T>::V2 v, int S) {
   return fx2{FxIo<T>::in(v.x, S), FxIo<T>::in(v.y, S)};
