@@ -354,6 +354,16 @@ __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zinv_x(con
       });
 }
 
+// The scale from the column's largest value leaves room for the growth of a
+// white column; one whose spectrum is no larger than its peak (all modes in
+// phase) loses the passes' quarters instead, 2 bits each.  Its later passes get
+// them back by a shift between passes 1 and 2, where an FP64 transform would be
+// the more accurate one without: from 256 points on, 384 excepted (relative
+// error of the products of a coherent spectrum at 256, 512, 1024, 1536 points:
+// FP64 transforms 2.6, 4.1, 2.8, 3.5e-16, without 2.8, 4.9, 8.4, 20e-16).
+template <typename T> constexpr bool fx_zfwd_mid(int E, int TPR) {
+  return std::is_same<T, double>::value && (E == 12 ? TPR > 32 : TPR >= 32);
+}
 template <typename T, int E, int TPR, int NC>
 __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zfwd_x(const double2* __restrict__ Pb,
                                                                        typename C2<T>::t* __restrict__ VV,
@@ -381,19 +391,27 @@ __global__ void __launch_bounds__(NC * TPR, fx_zminb<E, TPR, NC>()) k_zfwd_x(con
   }
   emax = group_reduce<kRedMax, TPR>(emax, buf, t);
   // |re|, |im| < 2^(emax - bias + 1)
+  constexpr bool MID = fx_zfwd_mid<T>(E, TPR);
+  constexpr int kIn = MID ? fx_bits(fx_growth_first(E), 62) : fx_forward_bits(E, TPR, 62);
   constexpr int kQuarters = fx_quarters(E, TPR);
-  const int S = emax == 0 ? 0 : fx_cap<T>(fx_forward_bits(E, TPR, 62) - (emax - Io::kBias + 1), kQuarters);
+  const int S = emax == 0 ? 0 : fx_cap<T>(kIn - (emax - Io::kBias + 1), kQuarters);
   fx2 a[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) a[e] = fx_load<double>(raw[e], S);
-  const int So = S - 2 * kQuarters;
+  int So = S - 2 * kQuarters;
   V2* dst = VV + (((size_t)p * d.nplanes + plane) * nxp + cx) * nzt + nz;
-  const bool nan = fx_nan<T>(So, emax == Io::kExpMax);
-  rfft<E, TPR, -1>(a, buf, t, tw, [&](int o, fx2 v) {
-    if (!active) return;
-    if (o <= nz) dst[o] = fx_store<T>(v, So, nan);
-    else if (o >= N - nz) dst[o - N] = fx_store<T>(v, So, nan);
-  });
+  rfft<E, TPR, -1>(
+      a, buf, t, tw,
+      [&](int o, fx2 v) {
+        if (!active) return;
+        const bool nan = fx_nan<T>(So, emax == Io::kExpMax);
+        if (o <= nz) dst[o] = fx_store<T>(v, So, nan);
+        else if (o >= N - nz) dst[o - N] = fx_store<T>(v, So, nan);
+      },
+      [&] {
+        if constexpr (MID)
+          So += fx_renormalise<E, TPR, fx_bits(fx_growth(E, TPR, false), 62)>(a, FxIo<T>::kSMax - So, buf, t);
+      });
 }
 
 // Row layout in shared memory: u and v in physical space (M each), then the

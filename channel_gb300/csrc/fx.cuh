@@ -1,18 +1,23 @@
 // 64-bit fixed-point arithmetic of the FP64 and double-float transforms.
 //
-// GB300 does 2 FP64 fused multiply-adds per SM and clock, but 32 integer
+// GB300 does 2 FP64 fused multiply-adds per SM and clock, but 72 integer
 // multiply-adds 32x32+64 -> 64 bits (one instruction of the heavy FMA pipe)
-// and 64 64-bit additions (measured).  A radix-2 butterfly costs 6 FP64
+// and 63 64-bit additions (measured).  A radix-2 butterfly costs 6 FP64
 // instructions (3 clocks of an SM) or, on integers with 62 significant bits,
-// 12 of those multiply-adds (0.4 clocks) and about as many additions.  So the
+// 12 of those multiply-adds and about as many additions (0.2 clocks each).  So the
 // transforms hold their data as block fixed point: every column or row of a
 // transform has one power-of-two scale S, an element x is the 64-bit integer
 // F = x 2^S, and S is chosen from the data so that no intermediate value of
 // the transform can overflow (fx_scale_sum, fx_forward_bits).  In and out are FP64
-// (or double-float) values; between them the rounding errors are a few units
-// of 2^-62 of the column's norm, below the 2^-53 of an FP64 transform
-// (measured over the workloads' and broadband fields in
-// tests/test_gpu_fixed_point.py).
+// (or double-float) values.  Bits held between them: the z-inverse 62 of the sum
+// of a column's moduli; the x rows 57 of a row's largest mode, 60 of its largest
+// physical value, 56 of the largest product two rows allow; the z-forward 56 to
+// 58 of a column's largest value; the forward passes scale by a quarter each
+// (2 bits), shifted back up between passes 1 and 2 in the x rows and in the long
+// z-forward ones.  In all that leaves an error below an FP64 transform's (white
+// and falling spectra 1.1 to 3.1e-16, FP64 transforms 2.5 to 6.1e-16, up to 1536
+// points; spectra in phase, at the bounds of the headroom, 1.3 to 4e-16, 2.2 to
+// 4.3e-16: tests/test_gpu_fixed_point.py and test_gpu_fixed_point_range.py).
 //
 // A product a W / 2^64 of 64-bit integers is formed from balanced 32-bit
 // halves (a = ah 2^32 + al, |al| <= 2^31): ah wh + (ah wl + al wh + 2^31) >> 32;

@@ -351,6 +351,11 @@ __host__ __device__ constexpr FxGrowth fx_growth(int E, int TPR, bool with_first
   }
   return FxGrowth{mx, g};
 }
+// The same of the first pass alone.
+__host__ __device__ constexpr FxGrowth fx_growth_first(int E) {
+  const double g = E == 24 ? 6.0 : (double)E;
+  return FxGrowth{g, g};
+}
 // Bits of the largest component with which every later modulus stays below
 // 2^62 and the outputs' below 2^final.
 __host__ __device__ constexpr int fx_bits(FxGrowth g, int final_bits) {
