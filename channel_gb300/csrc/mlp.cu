@@ -118,11 +118,13 @@ __device__ __forceinline__ void store1(unsigned char* dst, float x) {
 }
 
 // 1 / (1 + exp(-z)): the approximate reciprocal and one Newton-Raphson step,
-// which the operand's range [1, 6.1e37] lets go without the branch of a
-// general division, so that the independent activations of a lane interleave.
-// The same bits as the division for z in [-80, 80] (0 of 3 10^8 values differ).
+// which the operand's range [1, 3e38] lets go without the branch of a general
+// division, so that the independent activations of a lane interleave.  The
+// same bits as the division wherever that is a normal number, z >= -87.3 (every
+// float of [-90, 90] compared); 0 below, where the division is subnormal down
+// to -88.7 and then 0 too.
 __device__ __forceinline__ float sigmoid(float z) {
-  const float x = 1.0f + expf(fminf(-z, 87.0f));
+  const float x = fminf(1.0f + expf(-z), 3.0e38f);
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return fmaf(y, fmaf(-x, y, 1.0f), y);
