@@ -12,7 +12,9 @@ namespace chgpu {
 // while its blocks are one wave (16 pairs per 128-thread block, four blocks
 // on each SM, 9728 pairs on 152; ms per mixed step against four threads per
 // pair: 32x64x32 0.51 / 0.66, 47x96x47 1.07 / 1.28, 83x120x85 2.70 / 2.83, but
-// 127x192x127 6.97 / 6.45), then four threads, then the fused kernel.
+// 127x192x127 6.97 / 6.45), then four threads, then the fused kernel.  The line
+// is the same in FP64 and double-float: eight threads per pair take 0.79 of the
+// step of four at 1089 pairs, 0.96 at 7225, 0.99 at 9604, 1.06 at 12 321.
 inline int default_solve_form(long long pairs, int nsm) { return pairs <= 16ll * 4 * nsm ? 5 : pairs < 65536 ? 3 : 1; }
 
 // Eight threads per pair, blocks of 16 pairs: four parts (256 threads) where
@@ -27,6 +29,8 @@ inline bool solve_in_four_parts(int blocks, int nsm, double together) { return b
 // filled by one block, the FP32 path's latency is not).  Against a fixed 16:
 // FP64 0.285 -> 0.157 ms a step at 32x64x32, 0.487 -> 0.382 at 47x96x47,
 // 1.29 -> 1.06 at 79x101x75; mixed 0.138 -> 0.067, 0.184 -> 0.136, 0.35 -> 0.30.
+// Over nine sizes from 16x40x16 to 127x64x127 and 20x250x240 the choice is within
+// 8% of the best of 12 counts, at seven of them within 4%.
 //
 // Of the other handles of an ensemble one in eight counts: their steps run side
 // by side, but not all in k_rhs at once.  ms per step with none, an eighth and
