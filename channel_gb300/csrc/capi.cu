@@ -86,7 +86,7 @@ struct chgpu_handle {
   double2* rhs = nullptr;
   double2* F = nullptr;  // body force, plane-major like V
   bool use_F = false;
-  double* fac = nullptr;
+  double* fac = nullptr;  // behind rhs in its allocation
   double* fac_rest = nullptr;  // the second and third substeps' sets of factors, or none (take_fac_rest)
   double* der = nullptr;
   void* derT = nullptr;
@@ -197,10 +197,18 @@ double* fac_slot(const chgpu_handle* h, int slot) {
 // The sets of factors of the second and third substeps, for the sizes whose
 // default form factors ahead.  A step needs only one set, so these are given up
 // whenever memory is short: all handles together take a 64th of the device's
-// memory at most (a fifth of a handle's own buffers would go into them) and one
-// handle a 16th of what is free, an allocation that fails takes them back
-// (dev_malloc), and the forms that factor each substep by itself do without.
+// memory at most (a fifth of a handle's own buffers would go into them), an
+// allocation of the handle that fails takes them back (dev_malloc), and the
+// forms that factor each substep by itself do without.
 std::atomic<size_t> g_fac_rest_bytes{0};
+size_t fac_rest_most() {
+  static const size_t most = [] {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) cudaGetLastError();
+    return total / 64;
+  }();
+  return most;
+}
 
 void drop_graph(chgpu_handle* h) {  // the captured step holds the old launch sequence
   if (h->graph) {
@@ -222,12 +230,7 @@ void take_fac_rest(chgpu_handle* h) {
   if (h->solve_form < 3) drop_fac_rest(h);
   if (h->solve_form < 3 || h->d.npairs >= 65536 || h->fac_rest) return;
   const size_t bytes = 2 * sizeof(double) * fac_set(h);
-  size_t free = 0, total = 0;
-  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  if ((g_fac_rest_bytes += bytes) <= total / 64 && bytes <= free / 16) {
+  if ((g_fac_rest_bytes += bytes) <= fac_rest_most()) {
     if (cudaMalloc((void**)&h->fac_rest, bytes) == cudaSuccess) return;
     cudaGetLastError();
     h->fac_rest = nullptr;
@@ -842,7 +845,7 @@ void release(chgpu_handle* h) {
     cudaEventDestroy(pe.second.second);
   }
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
-  void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->fac, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
+  void* bufs[] = {h->V, h->F, h->old, h->VV, h->Zb, h->Pb, h->rhs, h->der, h->derT, h->derL, h->cst, h->d0lu, h->nud, h->lindd, h->yint, h->dy,
                   h->twz, h->twx, h->twh, h->twzr, h->twxr, h->fx.z, h->fx.x, h->fx.pack, h->rdy, h->sc, h->ex_W, h->ex_P, h->ex_out, h->ex_twz, h->ex_twx,
                   h->cl_G, h->cl_Z, h->cl_P, h->cl_tau, h->cl_wd, h->cl_twz, h->cl_twx, h->cl_twh,
                   h->tke_W, h->tke_N, h->tke_P, h->tke_Zt, h->tke_Xt, h->tke_acc, h->tke_mean,
@@ -991,8 +994,9 @@ int chgpu_create(const chgpu_params* p, chgpu_handle** out) {
     if ((rc = dev_alloc(&h->Zb, ts * 3 * nplanes * nxp * nzd, "z work buffer"))) break;
     if ((rc = dev_alloc(&h->Pb, std::max(ts * 6 * nplanes * nxp * nzd, sizeof(double2) * 3 * nplanes * nmodes),
                         "x work buffer"))) break;
-    if ((rc = dev_alloc((void**)&h->rhs, sizeof(double2) * 2 * (p->ny - 1) * nmodes, "rhs"))) break;
-    if ((rc = dev_alloc((void**)&h->fac, sizeof(double) * fac_set(h), "factors"))) break;
+    const size_t rhs_bytes = (sizeof(double2) * 2 * (p->ny - 1) * nmodes + 255) / 256 * 256;
+    if ((rc = dev_alloc((void**)&h->rhs, rhs_bytes + sizeof(double) * fac_set(h), "rhs and factors"))) break;
+    h->fac = reinterpret_cast<double*>(reinterpret_cast<char*>(h->rhs) + rhs_bytes);
     if ((rc = dev_alloc((void**)&h->der, sizeof(double) * t.der.size(), "der"))) break;
     if ((rc = dev_alloc((void**)&h->d0lu, sizeof(double) * t.d0lu.size(), "D0mat"))) break;
     if ((rc = dev_alloc((void**)&h->yint, sizeof(double) * std::max<size_t>(3, t.yint.size()), "yint"))) break;
