@@ -25,14 +25,14 @@
 // stencils read it), double-float.
 //
 // What bounds them (GB300, counters at 255x64x255): latency at 12 (k_xrow_x,
-// by its rows' shared memory) to 15 warps per SM, with 45-54% of the issue
-// slots and 57-59% of the integer multiply-add pipe taken; in the z kernels the
+// by its rows' shared memory) to 15 warps per SM, with 46-56% of the issue
+// slots and 58-59% of the integer multiply-add pipe taken; in the z kernels the
 // conversions of their inputs and outputs also take half of the FP64 pipe.  Not
 // memory: 2 TB/s in the z kernels.  Against the FP64-pipe transforms they
-// replace, ms per step: k_zinv, k_xrow, k_zfwd 3.77, 23.2, 7.47 -> 0.85, 4.7,
-// 1.56 at 127x192x127, 108, 853, 214 -> 24, 186, 47 at 383x384x383; the
-// double-float ones 41, 291, 70 -> 24, 186, 57.  In-place packing by pairs of
-// entries, one code path for the three inverse rows: k_xrow_x 38.7 -> 28.8 ms at
+// replace, ms per step: k_zinv, k_xrow, k_zfwd 3.77, 23.2, 7.47 -> 0.85, 4.75,
+// 1.55 at 127x192x127, 108, 853, 214 -> 24, 185, 49 at 383x384x383; the
+// double-float ones 41, 291, 70 -> 24, 185, 56.  In-place packing by pairs of
+// entries, one code path for the three inverse rows: k_xrow_x 38.7 -> 28.7 ms at
 // 255x256x255.
 #pragma once
 

@@ -15,9 +15,9 @@
 // 58 of a column's largest value; the forward passes scale by a quarter each
 // (2 bits), shifted back up between passes 1 and 2 in the x rows and in the long
 // z-forward ones.  In all that leaves an error below an FP64 transform's (white
-// and falling spectra 1.1 to 3.1e-16, FP64 transforms 2.5 to 6.1e-16, up to 1536
-// points; spectra in phase, at the bounds of the headroom, 1.3 to 4e-16, 2.2 to
-// 4.3e-16: tests/test_gpu_fixed_point.py and test_gpu_fixed_point_range.py).
+// and falling spectra 0.8 to 3.4e-16, FP64 transforms 2.5 to 6.1e-16, up to 1536
+// points; spectra in phase, at the bounds of the headroom, 1.3 to 3.9e-16, 2.2
+// to 4.4e-16: tests/test_gpu_fixed_point.py and test_gpu_fixed_point_range.py).
 //
 // A product a W / 2^64 of 64-bit integers is formed from balanced 32-bit
 // halves (a = ah 2^32 + al, |al| <= 2^31): ah wh + (ah wl + al wh + 2^31) >> 32;
